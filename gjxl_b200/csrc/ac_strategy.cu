@@ -11,7 +11,7 @@
 // FindBestFirstLevelDivision, SearchTile) over all 64x64 tiles. The
 // reference's CUDA path evaluates the candidates on the GPU, copies the cost
 // table to the host and merges there (src/gpu/ops/ac_strategy_search.cpp:
-// 626-740); here the merge runs on the device, one thread per tile, so the
+// 626-740); here the merge runs on the device, one warp per tile, so the
 // strategy grid never leaves HBM.
 //
 // Work layout: one kernel instantiation per transform family <W, H>; each CTA
@@ -1090,12 +1090,13 @@ __device__ __forceinline__ int CoveredH(int s) {
        : s == kDct16x32 ? 2 : 1;
 }
 
+// One tile's search state, in shared memory.
 struct TileState {
-  uint8_t cell[64];
+  float family_cost[kFamilyCount][64];  // the tile's candidate costs
   float cost[64];
+  uint8_t cell[64];
   uint8_t priority[64];
   int tile_w, tile_h;
-  int bx0, by0;
 };
 
 __device__ __forceinline__ uint8_t Encode(int s, bool anchor) {
@@ -1110,10 +1111,14 @@ __device__ void SetCells(TileState& t, int lx, int ly, int s) {
 
 // SearchGrid::CrossesHorizontalBoundary / CrossesVerticalBoundary
 // (ac_strategy.cpp:155-200), restricted to the tile (which they never leave).
+// kAligned: the start lies on its region's first column (row) and no transform
+// reaches into the region from before it, so a start that is no anchor crosses
+// and nothing outside the region is read.
+template <bool kAligned>
 __device__ bool CrossesHorizontal(const TileState& t, int start_x, int y, int end_x) {
   if (start_x >= t.tile_w || y >= t.tile_h || y % 8 == 0) return false;
   end_x = min(end_x, t.tile_w);
-  while (start_x != 0 && !(t.cell[y * 8 + start_x] & 1)) --start_x;
+  while (!kAligned && start_x != 0 && !(t.cell[y * 8 + start_x] & 1)) --start_x;
   for (int x = start_x; x < end_x;) {
     const uint8_t c = t.cell[y * 8 + x];
     if (!(c & 1)) return true;
@@ -1122,10 +1127,11 @@ __device__ bool CrossesHorizontal(const TileState& t, int start_x, int y, int en
   return false;
 }
 
+template <bool kAligned>
 __device__ bool CrossesVertical(const TileState& t, int x, int start_y, int end_y) {
   if (x >= t.tile_w || start_y >= t.tile_h || x % 8 == 0) return false;
   end_y = min(end_y, t.tile_h);
-  while (start_y != 0 && !(t.cell[start_y * 8 + x] & 1)) --start_y;
+  while (!kAligned && start_y != 0 && !(t.cell[start_y * 8 + x] & 1)) --start_y;
   for (int y = start_y; y < end_y;) {
     const uint8_t c = t.cell[y * 8 + x];
     if (!(c & 1)) return true;
@@ -1135,9 +1141,7 @@ __device__ bool CrossesVertical(const TileState& t, int x, int start_y, int end_
 }
 
 __device__ float Cost(const SearchParams& p, const TileState& t, int s, int lx, int ly) {
-  const int f = FamilyOfStrategy(s);
-  const size_t blocks = static_cast<size_t>(p.blocks_x) * p.blocks_y;
-  const float v = p.costs[f * blocks + static_cast<size_t>(t.by0 + ly) * p.blocks_x + t.bx0 + lx];
+  const float v = t.family_cost[FamilyOfStrategy(s)][ly * 8 + lx];
   if (!(IsFinite(v) && v >= 0.0f)) RaiseError(p.error, kErrorInternal);
   return v;
 }
@@ -1174,18 +1178,21 @@ __device__ void TryMerge(const SearchParams& p, TileState& t, int s, int lx, int
   t.cost[ly * 8 + lx] = candidate;
 }
 
-// FindBestFirstLevelDivision (ac_strategy.cpp:406-589).
+// FindBestFirstLevelDivision (ac_strategy.cpp:406-589). kAligned: the square
+// is one of the aligned ones during the aligned passes, whose borders nothing
+// crosses.
+template <bool kAligned>
 __device__ void FirstLevelDivision(const SearchParams& p, TileState& t, int blocks, int lx,
                                    int ly) {
   const int half = blocks / 2;
-  if (CrossesHorizontal(t, lx, ly, lx + blocks) ||
-      CrossesHorizontal(t, lx, ly + blocks, lx + blocks) ||
-      CrossesVertical(t, lx, ly, ly + blocks) ||
-      CrossesVertical(t, lx + blocks, ly, ly + blocks)) {
+  if (!kAligned && (CrossesHorizontal<false>(t, lx, ly, lx + blocks) ||
+                    CrossesHorizontal<false>(t, lx, ly + blocks, lx + blocks) ||
+                    CrossesVertical<false>(t, lx, ly, ly + blocks) ||
+                    CrossesVertical<false>(t, lx + blocks, ly, ly + blocks))) {
     return;
   }
-  const bool allow_vertical = !CrossesVertical(t, lx + half, ly, ly + blocks);
-  const bool allow_horizontal = !CrossesHorizontal(t, lx, ly + half, lx + blocks);
+  const bool allow_vertical = !CrossesVertical<kAligned>(t, lx + half, ly, ly + blocks);
+  const bool allow_horizontal = !CrossesHorizontal<kAligned>(t, lx, ly + half, lx + blocks);
   float quadrant[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
   for (int dy = 0; dy < blocks; ++dy)
     for (int dx = 0; dx < blocks; ++dx)
@@ -1233,62 +1240,101 @@ __device__ void FirstLevelDivision(const SearchParams& p, TileState& t, int bloc
   }
 }
 
-// SearchTile (ac_strategy.cpp:591-773).
-__global__ void __launch_bounds__(64) SearchTileKernel(const __grid_constant__ SearchParams p) {
-  const uint32_t tile = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tile >= p.tiles_x * p.tiles_y) return;
-  TileState t;
-  const int tx = tile % p.tiles_x, ty = tile / p.tiles_x;
-  t.bx0 = tx * 8;
-  t.by0 = ty * 8;
-  t.tile_w = min(8, static_cast<int>(p.blocks_x) - t.bx0);
-  t.tile_h = min(8, static_cast<int>(p.blocks_y) - t.by0);
-  for (int i = 0; i < 64; ++i) {
-    t.cell[i] = Encode(kDct8, true);
-    t.cost[i] = 0.0f;
-    t.priority[i] = 0;
-  }
-  const int w = t.tile_w, h = t.tile_h;
-  for (int y = 0; y < h; ++y)
-    for (int x = 0; x < w; ++x) t.cost[y * 8 + x] = Cost(p, t, kDct8, x, y) * p.baseline_multiplier;
+// SearchTile (ac_strategy.cpp:591-773), one warp per tile.
+//
+// Bound: latency (a tile is a few hundred dependent decisions on 1.8 KB of
+// costs). The warp first copies the tile's seven cost planes into shared
+// memory with independent loads. The aligned passes then run one region per
+// lane: their regions are disjoint, no transform placed so far crosses a
+// boundary between them (aligned 2x2 and 4x4 squares only ever hold
+// transforms of their own), and each decision reads its own region's costs
+// only, so the order among them does not matter. The unaligned passes
+// overlap their predecessors and stay in raster order on lane 0. One thread
+// per tile with every cost a dependent global load took 241 us at 256x256
+// and 243 us at 2048x1536.
+constexpr int kSearchWarps = 4;
 
-  const int merge_strategy[4] = {kDct16x8, kDct8x16, kDct16x32, kDct32x16};
-  const uint8_t merge_priority[4] = {2, 2, 4, 4};
-  for (int m = 0; m < 4; ++m) {
-    const int s = merge_strategy[m];
-    const int cw = CoveredW(s), ch = CoveredH(s);
-    for (int y = 0; y + ch <= h; y += ch) {
-      for (int x = 0; x + cw <= w; x += cw) {
-        if (y + 3 < h && x + 3 < w) {
-          if (s == kDct16x32) {
-            if ((y | x) % 4 == 0) FirstLevelDivision(p, t, 4, x, y);
-            continue;
-          }
-          if (s == kDct32x16) continue;
-        }
-        if ((s == kDct16x32 && y % 4 != 0) || (s == kDct32x16 && x % 4 != 0)) continue;
-        if (y + 1 < h && x + 1 < w) {
-          if (s == kDct8x16) {
-            if ((y | x) % 2 == 0) FirstLevelDivision(p, t, 2, x, y);
-            continue;
-          }
-          if (s == kDct16x8) continue;
-        }
-        if ((s == kDct8x16 && y % 2 == 1) || (s == kDct16x8 && x % 2 == 1)) continue;
-        TryMerge(p, t, s, x, y, merge_priority[m]);
-      }
+__global__ void __launch_bounds__(32 * kSearchWarps)
+SearchTileKernel(const __grid_constant__ SearchParams p) {
+  __shared__ TileState states[kSearchWarps];
+  const uint32_t tile = blockIdx.x * kSearchWarps + threadIdx.x / 32;
+  if (tile >= p.tiles_x * p.tiles_y) return;
+  const int lane = threadIdx.x % 32;
+  TileState& t = states[threadIdx.x / 32];
+  const int bx0 = (tile % p.tiles_x) * 8, by0 = (tile / p.tiles_x) * 8;
+  const int w = min(8, static_cast<int>(p.blocks_x) - bx0);
+  const int h = min(8, static_cast<int>(p.blocks_y) - by0);
+  const size_t blocks = static_cast<size_t>(p.blocks_x) * p.blocks_y;
+  float loaded[kFamilyCount][2];
+#pragma unroll
+  for (int f = 0; f < kFamilyCount; ++f) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int x = lane % 8, y = lane / 8 + 4 * q;
+      loaded[f][q] = x < w && y < h ? p.costs[f * blocks +
+                                              static_cast<size_t>(by0 + y) * p.blocks_x + bx0 + x]
+                                    : 0.0f;
     }
   }
-  for (int y = 0; y + 1 < h; ++y)
-    for (int x = 0; x + 1 < w; ++x)
-      if ((y | x) % 2 != 0) FirstLevelDivision(p, t, 2, x, y);
-  for (int y = 0; y + 3 < h; y += p.dct32_step)
-    for (int x = 0; x + 3 < w; x += p.dct32_step)
-      if ((y | x) % 4 != 0) FirstLevelDivision(p, t, 4, x, y);
+  if (lane == 0) {
+    t.tile_w = w;
+    t.tile_h = h;
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int i = lane + 32 * q;
+#pragma unroll
+    for (int f = 0; f < kFamilyCount; ++f) t.family_cost[f][i] = loaded[f][q];
+    t.cell[i] = Encode(kDct8, true);
+    t.priority[i] = 0;
+    t.cost[i] = i % 8 < w && i / 8 < h ? Cost(p, t, kDct8, i % 8, i / 8) * p.baseline_multiplier
+                                       : 0.0f;
+  }
+  __syncwarp();
 
-  for (int y = 0; y < h; ++y)
-    for (int x = 0; x < w; ++x)
-      p.cells[static_cast<size_t>(t.by0 + y) * p.blocks_x + t.bx0 + x] = t.cell[y * 8 + x];
+  // Two-block merges: each aligned 2x2 square that fits divides itself, and
+  // the odd last column / row of a partial tile merges in pairs.
+  if (lane < 16) {
+    const int x = (lane % 4) * 2, y = (lane / 4) * 2;
+    if (x + 1 < w && y + 1 < h) {
+      FirstLevelDivision<true>(p, t, 2, x, y);
+    } else if (x + 1 == w && y + 1 < h) {
+      TryMerge(p, t, kDct16x8, x, y, 2);
+    } else if (x + 1 < w && y + 1 == h) {
+      TryMerge(p, t, kDct8x16, x, y, 2);
+    }
+  }
+  __syncwarp();
+  // Four-block merges likewise over the aligned 4x4 squares; where fewer than
+  // four rows (columns) remain, a 4x2 (2x4) merge.
+  if (lane < 4) {
+    const int x = (lane % 2) * 4, y = (lane / 2) * 4;
+    if (x + 3 < w && y + 3 < h) {
+      FirstLevelDivision<true>(p, t, 4, x, y);
+    } else if (x + 3 < w && y + 1 < h) {
+      TryMerge(p, t, kDct16x32, x, y, 4);
+    } else if (x + 1 < w && y + 3 < h) {
+      TryMerge(p, t, kDct32x16, x, y, 4);
+    }
+  }
+  __syncwarp();
+  if (lane == 0) {
+    for (int y = 0; y + 1 < h; ++y)
+      for (int x = 0; x + 1 < w; ++x)
+        if ((y | x) % 2 != 0) FirstLevelDivision<false>(p, t, 2, x, y);
+    for (int y = 0; y + 3 < h; y += p.dct32_step)
+      for (int x = 0; x + 3 < w; x += p.dct32_step)
+        if ((y | x) % 4 != 0) FirstLevelDivision<false>(p, t, 4, x, y);
+  }
+  __syncwarp();
+
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int x = lane % 8, y = lane / 8 + 4 * q;
+    if (x < w && y < h) {
+      p.cells[static_cast<size_t>(by0 + y) * p.blocks_x + bx0 + x] = t.cell[y * 8 + x];
+    }
+  }
 }
 
 template <int W, int H, typename Acc = double>
@@ -1483,7 +1529,7 @@ int LaunchAcStrategySearch(const float* costs, size_t pw, size_t ph, float targe
   p.cells = cells;
   p.error = error;
   const unsigned tiles = p.tiles_x * p.tiles_y;
-  SearchTileKernel<<<(tiles + 63) / 64, 64, 0, stream>>>(p);
+  SearchTileKernel<<<(tiles + kSearchWarps - 1) / kSearchWarps, 32 * kSearchWarps, 0, stream>>>(p);
   return CheckLaunch("ac_strategy search");
 }
 
