@@ -93,65 +93,102 @@ __global__ void GatherKernel(const __grid_constant__ GatherParams p) {
 }
 
 // ---------------------------------------------------------------------------
-// Forward convolution: one thread per output pixel, all 32 output channels.
+// Forward convolution (SIMT, the training step's): 128 threads compute 128
+// output pixels x 32 channels, a thread 4 pixels x 8 channels.
+//
+// Bound: FP32 issue (9216 multiply-adds per pixel at 32 input channels). The
+// 4 x 8 register tile makes every 16-byte weight load feed 16 multiply-adds;
+// one pixel x 32 channels per thread fed 4 and waited for shared memory (63
+// us on average per 32-channel layer at 256 tiles, 53 now). An output's
+// terms keep their order (bias, then taps, then input channels).
+
+constexpr int kConvPixels = 4;  // pixels per thread
+constexpr int kConvOut = 8;     // channels per thread
+constexpr int kConvThreads = 128;
+constexpr int kConvGroups = kCnnC / kConvOut;              // channel groups
+constexpr int kConvLanes = kConvThreads / kConvGroups;     // pixel lanes
+constexpr int kConvTile = kConvLanes * kConvPixels;        // pixels per CTA
+
+// acc[j][k] += x[j] * w[k] for the thread's pixels and channels.
+__device__ __forceinline__ void ConvAccumulate(const float (&x)[kConvPixels], const float* w,
+                                               float (&acc)[kConvPixels][kConvOut]) {
+  const float4 w0 = reinterpret_cast<const float4*>(w)[0];
+  const float4 w1 = reinterpret_cast<const float4*>(w)[1];
+  const float wk[kConvOut] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+  for (int j = 0; j < kConvPixels; ++j) {
+#pragma unroll
+    for (int k = 0; k < kConvOut; ++k) acc[j][k] = fmaf(wk[k], x[j], acc[j][k]);
+  }
+}
 
 template <int CIN>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kConvThreads)
 ConvForwardKernel(const __nv_bfloat16* in, const float* params, int layer, int n,
                   __nv_bfloat16* out) {
+  constexpr int kStep = CIN < 8 ? CIN : 8;  // input channels per load
   const LayerShape L = Layer(layer);
   __shared__ __align__(16) float ws[9 * CIN * kCnnC];
-  __shared__ float bs[kCnnC];
   for (int i = threadIdx.x; i < 9 * CIN * kCnnC; i += blockDim.x) {
     const int co = i % kCnnC, ci = (i / kCnnC) % CIN, tap = i / (kCnnC * CIN);
     ws[i] = RoundBf16(params[L.w_offset + (co * 9 + tap) * CIN + ci]);
   }
-  if (threadIdx.x < kCnnC) bs[threadIdx.x] = params[L.b_offset + threadIdx.x];
   __syncthreads();
-  const size_t pixel = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const size_t per_tile = static_cast<size_t>(L.out_size) * L.out_size;
-  if (pixel >= static_cast<size_t>(n) * per_tile) return;
-  const size_t t = pixel / per_tile;
-  const int oy = static_cast<int>(pixel % per_tile) / L.out_size;
-  const int ox = static_cast<int>(pixel % per_tile) % L.out_size;
-  float acc[kCnnC];
+  const int co0 = (threadIdx.x % kConvGroups) * kConvOut;
+  const uint32_t per_tile = L.out_size * L.out_size;
+  const uint32_t total = n * per_tile;
+  const uint32_t pixel0 = blockIdx.x * kConvTile + threadIdx.x / kConvGroups;
+  int iy0[kConvPixels], ix0[kConvPixels];  // top-left tap
+  const __nv_bfloat16* base[kConvPixels];
+  float acc[kConvPixels][kConvOut];
 #pragma unroll
-  for (int co = 0; co < kCnnC; ++co) acc[co] = bs[co];
+  for (int j = 0; j < kConvPixels; ++j) {
+    const uint32_t pixel = min(pixel0 + j * kConvLanes, total - 1);
+    const uint32_t t = pixel / per_tile, r = pixel % per_tile;
+    iy0[j] = static_cast<int>(r) / L.out_size * L.stride - 1;
+    ix0[j] = static_cast<int>(r) % L.out_size * L.stride - 1;
+    base[j] = in + static_cast<size_t>(t) * L.in_size * L.in_size * CIN;
+#pragma unroll
+    for (int k = 0; k < kConvOut; ++k) acc[j][k] = params[L.b_offset + co0 + k];
+  }
   for (int tap = 0; tap < 9; ++tap) {
-    const int iy = oy * L.stride + tap / 3 - 1, ix = ox * L.stride + tap % 3 - 1;
-    if (iy < 0 || iy >= L.in_size || ix < 0 || ix >= L.in_size) continue;
-    const __nv_bfloat16* x = in + ((t * L.in_size + iy) * L.in_size + ix) * CIN;
-    for (int c8 = 0; c8 < CIN; c8 += (CIN < 8 ? CIN : 8)) {
-      float xv[CIN < 8 ? CIN : 8];
-      if constexpr (CIN >= 8) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(x + c8);
-        const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&raw);
+    const __nv_bfloat16* x[kConvPixels];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) xv[k] = __bfloat162float(h[k]);
-      } else {
+    for (int j = 0; j < kConvPixels; ++j) {
+      const int iy = iy0[j] + tap / 3, ix = ix0[j] + tap % 3;
+      const bool inside = iy >= 0 && iy < L.in_size && ix >= 0 && ix < L.in_size;
+      x[j] = inside ? base[j] + (iy * L.in_size + ix) * CIN : nullptr;
+    }
 #pragma unroll
-        for (int k = 0; k < CIN; ++k) xv[k] = __bfloat162float(x[k]);
+    for (int c = 0; c < CIN; c += kStep) {
+      __align__(16) __nv_bfloat16 h[kConvPixels][kStep];
+#pragma unroll
+      for (int j = 0; j < kConvPixels; ++j) {
+        if constexpr (CIN >= 8) {
+          *reinterpret_cast<uint4*>(h[j]) =
+            x[j] != nullptr ? *reinterpret_cast<const uint4*>(x[j] + c) : make_uint4(0, 0, 0, 0);
+        } else {
+          *reinterpret_cast<uint2*>(h[j]) =
+            x[j] != nullptr ? *reinterpret_cast<const uint2*>(x[j]) : make_uint2(0, 0);
+        }
       }
 #pragma unroll
-      for (int k = 0; k < (CIN < 8 ? CIN : 8); ++k) {
-        const float4* w4 = reinterpret_cast<const float4*>(ws + (tap * CIN + c8 + k) * kCnnC);
-#pragma unroll
-        for (int q = 0; q < kCnnC / 4; ++q) {
-          const float4 w = w4[q];
-          acc[4 * q + 0] = fmaf(w.x, xv[k], acc[4 * q + 0]);
-          acc[4 * q + 1] = fmaf(w.y, xv[k], acc[4 * q + 1]);
-          acc[4 * q + 2] = fmaf(w.z, xv[k], acc[4 * q + 2]);
-          acc[4 * q + 3] = fmaf(w.w, xv[k], acc[4 * q + 3]);
-        }
+      for (int k = 0; k < kStep; ++k) {
+        const float xv[kConvPixels] = {__bfloat162float(h[0][k]), __bfloat162float(h[1][k]),
+                                       __bfloat162float(h[2][k]), __bfloat162float(h[3][k])};
+        ConvAccumulate(xv, ws + (tap * CIN + c + k) * kCnnC + co0, acc);
       }
     }
   }
-  __align__(16) __nv_bfloat16 o[kCnnC];
 #pragma unroll
-  for (int co = 0; co < kCnnC; ++co) o[co] = __float2bfloat16_rn(fmaxf(acc[co], 0.0f));
-  uint4* dst = reinterpret_cast<uint4*>(out + pixel * kCnnC);
+  for (int j = 0; j < kConvPixels; ++j) {
+    if (pixel0 + j * kConvLanes >= total) break;
+    __align__(16) __nv_bfloat16 o[kConvOut];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) dst[q] = reinterpret_cast<const uint4*>(o)[q];
+    for (int k = 0; k < kConvOut; ++k) o[k] = __float2bfloat16_rn(fmaxf(acc[j][k], 0.0f));
+    *reinterpret_cast<uint4*>(out + static_cast<size_t>(pixel0 + j * kConvLanes) * kCnnC + co0) =
+      *reinterpret_cast<const uint4*>(o);
+  }
 }
 
 // The same convolution as implicit GEMMs on the fifth-generation tensor
@@ -361,170 +398,246 @@ __global__ void LossKernel(const float* head, const uint8_t* labels, const float
   if (threadIdx.x == 0) partial[blockIdx.x] = sums[0];
 }
 
+// One warp: lane i sums partials i, i + 32, ..., then the lanes' sums.
 __global__ void LossReduceKernel(const float* partial, int count, int n, float* loss) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
   float s = 0.0f;
-  for (int i = 0; i < count; ++i) s += partial[i];
-  *loss = s / (static_cast<float>(n) * 64.0f);
+  for (int i = threadIdx.x; i < count; i += 32) s += partial[i];
+  s = WarpSum(s);
+  if (threadIdx.x == 0) *loss = s / (static_cast<float>(n) * 64.0f);
 }
 
-// Head backward: input gradient of the conv4 output (zero off the centre)
-// and per-chunk weight-gradient partials.
-__global__ void HeadBackwardInputKernel(const float* dhead, const float* params, int n,
-                                        float* da4) {
-  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= static_cast<size_t>(n) * 100) return;
-  const size_t t = i / 100;
-  const int cy = static_cast<int>(i % 100) / 10, cx = static_cast<int>(i % 100) % 10;
-  float* d = da4 + i * kCnnC;
-  if (cy < 1 || cy > 8 || cx < 1 || cx > 8) {
-    for (int c = 0; c < kCnnC; ++c) d[c] = 0.0f;
-    return;
-  }
-  const float* g = dhead + (t * 64 + (cy - 1) * 8 + (cx - 1)) * kCnnHead;
-  for (int c = 0; c < kCnnC; ++c) {
-    float acc = 0.0f;
-    for (int k = 0; k < kCnnHead; ++k) acc = fmaf(RoundBf16(params[kCnnWh + k * kCnnC + c]), g[k], acc);
-    d[c] = acc;
-  }
-}
-
-constexpr int kHeadChunk = 256;  // cells per partial
-
-__global__ void HeadBackwardWeightKernel(const float* dhead, const __nv_bfloat16* a4, int n,
-                                         float* partial) {
-  // One CTA per chunk of cells; thread j < 28 * 33 owns dWh[k][c] (c < 32)
-  // or dbh[k] (c == 32).
-  const int j = threadIdx.x;
-  if (j >= kCnnHead * (kCnnC + 1)) return;
-  const int k = j / (kCnnC + 1), c = j % (kCnnC + 1);
-  const size_t begin = static_cast<size_t>(blockIdx.x) * kHeadChunk;
-  const size_t end = min(begin + kHeadChunk, static_cast<size_t>(n) * 64);
-  float acc = 0.0f;
-  for (size_t i = begin; i < end; ++i) {
-    const size_t t = i / 64;
-    const int cell = static_cast<int>(i % 64);
-    const float g = dhead[i * kCnnHead + k];
-    const float x = c == kCnnC ? 1.0f
-                               : __bfloat162float(a4[((t * 10 + cell / 8 + 1) * 10 + cell % 8 + 1) *
-                                                        kCnnC + c]);
-    acc = fmaf(g, x, acc);
-  }
-  partial[static_cast<size_t>(blockIdx.x) * kCnnHead * (kCnnC + 1) + j] = acc;
-}
-
-// Convolution backward. dz = dy * (y > 0) is formed on the fly.
-constexpr int kConvChunk = 512;  // output pixels per weight-gradient partial
-
-template <int CIN>
+// Head backward: gradient of conv4's pre-activation (its ReLU's mask
+// applied; zero off the centre), one warp lane per channel.
 __global__ void __launch_bounds__(256)
-ConvBackwardWeightKernel(const float* dy, const __nv_bfloat16* y, const __nv_bfloat16* x,
-                         int layer, int n, float* partial) {
-  // Thread (cg, pg): output channels 4cg..4cg+3 x patch entries 9pg..9pg+8
-  // (patch entry = tap * CIN + ci); thread 0..31 also sums the bias of its co.
-  constexpr int kPatch = 9 * CIN;
-  constexpr int kGroups = kPatch / 9;
-  const LayerShape L = Layer(layer);
-  __shared__ float dz[kCnnC];
-  __shared__ float patch[kPatch];
-  const int tid = threadIdx.x;
-  const int cg = tid / kGroups, pg = tid % kGroups;
-  const bool active = tid < 8 * kGroups;
-  float acc[4][9] = {};
-  float bias = 0.0f;
-  const size_t per_tile = static_cast<size_t>(L.out_size) * L.out_size;
-  const size_t total = static_cast<size_t>(n) * per_tile;
-  const size_t begin = static_cast<size_t>(blockIdx.x) * kConvChunk;
-  const size_t end = min(begin + kConvChunk, total);
-  for (size_t pixel = begin; pixel < end; ++pixel) {
-    const size_t t = pixel / per_tile;
-    const int oy = static_cast<int>(pixel % per_tile) / L.out_size;
-    const int ox = static_cast<int>(pixel % per_tile) % L.out_size;
-    __syncthreads();
-    if (tid < kCnnC) {
-      const float yv = __bfloat162float(y[pixel * kCnnC + tid]);
-      dz[tid] = yv > 0.0f ? dy[pixel * kCnnC + tid] : 0.0f;
-    }
-    for (int e = tid; e < kPatch; e += blockDim.x) {
-      const int tap = e / CIN, ci = e % CIN;
-      const int iy = oy * L.stride + tap / 3 - 1, ix = ox * L.stride + tap % 3 - 1;
-      patch[e] = (iy < 0 || iy >= L.in_size || ix < 0 || ix >= L.in_size)
-                   ? 0.0f
-                   : __bfloat162float(x[((t * L.in_size + iy) * L.in_size + ix) * CIN + ci]);
-    }
-    __syncthreads();
-    if (active) {
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const float g = dz[4 * cg + a];
-#pragma unroll
-        for (int b = 0; b < 9; ++b) acc[a][b] = fmaf(g, patch[9 * pg + b], acc[a][b]);
-      }
-    }
-    if (tid < kCnnC) bias += dz[tid];
-  }
-  float* out = partial + static_cast<size_t>(blockIdx.x) * (kCnnC * kPatch + kCnnC);
-  if (active) {
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 9; ++b) {
-        const int co = 4 * cg + a, e = 9 * pg + b;
-        // Stored in the parameter layout [co][tap][ci].
-        out[co * kPatch + e] = acc[a][b];
-      }
-  }
-  if (tid < kCnnC) out[kCnnC * kPatch + tid] = bias;
-}
-
-template <int CIN>
-__global__ void __launch_bounds__(128)
-ConvBackwardInputKernel(const float* dy, const __nv_bfloat16* y, const float* params, int layer,
-                        int n, float* dx) {
-  const LayerShape L = Layer(layer);
-  __shared__ __align__(16) float ws[9 * CIN * kCnnC];
-  for (int i = threadIdx.x; i < 9 * CIN * kCnnC; i += blockDim.x) {
-    const int co = i % kCnnC, ci = (i / kCnnC) % CIN, tap = i / (kCnnC * CIN);
-    ws[i] = RoundBf16(params[L.w_offset + (co * 9 + tap) * CIN + ci]);
+HeadBackwardInputKernel(const float* dhead, const float* params, const __nv_bfloat16* a4, int n,
+                        float* dz4) {
+  __shared__ float wh[kCnnHead * kCnnC];
+  for (int i = threadIdx.x; i < kCnnHead * kCnnC; i += blockDim.x) {
+    wh[i] = RoundBf16(params[kCnnWh + i]);
   }
   __syncthreads();
-  const size_t pixel = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const size_t per_tile = static_cast<size_t>(L.in_size) * L.in_size;
-  if (pixel >= static_cast<size_t>(n) * per_tile) return;
-  const size_t t = pixel / per_tile;
-  const int iy = static_cast<int>(pixel % per_tile) / L.in_size;
-  const int ix = static_cast<int>(pixel % per_tile) % L.in_size;
-  float acc[CIN];
+  const size_t i = static_cast<size_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32;
+  if (i >= static_cast<size_t>(n) * 100) return;
+  const int c = threadIdx.x % 32;
+  const size_t t = i / 100;
+  const int cy = static_cast<int>(i % 100) / 10, cx = static_cast<int>(i % 100) % 10;
+  float acc = 0.0f;
+  if (cy >= 1 && cy <= 8 && cx >= 1 && cx <= 8) {
+    const float* g = dhead + (t * 64 + (cy - 1) * 8 + (cx - 1)) * kCnnHead;
 #pragma unroll
-  for (int ci = 0; ci < CIN; ++ci) acc[ci] = 0.0f;
-  for (int tap = 0; tap < 9; ++tap) {
-    const int ny = iy + 1 - tap / 3, nx = ix + 1 - tap % 3;
-    if (ny < 0 || nx < 0 || ny % L.stride || nx % L.stride) continue;
-    const int oy = ny / L.stride, ox = nx / L.stride;
-    if (oy >= L.out_size || ox >= L.out_size) continue;
-    const size_t o = (t * L.out_size + oy) * L.out_size + ox;
-    float dz[kCnnC];
-#pragma unroll
-    for (int co = 0; co < kCnnC; ++co) {
-      const float yv = __bfloat162float(y[o * kCnnC + co]);
-      dz[co] = yv > 0.0f ? dy[o * kCnnC + co] : 0.0f;
+    for (int k = 0; k < kCnnHead; ++k) acc = fmaf(wh[k * kCnnC + c], g[k], acc);
+  }
+  dz4[i * kCnnC + c] = __bfloat162float(a4[i * kCnnC + c]) > 0.0f ? acc : 0.0f;
+}
+
+// One CTA per tile: thread j < 28 * 33 owns dWh[k][c] (c < 32) or dbh[k]
+// (c == 32) over the tile's 64 cells, staged in shared memory.
+__global__ void __launch_bounds__(kCnnHead * (kCnnC + 1))
+HeadBackwardWeightKernel(const float* dhead, const __nv_bfloat16* a4, float* partial) {
+  __shared__ float g[64 * kCnnHead];
+  __shared__ float x[64 * (kCnnC + 1)];  // the bias's input 1 in the last column
+  const size_t t = blockIdx.x;
+  for (int i = threadIdx.x; i < 64 * kCnnHead; i += blockDim.x) {
+    g[i] = dhead[t * 64 * kCnnHead + i];
+  }
+  for (int i = threadIdx.x; i < 64 * (kCnnC + 1); i += blockDim.x) {
+    const int cell = i / (kCnnC + 1), c = i % (kCnnC + 1);
+    x[i] = c == kCnnC ? 1.0f
+                      : __bfloat162float(a4[((t * 10 + cell / 8 + 1) * 10 + cell % 8 + 1) * kCnnC +
+                                            c]);
+  }
+  __syncthreads();
+  const int j = threadIdx.x, k = j / (kCnnC + 1), c = j % (kCnnC + 1);
+  float acc = 0.0f;
+#pragma unroll 8
+  for (int cell = 0; cell < 64; ++cell) {
+    acc = fmaf(g[cell * kCnnHead + k], x[cell * (kCnnC + 1) + c], acc);
+  }
+  partial[t * kCnnHead * (kCnnC + 1) + j] = acc;
+}
+
+// Weight gradients dW[co][tap][ci] = sum over output pixels of dz[co] *
+// x[tap's pixel][ci], and the bias's sum of dz.
+//
+// Bound: FP32 issue (9216 multiply-adds per output pixel at 32 input
+// channels). A unit is one output row of one tile; CTAs walk their share of
+// the units, so each keeps one set of partial sums. Per unit the CTA stages
+// dz and the three input rows (with their zero borders) as FP32 in shared
+// memory; a thread owns 8 output channels x 1 input channel x 9 taps, so the
+// two 16-byte loads of dz and the 3 to 9 of x (the taps that the previous
+// pixel did not share) feed 72 multiply-adds. With 32 input channels four
+// threads cover the output channels and the CTA's two halves take alternate
+// pixels; with 4 input channels the CTA's 16 groups of 16 threads do. The
+// groups' sums are added in a fixed order at the end. One pixel at a time
+// between two barriers, 13 scalar shared loads per 36 multiply-adds, took
+// 717 us on average per 32-channel layer and 1321 us for the first at 256
+// tiles; 52 and 117 us now.
+constexpr int kConvGradThreads = 256;
+constexpr int kConvGradOut = 8;
+
+template <int CIN>
+struct ConvGradLayout {
+  static constexpr int kGroupThreads = (kCnnC / kConvGradOut) * CIN;
+  static constexpr int kGroups = kConvGradThreads / kGroupThreads;
+  static constexpr int kPatch = 9 * CIN;
+  static constexpr int kWidth = kCnnC * kPatch + kCnnC;  // weights, then biases
+  __host__ __device__ static constexpr int RowFloats(int in_size) { return (in_size + 2) * CIN; }
+  static constexpr size_t SharedBytes(int in_size, int out_size) {
+    const size_t staged = 3 * RowFloats(in_size) + out_size * kCnnC;
+    return sizeof(float) * (staged > kWidth ? staged : kWidth);
+  }
+};
+
+template <int CIN, int kStride>
+__global__ void __launch_bounds__(kConvGradThreads)
+ConvBackwardWeightKernel(const float* dz, const __nv_bfloat16* x, int layer, int n,
+                         float* partial) {
+  using G = ConvGradLayout<CIN>;
+  const LayerShape L = Layer(layer);
+  extern __shared__ __align__(16) float grad_smem[];
+  float* rows = grad_smem;                             // [3][in_size + 2][CIN]
+  float* grad = rows + 3 * G::RowFloats(L.in_size);    // [out_size][32]
+  const int tid = threadIdx.x;
+  const int group = tid / G::kGroupThreads, member = tid % G::kGroupThreads;
+  const int ci = member % CIN, co0 = member / CIN * kConvGradOut;
+  float acc[9][kConvGradOut] = {};
+  float bias = 0.0f;
+  const int units = n * L.out_size;
+  const int pairs = L.in_size * CIN / 2;  // two input channels per 32-bit load
+  for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+    const int t = unit / L.out_size, oy = unit % L.out_size;
+    __syncthreads();
+    for (int i = tid; i < 3 * pairs; i += kConvGradThreads) {
+      const int row = i / pairs, e = i % pairs;
+      const int iy = oy * kStride + row - 1;
+      uint32_t v = 0;
+      if (iy >= 0 && iy < L.in_size) {
+        v = *reinterpret_cast<const uint32_t*>(
+          x + (static_cast<size_t>(t) * L.in_size + iy) * L.in_size * CIN + 2 * e);
+      }
+      float* dst = rows + row * G::RowFloats(L.in_size) + CIN + 2 * e;
+      dst[0] = __uint_as_float(v << 16);
+      dst[1] = __uint_as_float(v & 0xFFFF0000u);
     }
+    for (int i = tid; i < 3 * 2 * CIN; i += kConvGradThreads) {
+      const int row = i / (2 * CIN), side = i / CIN % 2, c = i % CIN;
+      rows[row * G::RowFloats(L.in_size) + (side ? (L.in_size + 1) * CIN : 0) + c] = 0.0f;
+    }
+    const float4* src = reinterpret_cast<const float4*>(
+      dz + (static_cast<size_t>(t) * L.out_size + oy) * L.out_size * kCnnC);
+    for (int i = tid; i < L.out_size * kCnnC / 4; i += kConvGradThreads) {
+      reinterpret_cast<float4*>(grad)[i] = src[i];
+    }
+    __syncthreads();
+    for (int ox = group; ox < L.out_size; ox += G::kGroups) {
+      const float4 g0 = *reinterpret_cast<const float4*>(grad + ox * kCnnC + co0);
+      const float4 g1 = *reinterpret_cast<const float4*>(grad + ox * kCnnC + co0 + 4);
+      const float g[kConvGradOut] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
 #pragma unroll
-    for (int ci = 0; ci < CIN; ++ci) {
-      const float4* w4 = reinterpret_cast<const float4*>(ws + (tap * CIN + ci) * kCnnC);
+      for (int tap = 0; tap < 9; ++tap) {
+        const float v =
+          rows[tap / 3 * G::RowFloats(L.in_size) + (ox * kStride + tap % 3) * CIN + ci];
 #pragma unroll
-      for (int q = 0; q < kCnnC / 4; ++q) {
-        const float4 w = w4[q];
-        acc[ci] = fmaf(w.x, dz[4 * q + 0], acc[ci]);
-        acc[ci] = fmaf(w.y, dz[4 * q + 1], acc[ci]);
-        acc[ci] = fmaf(w.z, dz[4 * q + 2], acc[ci]);
-        acc[ci] = fmaf(w.w, dz[4 * q + 3], acc[ci]);
+        for (int k = 0; k < kConvGradOut; ++k) acc[tap][k] = fmaf(g[k], v, acc[tap][k]);
+      }
+    }
+    if (tid < kCnnC) {
+      for (int ox = 0; ox < L.out_size; ++ox) bias += grad[ox * kCnnC + tid];
+    }
+  }
+  // The groups' sums in group order, in the parameter layout [co][tap][ci].
+  for (int turn = 0; turn < G::kGroups; ++turn) {
+    __syncthreads();
+    if (group == turn) {
+#pragma unroll
+      for (int tap = 0; tap < 9; ++tap) {
+#pragma unroll
+        for (int k = 0; k < kConvGradOut; ++k) {
+          float* out = grad_smem + (co0 + k) * G::kPatch + tap * CIN + ci;
+          *out = turn == 0 ? acc[tap][k] : *out + acc[tap][k];
+        }
       }
     }
   }
-  float* d = dx + pixel * CIN;
+  __syncthreads();
+  float* out = partial + static_cast<size_t>(blockIdx.x) * G::kWidth;
+  for (int i = tid; i < kCnnC * G::kPatch; i += kConvGradThreads) out[i] = grad_smem[i];
+  if (tid < kCnnC) out[kCnnC * G::kPatch + tid] = bias;
+}
+
+// Input gradients, with the mask of the ReLU that produced the input: the
+// next layer's dz. 128 threads compute 128 input pixels x 32 channels, a
+// thread 4 pixels x 8 channels as in ConvForwardKernel. At stride 2 the taps
+// that reach a pixel depend on the parity of its row and column:
+// blockIdx.y is the parity class, so a CTA's pixels share their taps (1, 2,
+// 2 and 4 of the 9). One pixel x 32 channels per thread with its own taps
+// and the mask formed at every use took 207 us on average at 256 tiles, 64 now.
+template <int kStride>
+__global__ void __launch_bounds__(kConvThreads)
+ConvBackwardInputKernel(const float* dz, const __nv_bfloat16* x, const float* params, int layer,
+                        int n, float* dx) {
+  const LayerShape L = Layer(layer);
+  __shared__ __align__(16) float ws[9 * kCnnC * kCnnC];  // [tap][co][ci]
+  for (int i = threadIdx.x; i < 9 * kCnnC * kCnnC; i += blockDim.x) {
+    const int ci = i % kCnnC, tap = i / kCnnC % 9, co = i / (9 * kCnnC);
+    ws[(tap * kCnnC + co) * kCnnC + ci] = RoundBf16(params[L.w_offset + i]);
+  }
+  __syncthreads();
+  const int ci0 = (threadIdx.x % kConvGroups) * kConvOut;
+  const int py = blockIdx.y / kStride, px = blockIdx.y % kStride;  // parity class
+  const int side = L.in_size / kStride;
+  const uint32_t per_tile = side * side;
+  const uint32_t total = n * per_tile;
+  const uint32_t first = blockIdx.x * kConvTile + threadIdx.x / kConvGroups;
+  int iy[kConvPixels], ix[kConvPixels];
+  size_t tile[kConvPixels];
+  float acc[kConvPixels][kConvOut] = {};
 #pragma unroll
-  for (int ci = 0; ci < CIN; ++ci) d[ci] = acc[ci];
+  for (int j = 0; j < kConvPixels; ++j) {
+    const uint32_t i = min(first + j * kConvLanes, total - 1);
+    tile[j] = i / per_tile;
+    iy[j] = static_cast<int>(i % per_tile) / side * kStride + py;
+    ix[j] = static_cast<int>(i % per_tile) % side * kStride + px;
+  }
+  for (int tap = 0; tap < 9; ++tap) {
+    // Output pixels reached: (i + 1 - k) / stride where it divides.
+    if ((py + 1 - tap / 3) % kStride != 0 || (px + 1 - tap % 3) % kStride != 0) continue;
+    const float* g[kConvPixels];
+#pragma unroll
+    for (int j = 0; j < kConvPixels; ++j) {
+      const int ny = iy[j] + 1 - tap / 3, nx = ix[j] + 1 - tap % 3;
+      const int oy = ny / kStride, ox = nx / kStride;
+      const bool inside = ny >= 0 && nx >= 0 && oy < L.out_size && ox < L.out_size;
+      g[j] = inside ? dz + ((tile[j] * L.out_size + oy) * L.out_size + ox) * kCnnC : nullptr;
+    }
+#pragma unroll 2
+    for (int co = 0; co < kCnnC; co += 4) {
+      __align__(16) float v[kConvPixels][4];
+#pragma unroll
+      for (int j = 0; j < kConvPixels; ++j) {
+        *reinterpret_cast<float4*>(v[j]) = g[j] != nullptr
+                                             ? *reinterpret_cast<const float4*>(g[j] + co)
+                                             : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float gv[kConvPixels] = {v[0][k], v[1][k], v[2][k], v[3][k]};
+        ConvAccumulate(gv, ws + (tap * kCnnC + co + k) * kCnnC + ci0, acc);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kConvPixels; ++j) {
+    if (first + j * kConvLanes >= total) break;
+    const size_t at = ((tile[j] * L.in_size + iy[j]) * L.in_size + ix[j]) * kCnnC + ci0;
+    const uint4 raw = *reinterpret_cast<const uint4*>(x + at);
+    const __nv_bfloat16* xv = reinterpret_cast<const __nv_bfloat16*>(&raw);
+    __align__(16) float d[kConvOut];
+#pragma unroll
+    for (int k = 0; k < kConvOut; ++k) d[k] = __bfloat162float(xv[k]) > 0.0f ? acc[j][k] : 0.0f;
+    reinterpret_cast<float4*>(dx + at)[0] = reinterpret_cast<const float4*>(d)[0];
+    reinterpret_cast<float4*>(dx + at)[1] = reinterpret_cast<const float4*>(d)[1];
+  }
 }
 
 __global__ void HeadGradScatterKernel(const float* reduced, float* grads) {
@@ -538,13 +651,27 @@ __global__ void HeadGradScatterKernel(const float* reduced, float* grads) {
   }
 }
 
-// Fixed-order sum of `chunks` partial rows of `width` values into grads.
-__global__ void ReducePartialsKernel(const float* partial, int chunks, int width,
-                                     float* grads) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= width) return;
+// Fixed-order sum of `chunks` partial rows of `width` values into grads: 32
+// columns x 8 slices of the rows per CTA, then the slices in order.
+constexpr int kReduceSlices = 8;
+
+__global__ void __launch_bounds__(32 * kReduceSlices)
+ReducePartialsKernel(const float* partial, int chunks, int width, float* grads) {
+  __shared__ float sums[kReduceSlices][32];
+  const int lane = threadIdx.x % 32, slice = threadIdx.x / 32;
+  const int j = blockIdx.x * 32 + lane;
   float s = 0.0f;
-  for (int c = 0; c < chunks; ++c) s += partial[static_cast<size_t>(c) * width + j];
+  if (j < width) {
+#pragma unroll 8
+    for (int c = slice; c < chunks; c += kReduceSlices) {
+      s += partial[static_cast<size_t>(c) * width + j];
+    }
+  }
+  sums[slice][lane] = s;
+  __syncthreads();
+  if (slice != 0 || j >= width) return;
+#pragma unroll
+  for (int k = 1; k < kReduceSlices; ++k) s += sums[k][lane];
   grads[j] = s;
 }
 
@@ -695,12 +822,13 @@ int CnnForward(const float* params, const CnnActivations& a, int n, cudaStream_t
   for (int l = 0; l < 4; ++l) {
     const LayerShape L = Layer(l);
     const size_t pixels = static_cast<size_t>(n) * L.out_size * L.out_size;
-    const unsigned grid = static_cast<unsigned>((pixels + 127) / 128);
+    const unsigned grid = static_cast<unsigned>((pixels + kConvTile - 1) / kConvTile);
     if (l == 0) {
-      ConvForwardKernel<kCnnInChannels><<<grid, 128, 0, stream>>>(a.act[0], params, 0, n,
-                                                                  a.act[1]);
+      ConvForwardKernel<kCnnInChannels><<<grid, kConvThreads, 0, stream>>>(a.act[0], params, 0, n,
+                                                                           a.act[1]);
     } else {
-      ConvForwardKernel<kCnnC><<<grid, 128, 0, stream>>>(a.act[l], params, l, n, a.act[l + 1]);
+      ConvForwardKernel<kCnnC><<<grid, kConvThreads, 0, stream>>>(a.act[l], params, l, n,
+                                                                  a.act[l + 1]);
     }
   }
   const size_t cells = static_cast<size_t>(n) * 64;
@@ -718,12 +846,37 @@ int CnnPropose(const float* head, int n, size_t blocks_x, size_t blocks_y, uint8
   return CheckLaunch("cnn propose");
 }
 
+// Rows of weight-gradient partial sums that the training scratch holds.
+size_t ConvPartialRows(int n) { return (static_cast<size_t>(n) * 40 * 40 + 511) / 512; }
+
+// Weight-gradient partials of layer `layer`: as many CTAs as the device runs
+// at once (two per SM), the scratch holds rows for, and there are units.
+template <int CIN, int kStride>
+int LaunchConvWeights(const float* dz, const __nv_bfloat16* x, int layer, int n, float* partial,
+                      int* width, int* chunks, cudaStream_t stream) {
+  using G = ConvGradLayout<CIN>;
+  const LayerShape L = Layer(layer);
+  int device = 0, sms = 0;
+  int status = CheckCuda(cudaGetDevice(&device), "cnn device");
+  if (status != GJXL_B200_OK) return status;
+  status = CheckCuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device),
+                     "cnn SM count");
+  if (status != GJXL_B200_OK) return status;
+  const size_t units = static_cast<size_t>(n) * L.out_size;
+  *chunks = static_cast<int>(
+    std::min({static_cast<size_t>(2 * sms), units, ConvPartialRows(n)}));
+  *width = G::kWidth;
+  ConvBackwardWeightKernel<CIN, kStride>
+    <<<*chunks, kConvGradThreads, G::SharedBytes(L.in_size, L.out_size), stream>>>(
+      dz, x, layer, n, partial);
+  return CheckLaunch("cnn weight gradients");
+}
+
 size_t CnnTrainScratchBytes(int n) {
   // dhead, two gradient planes of the largest activation, partials.
   const size_t dhead = static_cast<size_t>(n) * 64 * kCnnHead * 4;
   const size_t plane = static_cast<size_t>(n) * 40 * 40 * kCnnC * 4;
-  const size_t l1_chunks = (static_cast<size_t>(n) * 40 * 40 + kConvChunk - 1) / kConvChunk;
-  const size_t partial = l1_chunks * (kCnnC * 9 * kCnnC + kCnnC) * 4;
+  const size_t partial = ConvPartialRows(n) * (kCnnC * 9 * kCnnC + kCnnC) * 4;
   const size_t loss = ((static_cast<size_t>(n) * 64 + 255) / 256 + 1) * 4;
   return Align(dhead, 256) + 2 * Align(plane, 256) + Align(partial, 256) + Align(loss, 256);
 }
@@ -739,51 +892,56 @@ int CnnTrainStep(const float* params, const CnnActivations& a, int n, const uint
   p += Align(plane, 256);
   float* g1 = reinterpret_cast<float*>(p);
   p += Align(plane, 256);
-  const size_t l1_chunks = (static_cast<size_t>(n) * 40 * 40 + kConvChunk - 1) / kConvChunk;
   float* partial = reinterpret_cast<float*>(p);
-  p += Align(l1_chunks * (kCnnC * 9 * kCnnC + kCnnC) * 4, 256);
+  p += Align(ConvPartialRows(n) * (kCnnC * 9 * kCnnC + kCnnC) * 4, 256);
   float* loss_partial = reinterpret_cast<float*>(p);
 
   const size_t cells = static_cast<size_t>(n) * 64;
   const unsigned loss_blocks = static_cast<unsigned>((cells + 255) / 256);
   LossKernel<<<loss_blocks, 256, 0, stream>>>(a.head, labels, targets, weights, n, qf_weight,
                                               dhead, loss_partial);
-  LossReduceKernel<<<1, 1, 0, stream>>>(loss_partial, static_cast<int>(loss_blocks), n, loss);
+  LossReduceKernel<<<1, 32, 0, stream>>>(loss_partial, static_cast<int>(loss_blocks), n, loss);
   // Head.
-  const unsigned head_chunks = static_cast<unsigned>((cells + kHeadChunk - 1) / kHeadChunk);
-  HeadBackwardWeightKernel<<<head_chunks, kCnnHead * (kCnnC + 1), 0, stream>>>(dhead, a.act[4],
-                                                                                n, partial);
-  // Partials are [chunk][k][c + bias]; reduce, then scatter into Wh / bh.
-  ReducePartialsKernel<<<(kCnnHead * (kCnnC + 1) + 127) / 128, 128, 0, stream>>>(
-    partial, static_cast<int>(head_chunks), kCnnHead * (kCnnC + 1), g1);
+  constexpr int kHeadWidth = kCnnHead * (kCnnC + 1);
+  HeadBackwardWeightKernel<<<n, kHeadWidth, 0, stream>>>(dhead, a.act[4], partial);
+  // Partials are [tile][k][c + bias]; reduce, then scatter into Wh / bh.
+  ReducePartialsKernel<<<(kHeadWidth + 31) / 32, 32 * kReduceSlices, 0, stream>>>(
+    partial, n, kHeadWidth, g1);
   // g1 holds [k][c | bias]; scatter into the parameter layout.
-  HeadGradScatterKernel<<<(kCnnHead * (kCnnC + 1) + 127) / 128, 128, 0, stream>>>(g1, grads);
-  HeadBackwardInputKernel<<<static_cast<unsigned>((static_cast<size_t>(n) * 100 + 127) / 128),
-                            128, 0, stream>>>(dhead, params, n, g0);
-  // Convolutions, last to first. g_in holds dL/d(output of layer l).
+  HeadGradScatterKernel<<<(kHeadWidth + 127) / 128, 128, 0, stream>>>(g1, grads);
+  HeadBackwardInputKernel<<<static_cast<unsigned>((static_cast<size_t>(n) * 100 + 7) / 8), 256, 0,
+                            stream>>>(dhead, params, a.act[4], n, g0);
+  // Convolutions, last to first. g_in holds layer l's dz.
   float* g_in = g0;
   float* g_out = g1;
   for (int l = 3; l >= 0; --l) {
-    const LayerShape L = Layer(l);
-    const size_t out_pixels = static_cast<size_t>(n) * L.out_size * L.out_size;
-    const unsigned chunks = static_cast<unsigned>((out_pixels + kConvChunk - 1) / kConvChunk);
-    const int patch = 9 * L.cin;
+    int width, chunks, status;
     if (l == 0) {
-      ConvBackwardWeightKernel<kCnnInChannels><<<chunks, 256, 0, stream>>>(
-        g_in, a.act[1], a.act[0], 0, n, partial);
+      status = LaunchConvWeights<kCnnInChannels, 2>(g_in, a.act[0], 0, n, partial, &width,
+                                                    &chunks, stream);
+    } else if (l == 3) {
+      status = LaunchConvWeights<kCnnC, 1>(g_in, a.act[3], 3, n, partial, &width, &chunks, stream);
     } else {
-      ConvBackwardWeightKernel<kCnnC><<<chunks, 256, 0, stream>>>(g_in, a.act[l + 1], a.act[l],
-                                                                  l, n, partial);
+      status = LaunchConvWeights<kCnnC, 2>(g_in, a.act[l], l, n, partial, &width, &chunks, stream);
     }
+    if (status != GJXL_B200_OK) return status;
     // Partials are [chunk][co * patch + e | 32 biases]: W then b, contiguous
     // in the parameter layout.
-    const int width = kCnnC * patch + kCnnC;
-    ReducePartialsKernel<<<(width + 127) / 128, 128, 0, stream>>>(partial, static_cast<int>(chunks),
-                                                                  width, grads + L.w_offset);
+    const LayerShape L = Layer(l);
+    ReducePartialsKernel<<<(width + 31) / 32, 32 * kReduceSlices, 0, stream>>>(
+      partial, chunks, width, grads + L.w_offset);
     if (l > 0) {
-      const size_t in_pixels = static_cast<size_t>(n) * L.in_size * L.in_size;
-      ConvBackwardInputKernel<kCnnC><<<static_cast<unsigned>((in_pixels + 127) / 128), 128, 0,
-                                       stream>>>(g_in, a.act[l + 1], params, l, n, g_out);
+      const int side = L.in_size / L.stride;
+      const unsigned pixel_tiles = static_cast<unsigned>(
+        (static_cast<size_t>(n) * side * side + kConvTile - 1) / kConvTile);
+      const dim3 grid(pixel_tiles, L.stride * L.stride);
+      if (L.stride == 1) {
+        ConvBackwardInputKernel<1><<<grid, kConvThreads, 0, stream>>>(g_in, a.act[l], params, l, n,
+                                                                      g_out);
+      } else {
+        ConvBackwardInputKernel<2><<<grid, kConvThreads, 0, stream>>>(g_in, a.act[l], params, l, n,
+                                                                      g_out);
+      }
       float* t = g_in;
       g_in = g_out;
       g_out = t;
