@@ -230,27 +230,33 @@ struct PopulationParams {
   uint32_t* present_mask;
 };
 
-// One CTA per group and channel (blockIdx.y). The group's anchors are first
-// listed per family, with the log2 of their footprint width; then, family by
+// One CTA per strip of kStripRows block rows of a group (blockIdx.z) and
+// channel (blockIdx.y): a whole group per CTA left all but 3 SMs idle on a
+// 256x256 image and waited for one load after another (119 us there, 152 us
+// at 2048x1536). The strip's anchors are first listed per family, with the log2 of their footprint width; then, family by
 // family, each thread owns one physical index (and a share of the anchors
 // when the family has fewer than 256 indices) and counts zeros in a
 // register, four anchors' coefficients loaded at a time, so shared-memory
 // atomics happen once per thread and index, not once per coefficient.
+constexpr int kStripRows = 4;
+constexpr int kStripBlocks = kStripRows * kGroupBlocks;
+
 __global__ void __launch_bounds__(256) PopulationKernel(const __grid_constant__ PopulationParams p) {
   __shared__ uint32_t counts[kPopulationStride + 64];  // this channel; then the DCT8 sample
-  __shared__ short2 anchors[5][kGroupBlocks * kGroupBlocks];
-  __shared__ uint8_t anchor_shift[5][kGroupBlocks * kGroupBlocks];
-  __shared__ uint8_t sampled[kGroupBlocks * kGroupBlocks];
+  __shared__ short2 anchors[5][kStripBlocks];
+  __shared__ uint8_t anchor_shift[5][kStripBlocks];
+  __shared__ uint8_t sampled[kStripBlocks];
   __shared__ int anchor_count[5];
   __shared__ uint32_t present;
   const int c = blockIdx.y;
+  const int x0 = (blockIdx.x % p.groups_x) * kGroupBlocks;
+  const int y0 = (blockIdx.x / p.groups_x) * kGroupBlocks + blockIdx.z * kStripRows;
+  const int w = min(kGroupBlocks, p.blocks_x - x0), h = min(kStripRows, p.blocks_y - y0);
+  if (h <= 0) return;
   for (int i = threadIdx.x; i < kPopulationStride + 64; i += blockDim.x) counts[i] = 0;
   if (threadIdx.x < 5) anchor_count[threadIdx.x] = 0;
   if (threadIdx.x == 0) present = 0;
   __syncthreads();
-  const int x0 = (blockIdx.x % p.groups_x) * kGroupBlocks;
-  const int y0 = (blockIdx.x / p.groups_x) * kGroupBlocks;
-  const int w = min(kGroupBlocks, p.blocks_x - x0), h = min(kGroupBlocks, p.blocks_y - y0);
   for (int b = threadIdx.x; b < w * h; b += blockDim.x) {
     const int bx = x0 + b % w, by = y0 + b / w;
     const TaskShape t = ShapeAt(p.cells, by * p.blocks_x + bx);
@@ -836,7 +842,7 @@ extern "C" int gjxl_b200_ac_tokenize(gjxl_b200_ac_tokens* s, const uint8_t* stra
     pp.sample = s->sample;
     pp.population = s->population;
     pp.present_mask = s->masks;
-    PopulationKernel<<<dim3(groups, 3), 256, 0, stream>>>(pp);
+    PopulationKernel<<<dim3(groups, 3, kGroupBlocks / kStripRows), 256, 0, stream>>>(pp);
   }
   if (order_mode != 0) {
     OrderParams op;
