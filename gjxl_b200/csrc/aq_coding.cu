@@ -731,31 +731,22 @@ __device__ void AdjustFinish(int channel, int strategy, const AdjustSums& sums,
   *raw_quant = adjusted;
 }
 
-// ConvertLowFrequenciesToDc (dc_conversion.cpp:174-236) of one channel.
+// ConvertLowFrequenciesToDc (dc_conversion.cpp:174-236): the DC of block
+// (y, x) of one channel's transform. One thread per block: a thread that ran
+// all 16 of a 32x32 transform held its CTA up for most of its life.
 template <int W, int H>
-__device__ void LowFrequenciesToDc(const float* coef, float* out) {
+__device__ float LowFrequencyDc(const float* coef, int y, int x) {
   using S = TransformShape<W, H>;
   constexpr int CW = S::CW, CH = S::CH;
   const int lh = LenIndex(CH), lw = LenIndex(CW);
-  double scaled[16];
+  double value = 0.0;
+#pragma unroll
   for (int v = 0; v < CH; ++v) {
     for (int u = 0; u < CW; ++u) {
-      const int small = CH < CW ? v * CW + u : u * CH + v;
-      scaled[small] = static_cast<double>(coef[S::Index(v, u)]) *
-                      static_cast<double>(c_dc_tables.downsample[lh][v]) *
-                      static_cast<double>(c_dc_tables.downsample[lw][u]);
-    }
-  }
-  for (int y = 0; y < CH; ++y) {
-    for (int x = 0; x < CW; ++x) {
-      double value = 0.0;
-      for (int v = 0; v < CH; ++v) {
-        for (int u = 0; u < CW; ++u) {
-          const int small = CH < CW ? v * CW + u : u * CH + v;
-          value += scaled[small] * c_dc_tables.inverse[lh][v][y] * c_dc_tables.inverse[lw][u][x];
-        }
-      }
-      out[y * CW + x] = static_cast<float>(value);
+      const double scaled = static_cast<double>(coef[S::Index(v, u)]) *
+                            static_cast<double>(c_dc_tables.downsample[lh][v]) *
+                            static_cast<double>(c_dc_tables.downsample[lw][u]);
+      value += scaled * c_dc_tables.inverse[lh][v][y] * c_dc_tables.inverse[lw][u][x];
     }
   }
 }
@@ -819,7 +810,12 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
   __shared__ float inverse_dequant[3][N];
   __shared__ float thresholds[3][4];
   __shared__ int candidates[3];
-  __shared__ float adjust_err[3][N];   // per coefficient |value - quantized|, 0 on the LLF
+  // Per coefficient |value - quantized|, 0 on the LLF; and the border terms in
+  // storage order: the last column of rows 4..6 of 8, the larger corner's
+  // rows, and the last row's second half.
+  constexpr int kBorder = 3 * (S::SH / 8) + (S::SH / 8 - 1) * (S::SW / 8) + 4 * (S::SW / 8);
+  __shared__ __align__(16) float adjust_err[3][N];
+  __shared__ float border[3][kBorder];
   __shared__ uint32_t adjust_sum[2][3][5];  // per warp and channel: sum |q|, per quadrant
   __shared__ uint32_t adjust_max[2][4];     // per warp: Y max error per quadrant (float bits)
   __shared__ int adjust_big[2];             // per warp: a |q| sum reached 2^24
@@ -858,6 +854,7 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
   using Sh = TransformShape<W, H>;
   constexpr int xsize = Sh::SW / 8, ysize = Sh::SH / 8;
   const float qac = q.scale * static_cast<float>(initial_raw);
+#pragma unroll
   float t0[4];
   AdjustThresholds<W, H>(t0);
   {
@@ -877,6 +874,7 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
         }
         const int quadrant = (y >= Sh::SH / 2) * 2 + (x >= Sh::SW / 2);
         const float value = coef[c][index] * (inverse_dequant[c][index] * qac * mm);
+  return static_cast<float>(value);
         const float quantized = fabsf(value) < t0[quadrant] ? 0.0f : rintf(value);
         const float err = fabsf(value - quantized);
         adjust_err[c][index] = err;
@@ -911,6 +909,34 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
       if (lane == 0) adjust_max[warp][k] = m;
     }
     const bool any_big = __any_sync(0xffffffffu, big);
+// t[0] + t[1] + ... + t[N-1] in order, 16 terms at a time with the next 16
+// loaded during the adds; `t` 16-byte aligned.
+template <int N>
+__device__ __forceinline__ float CodingOrderedSum(const float* t) {
+  static_assert(N % 16 == 0, "whole groups");
+  const float4* v = reinterpret_cast<const float4*>(t);
+  float4 now[4], next[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) now[k] = next[k] = v[k];
+  float sum = 0.0f;
+#pragma unroll 2
+  for (int j = 0; j < N / 4; j += 4) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (j + 4 < N / 4) next[k] = v[j + 4 + k];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      sum += now[k].x;
+      sum += now[k].y;
+      sum += now[k].z;
+      sum += now[k].w;
+      now[k] = next[k];
+    }
+  }
+  return sum;
+}
+
     if (lane == 0) adjust_big[warp] = any_big ? 1 : 0;
   }
   __syncthreads();
@@ -925,25 +951,11 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
                              inverse_dequant[c], t, &sums);
     } else {
       // The ordered sums: error terms in storage order (+0.0 on the LLF
-      // leaves the never -0.0 sum unchanged), and the border terms, which
-      // all lie in the larger corner, in storage order.
-      float error_sum = 0.0f;
-#pragma unroll 8
-      for (int index = 0; index < N; ++index) error_sum += adjust_err[c][index];
+      // leaves the never -0.0 sum unchanged), and the border terms.
+      const float error_sum = CodingOrderedSum<N>(adjust_err[c]);
       float border_sum = 0.0f;
-      const float mm = c == 0 ? mm0 : c == 1 ? mm1 : mm2;
-      for (int y = 4 * ysize; y < Sh::SH; ++y) {
-        for (int x = 4 * xsize; x < Sh::SW; ++x) {
-          const bool in_corner = y >= 7 * ysize && x >= 7 * xsize;
-          const bool on_border = y + 1 == Sh::SH || x + 1 == Sh::SW;
-          if (!(in_corner || on_border)) continue;
-          const int index = y * Sh::SW + x;
-          const int quadrant = (y >= Sh::SH / 2) * 2 + (x >= Sh::SW / 2);
-          const float value = coef[c][index] * (inverse_dequant[c][index] * qac * mm);
-          const float quantized = fabsf(value) < t[quadrant] ? 0.0f : rintf(value);
-          if (quantized != 0.0f) border_sum += fabsf(value);
-        }
-      }
+#pragma unroll 4
+      for (int i = 0; i < kBorder; ++i) border_sum += border[c][i];
       sums.error_sum = error_sum;
       sums.border_sum = border_sum;
       sums.value_sum = static_cast<float>(total);
@@ -956,14 +968,11 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
     AdjustFinish<W, H>(c, strategy, sums, t, &candidate);
     for (int i = 0; i < 4; ++i) thresholds[c][i] = t[i];
     candidates[c] = candidate;
-  } else if (tid == 32) {
+  } else if (tid >= 32 && tid < 32 + covered) {
     // Y DC from the unquantized Y coefficients.
-    float dc[16];
-    LowFrequenciesToDc<W, H>(coef[1], dc);
-    for (int dy = 0; dy < S::CH; ++dy)
-      for (int dx = 0; dx < S::CW; ++dx)
-        p.dc[1 * p.dc_pitch + static_cast<size_t>(a.y + dy) * p.blocks_x + a.x + dx] =
-          dc[dy * S::CW + dx];
+    const int dy = (tid - 32) / S::CW, dx = (tid - 32) % S::CW;
+    p.dc[1 * p.dc_pitch + static_cast<size_t>(a.y + dy) * p.blocks_x + a.x + dx] =
+      LowFrequencyDc<W, H>(coef[1], dy, dx);
   }
   __syncthreads();
   const int raw = max(candidates[0], max(candidates[1], candidates[2]));
@@ -990,14 +999,10 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
     coef[2][j] -= f2 * coef[1][j];
   }
   __syncthreads();
-  if (tid == 0 || tid == 32) {
-    const int c = tid == 0 ? 0 : 2;
-    float dc[16];
-    LowFrequenciesToDc<W, H>(coef[c], dc);
-    for (int dy = 0; dy < S::CH; ++dy)
-      for (int dx = 0; dx < S::CW; ++dx)
-        p.dc[c * p.dc_pitch + static_cast<size_t>(a.y + dy) * p.blocks_x + a.x + dx] =
-          dc[dy * S::CW + dx];
+  if (tid % 32 < covered) {
+    const int c = tid < 32 ? 0 : 2, dy = tid % 32 / S::CW, dx = tid % 32 % S::CW;
+    p.dc[c * p.dc_pitch + static_cast<size_t>(a.y + dy) * p.blocks_x + a.x + dx] =
+      LowFrequencyDc<W, H>(coef[c], dy, dx);
   }
   float t[4];
   ChromaThresholds(covered, t);
@@ -1015,6 +1020,24 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
 
 // ---------------------------------------------------------------------------
 // Prediction-aware DC quantization with the weighted predictor.
+    for (int i = tid; i < 3 * kBorder; i += kT) {
+      const int c = i / kBorder, j = i % kBorder;
+      constexpr int kColumn = 3 * ysize, kCorner = (ysize - 1) * xsize;
+      int y = Sh::SH - 1, x = 4 * xsize + j - kColumn - kCorner;
+      if (j < kColumn) {
+        y = 4 * ysize + j;
+        x = Sh::SW - 1;
+      } else if (j < kColumn + kCorner) {
+        y = 7 * ysize + (j - kColumn) / xsize;
+        x = 7 * xsize + (j - kColumn) % xsize;
+      }
+      const int index = y * Sh::SW + x;
+      const int quadrant = (y >= Sh::SH / 2) * 2 + (x >= Sh::SW / 2);
+      const float mm = c == 0 ? mm0 : c == 1 ? mm1 : mm2;
+      const float value = coef[c][index] * (inverse_dequant[c][index] * qac * mm);
+      const float quantized = fabsf(value) < t0[quadrant] ? 0.0f : rintf(value);
+      border[c][j] = quantized != 0.0f ? fabsf(value) : 0.0f;
+    }
 //
 // The reference walks each 256x256-block DC group in raster order, channel
 // by channel (Y, X, B), resetting the predictor per channel. A sample at
