@@ -69,7 +69,9 @@ ForwardCoefficientsKernel(const float* opsin, size_t stride, size_t pitch, const
   using Batch = PlaneBatch<W, H, KC>;
   static_assert(Batch::Items == kTransformThreads, "one chunk per thread and pass");
   extern __shared__ __align__(16) unsigned char smem[];
-  double* tmp = reinterpret_cast<double*>(smem);                  // [KC] padded planes
+  constexpr int kBasis = W == 32 || H == 32 ? 32 * 32 : 0;  // staged length-32 basis
+  double* basis = reinterpret_cast<double*>(smem);
+  double* tmp = basis + kBasis;                                   // [KC] padded planes
   float* px = reinterpret_cast<float*>(tmp + Batch::Elements);    // [KC] padded planes
   const uint32_t first = blockIdx.x * K;
   // The anchor loads do not wait for the count: the list index is clamped to
@@ -105,9 +107,14 @@ ForwardCoefficientsKernel(const float* opsin, size_t stride, size_t pitch, const
   }
   __syncthreads();
   const auto present = [&](int plane) { return plane < 3 * active; };
-  BatchRowPass<W, H, KC, true>(px, tmp, threadIdx.x, kTransformThreads, present);
+  for (int i = threadIdx.x; i < kBasis / 2; i += kTransformThreads) {
+    reinterpret_cast<double2*>(basis)[i] =
+      __ldg(reinterpret_cast<const double2*>(kDctStagedForwardT32) + i);
+  }
+  const double* staged = kBasis > 0 ? basis : nullptr;
+  BatchRowPass<W, H, KC, true>(px, tmp, threadIdx.x, kTransformThreads, present, staged);
   __syncthreads();
-  BatchColumnPass<W, H, KC, true>(tmp, px, threadIdx.x, kTransformThreads, present);
+  BatchColumnPass<W, H, KC, true>(tmp, px, threadIdx.x, kTransformThreads, present, staged);
   __syncthreads();
   // Coefficient j = coefficient_index(v, u) goes to footprint (j % W, j / W).
   for (int i = threadIdx.x; i < active * 3 * N; i += kTransformThreads) {
@@ -1216,36 +1223,43 @@ DcQuantKernel(const __grid_constant__ DcQuantParams p) {
   // The sample of the next position is loaded one wave ahead, so its
   // global-memory latency overlaps this wave's work and barrier.
   const size_t row_index = static_cast<size_t>(gy0 + min(y, gh - 1)) * stride + gx0;
-  uint32_t pending = y < gh ? source[row_index] : 0u;  // idle threads have y >= gh
-  // This row's previous quantized value and signed error (its west
-  // neighbour), kept in registers.
-  int32_t own_q = 0, own_e = 0;
-  const int waves = (gw - 1) + 2 * (gh - 1) + 2;
-  for (int t = 0; t < waves; ++t) {
-    const int x = t - lag - 2 * y;
-    const int wide = r.wide;
-    if (y < gh && x >= 0 && x < gw) {
-      const uint32_t sample = pending;
-      if (x + 1 < gw) pending = source[row_index + x + 1];
-      const int s = x & 7, sw = (x - 1) & 7, sne = (x + 1 < gw ? x + 1 : x) & 7;
-      const int snw = (x ? x - 1 : x) & 7;
-      const int up = y - 1, up2 = y - 2;
-      const int32_t w = x ? own_q : y ? Q[s][up] : 0;
-      const int32_t n = y ? Q[s][up] : w;
-      const int32_t nw = x && y ? Q[sw][up] : w;
-      const int32_t ne = y && x + 1 < gw ? Q[(x + 1) & 7][up] : n;
-      const int32_t nn = y > 1 ? Q[s][up2] : n;
-      const int32_t ew = x ? own_e : 0;
-      const int32_t en = y ? E[s][up] : 0;
-      const int32_t enw = y ? E[snw][up] : 0;
-      const int32_t ene = y ? E[sne][up] : 0;
-      // Sub-predictor error sums (prediction.h:73-90). The signed errors of
-      // row -1 read as zeros. The error sums of row 0 read the predictor's
-      // other rolling row, which by then holds only row 0's own "+="
-      // updates: its entry j carries the error of (j - 1, 0) once that
-      // sample is done, so north = err(x-1), northwest = err(x-2) and
-      // northeast (not yet written) = 0, or north at the right edge.
-      uint32_t errors[4];
+  const uint32_t* source = (kReplay ? reinterpret_cast<const uint32_t*>(p.replay)
+                                    : reinterpret_cast<const uint32_t*>(p.dc)) +
+                           c * p.pitch + row_index;
+  int32_t* plane = kReplay ? nullptr : p.quantized + c * p.pitch + row_index;
+  uint2* tokens = !kTokens ? nullptr
+                           : p.tokens + DcTokenOffset(blockIdx.x, blockIdx.y, p.width, p.height) +
+                               (static_cast<size_t>(DcChannelRank(c)) * gh + y) * gw;
+  uint32_t* ring = &r.samples[0][threadIdx.x];
+  // The row above at x-1, x, x+1 (zero errors above the group's first row),
+  // this row's last sample, and its sub-predictor errors at x-2. Past the
+  // row's ends the nearest sample stands in, as the reference reads it: the
+  // west side is set up one step before the row starts, and on the east side
+  // the lane above has stopped at its last sample.
+  DcSample above_w = {}, above = {}, above_e = {}, own = {};
+  uint32_t before_own[4] = {0, 0, 0, 0};
+  DcSample next = {};  // lane 0: the predecessor warp's sample of the next step
+  int wide = 0;
+  const int steps = kDcLead + gw + 2 * ((gh - 1) % kDcRows) + (warps - 1) * kDcWarpSkew +
+                    (blockIdx.z == 0 ? 0 : kDcSync);
+  for (int t = 0; t < steps; ++t) {
+    const int first = t - kDcLead - start;  // lane 0's position
+    if (first >= -kDcLead && first < gw + 2 * (kDcRows - 1)) {
+      const int x = first - 2 * lane;
+      // Samples arrive kDcLead steps ahead of their use.
+      if (y < gh && x >= -kDcLead && x + kDcLead < gw) {
+        const uint32_t slot = static_cast<uint32_t>(
+          __cvta_generic_to_shared(ring + ((x + kDcLead) & (kDcSampleSlots - 1)) * kDcThreads));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(slot),
+                     "l"(source + x + kDcLead)
+                     : "memory");
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      above_w = above;
+      above = above_e;
+      above_e.q = __shfl_up_sync(0xffffffffu, own.q, 1);
+      above_e.e = __shfl_up_sync(0xffffffffu, own.e, 1);
+      above_e.n = __shfl_up_sync(0xffffffffu, own.n, 1);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         if (y) {
