@@ -20,6 +20,8 @@
 // anchored at block (bx, by) occupy its own W x H pixel footprint of a padded
 // plane, coefficient i at (bx*8 + i % W, by*8 + i / W).
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -105,12 +107,12 @@ ForwardCoefficientsKernel(const float* opsin, size_t stride, size_t pitch, const
     const int k = i / (3 * N), r = i % (3 * N), c = r / N, yx = r % N;
     px[Batch::At(k * 3 + c, yx / W, yx % W)] = value[q];
   }
-  __syncthreads();
-  const auto present = [&](int plane) { return plane < 3 * active; };
   for (int i = threadIdx.x; i < kBasis / 2; i += kTransformThreads) {
     reinterpret_cast<double2*>(basis)[i] =
       __ldg(reinterpret_cast<const double2*>(kDctStagedForwardT32) + i);
   }
+  __syncthreads();
+  const auto present = [&](int plane) { return plane < 3 * active; };
   const double* staged = kBasis > 0 ? basis : nullptr;
   BatchRowPass<W, H, KC, true>(px, tmp, threadIdx.x, kTransformThreads, present, staged);
   __syncthreads();
@@ -318,11 +320,8 @@ __global__ void __launch_bounds__(1024) SelectDigitKernel(int pass, int n, bool 
 }
 
 // CreateQuantizerFromField + ComputeQuantizerParams + Quantizer::Create.
-__global__ void QuantizerKernel(const SelectState* st, const AqPolicy* policy, AqQuantizer* q,
-                                uint32_t* error) {
-  const float median = __uint_as_float(st->median_bits);
-  const float mad = __uint_as_float(st->mad_bits);
-  const float quant_dc = policy->quant_dc;
+__device__ AqQuantizer MakeQuantizer(float median, float mad, float quant_dc, bool* in_range) {
+  AqQuantizer q;
   float scale = 65536.0f * (median - mad) / 5.0f;
   scale = fminf(fmaxf(scale, 1.0f), 32768.0f);
   int global_scale = static_cast<int>(scale);
@@ -331,18 +330,16 @@ __global__ void QuantizerKernel(const SelectState* st, const AqPolicy* policy, A
   const float inverse_global_scale = 65536.0f / static_cast<float>(global_scale);
   const float quant_dc_value = fminf(65536.0f, quant_dc * inverse_global_scale + 0.5f);
   const uint32_t qdc = static_cast<uint32_t>(quant_dc_value);
-  q->global_scale = static_cast<uint32_t>(global_scale);
-  q->quant_dc = qdc;
-  if (global_scale < 1 || global_scale > 32768 || qdc == 0 || qdc > 65536) {
-    RaiseError(error, kErrorRange);
-  }
-  q->scale = static_cast<float>(global_scale) / 65536.0f;
-  q->inverse_global_scale = 65536.0f / static_cast<float>(global_scale);
-  const float inverse_quant_dc = q->inverse_global_scale / static_cast<float>(qdc);
+  q.global_scale = static_cast<uint32_t>(global_scale);
+  q.quant_dc = qdc;
+  *in_range = global_scale >= 1 && global_scale <= 32768 && qdc != 0 && qdc <= 65536;
+  q.scale = static_cast<float>(global_scale) / 65536.0f;
+  q.inverse_global_scale = 65536.0f / static_cast<float>(global_scale);
+  const float inverse_quant_dc = q.inverse_global_scale / static_cast<float>(qdc);
   const float kInverseDcQuant[3] = {4096.0f, 512.0f, 256.0f};
   for (int c = 0; c < 3; ++c) {
-    q->dc_steps[c] = inverse_quant_dc / kInverseDcQuant[c];
-    q->inverse_dc_steps[c] = kInverseDcQuant[c] * q->scale * static_cast<float>(qdc);
+    q.dc_steps[c] = inverse_quant_dc / kInverseDcQuant[c];
+    q.inverse_dc_steps[c] = kInverseDcQuant[c] * q.scale * static_cast<float>(qdc);
   }
 }
 
@@ -1402,6 +1399,17 @@ unsigned Blocks(size_t n, unsigned threads = kThreads) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
+  __syncthreads();
+  // Warps past the group's rows, and X's unused half, have nothing to do.
+  const int warps = (gh + kDcRows - 1) / kDcRows;
+  const int half = static_cast<int>(threadIdx.x) / kDcGroup;
+  const int warp = static_cast<int>(threadIdx.x) % kDcGroup / kDcRows;
+  const int lane = static_cast<int>(threadIdx.x) % kDcRows;
+  if (warp >= warps || (blockIdx.z == 0 && half == 1)) return;
+  const int working = warps * kDcRows * (blockIdx.z == 0 ? 1 : 2);
+  const int c = blockIdx.z == 0 ? 0 : 1 + half;  // X; Y, B
+  const int y = warp * kDcRows + lane;
+  const int start = warp * kDcWarpSkew + (c == 2 ? kDcSync : 0);
 // Host launchers.
 
 void UploadDcTables() {
