@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include <cuda_bf16.h>
 
@@ -96,6 +97,8 @@ struct CostParams {
   const CandidateDesc* batch;
   float* batch_costs;
   int batch_resident;
+  // Rows of eight pixels start on 16-byte boundaries (set at launch).
+  bool opsin_aligned, mask_aligned;
 };
 
 // Candidates scored: every tile's, or those of the kept tiles.
@@ -135,31 +138,64 @@ struct CostLayout {
   // plane, same index at the same time) of each quarter warp hit distinct
   // banks.
   static constexpr int TermPitch = N + 4;
-  // Families with a length-32 side read that pass's basis from a shared copy
-  // (the forward table through the forward passes, then the inverse table).
+  // Families with a length-32 side read that pass's forward basis from a
+  // shared copy, whose place the pixel mask takes after the forward passes.
   static constexpr bool kStagedBasis = (W == 32 || H == 32) && sizeof(Acc) == 8;
   static constexpr int BasisDoubles = kStagedBasis ? 32 * 32 : 0;
   static constexpr size_t SharedBytes = static_cast<size_t>(BasisDoubles) * 8 +
                                         static_cast<size_t>(Planes) * (4 + 4 + sizeof(Acc)) +
-                                        static_cast<size_t>(KC) * TermPitch * 4;
-  static_assert(K * N <= Planes, "the pixel mask fits the residual buffer");
+                                        static_cast<size_t>(KC) * TermPitch * 4 +
+                                        (kStagedBasis ? 0 : static_cast<size_t>(K) * N * 4);
+  static_assert(BasisDoubles == 0 || K * N * 4 <= BasisDoubles * 8, "the mask fits the basis");
+  static_assert(Planes % 4 == 0 && TermPitch % 4 == 0, "16-byte aligned buffers");
   static_assert(Batch::Items == kCostThreads, "one chunk per thread and pass");
+
+  // The element-wise stages give each channel 128 threads: thread t of a
+  // channel owns elements t + 128 q, q = 0..7, of the channel's K planes of N,
+  // so that channel and candidate are warp-uniform and the position in the
+  // plane takes kPositions values per thread.
+  static constexpr int kChannelThreads = kCostThreads / 3;
+  static constexpr int kPerThread = K * N / kChannelThreads;
+  static constexpr int kPositions = N <= kChannelThreads ? 1 : N / kChannelThreads;
+  __device__ static int Candidate(int t, int q) {
+    return N <= kChannelThreads ? t / N + q * (kChannelThreads / N) : q / kPositions;
+  }
+  __device__ static int Position(int t, int q) {
+    return N <= kChannelThreads ? t % N : t + kChannelThreads * (q % kPositions);
+  }
 };
 
 // Sequential float sum t[0] + t[1] + ... + t[n-1] (the reference's loop
-// order), read four terms at a time.
+// order), 16 terms at a time with the next 16 loaded during the adds.
 template <int kCount>
 __device__ __forceinline__ float OrderedSum(const float* t) {
+  static_assert(kCount % 16 == 0, "whole groups");
+  float4 now[4], next[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) now[q] = reinterpret_cast<const float4*>(t)[q];
   float sum = 0.0f;
-#pragma unroll 4
-  for (int j = 0; j < kCount; j += 4) {
-    const float4 v = *reinterpret_cast<const float4*>(t + j);
-    sum += v.x;
-    sum += v.y;
-    sum += v.z;
-    sum += v.w;
+#pragma unroll 2
+  for (int j = 0; j < kCount; j += 16) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (j + 16 < kCount) next[q] = reinterpret_cast<const float4*>(t + j + 16)[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      sum += now[q].x;
+      sum += now[q].y;
+      sum += now[q].z;
+      sum += now[q].w;
+      now[q] = next[q];
+    }
   }
   return sum;
+}
+
+// Four consecutive floats, in one load where their alignment allows.
+__device__ __forceinline__ float4 LoadFour(const float* p, bool aligned) {
+  if (aligned) return __ldg(reinterpret_cast<const float4*>(p));
+  return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
 }
 
 // Sum of each plane's N terms by kThreads / KC threads per plane (a fixed
@@ -331,6 +367,16 @@ __device__ __forceinline__ float CandidateCost(const CostParams& p, const float 
 // Acc = double: the bit-exact restatement (FP64 products, separately
 // rounded, sequential sums). Acc = float: the fast mode's FP32 passes for the
 // 8-pixel families (fused multiply-adds on the bases rounded to float).
+//
+// Bound: FP64 issue of the exact forward passes, which the sequential sums
+// prescribe (16 instructions per sample and 8 outputs). The inverse passes
+// are folded (line_dct.cuh): a quarter of the FP64 instructions, and columns
+// whose rounding that does not settle are transformed again sequentially.
+// The element-wise stages, which took more issue slots than the transforms
+// (1400 of the 8x8 family's 2156 instructions per thread), keep channel and
+// candidate warp-uniform and the position in the plane fixed per thread, move
+// pixels in 16-byte loads, and skip the square roots of a warp's 32
+// coefficients that all quantize to zero.
 template <int W, int H, typename Acc>
 __global__ void __launch_bounds__(kCostThreads, 3)
 CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_count) {
@@ -338,6 +384,7 @@ CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_cou
   using Lay = CostLayout<W, H, Acc>;
   constexpr bool kExact = sizeof(Acc) == 8;
   constexpr int N = S::N, K = Lay::K, KC = Lay::KC;
+  constexpr int kPerThread = Lay::kPerThread;
   static_assert(K == S::K, "candidates per CTA");
   static_assert(kExact || (W <= 16 && H <= 16), "FP32 passes cover lengths 8 and 16");
   extern __shared__ __align__(16) unsigned char smem[];
@@ -346,17 +393,23 @@ CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_cou
   float* A = reinterpret_cast<float*>(T + Lay::Planes);    // [KC][H][W+1] pixels, residuals
   float* B = A + Lay::Planes;                              // [KC][H][W+1] coefficients, pixels
   float* terms = B + Lay::Planes;                          // [KC][N + 4] ordered sum terms
-  float* mask = A;  // [K][H][W] pixel mask, once the inverse row pass has read A
+  // [K][H][W] pixel mask
+  float* mask = Lay::kStagedBasis ? reinterpret_cast<float*>(basis) : terms + KC * Lay::TermPitch;
   __shared__ int anchor_x[K], anchor_y[K];
-  __shared__ float quant_norm[K], cfl[K][3];
+  __shared__ size_t pixel_base[K], mask_base[K];  // first pixel of the candidate
+  // Per candidate and channel: CfL factor, quant norm.
+  __shared__ float2 scale[K][3];
   __shared__ float magnitude[K][3], loss_sum[K][3];
   __shared__ uint32_t nonzero[K][3];
-
-  const int tid = threadIdx.x;
-  // Anchors first (integer arithmetic only), so that the pixel loads can
-  // start before the quant norms and CfL factors arrive.
+  __shared__ __align__(16) float row_magnitude[kExact ? KC * H : 4];
+  __shared__ FoldedAgain<W, kExact ? KC : 1> again;  // columns to transform again
   __shared__ float entropy[K];
   __shared__ int invalid[K];
+
+  const int tid = threadIdx.x;
+  const int c = tid / Lay::kChannelThreads, t = tid % Lay::kChannelThreads;
+  // Anchors first (integer arithmetic only), so that the pixel loads can
+  // start before the quant norms and CfL factors arrive.
   candidate_count = ScoredCandidates(p, candidate_count);
   if (blockIdx.x * K >= candidate_count) return;  // past the kept tiles' candidates
   if (tid < K) {
@@ -390,59 +443,69 @@ CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_cou
     }
     anchor_x[tid] = ax;
     anchor_y[tid] = ay;
+    pixel_base[tid] = static_cast<size_t>(max(ay, 0)) * 8 * p.stride + max(ax, 0) * 8;
+    mask_base[tid] = static_cast<size_t>(max(ay, 0)) * 8 * p.mask_stride + max(ax, 0) * 8;
     magnitude[tid][0] = magnitude[tid][1] = magnitude[tid][2] = 0.0f;
     nonzero[tid][0] = nonzero[tid][1] = nonzero[tid][2] = 0;
   }
+  if constexpr (kExact) ClearAgain(again, tid);
   __syncthreads();
 
-  // Pixels into A (one W-float run of the source per row) and the forward
-  // length-32 basis into `basis`: every load of a thread is issued before the
-  // first store, so their latencies overlap.
+  // Pixels into A and the forward length-32 basis into `basis`: every load of
+  // a thread is issued before the first store, so their latencies overlap.
   constexpr int kBasisLoads = (Lay::BasisDoubles / 2 + kCostThreads - 1) / kCostThreads;
   const double2* staged_forward = reinterpret_cast<const double2*>(kDctStagedForwardT32);
-  const double2* staged_inverse = reinterpret_cast<const double2*>(kDctStagedInverse32);
   double2* basis2 = reinterpret_cast<double2*>(basis);
   {
-    constexpr int kPixelLoads = KC * N / kCostThreads;
-    float pixel[kPixelLoads];
     double2 table[kBasisLoads > 0 ? kBasisLoads : 1];
 #pragma unroll
     for (int q = 0; q < kBasisLoads; ++q) {
       const int i = tid + q * kCostThreads;
       if (i < Lay::BasisDoubles / 2) table[q] = __ldg(staged_forward + i);
     }
+    // Four pixels at once: quads t and t + 128 of the channel's K * N / 4.
+    constexpr int kQuads = kPerThread / 4;
+    static_assert(kQuads * 4 == kPerThread && K * N / 4 <= kCostThreads, "quads per thread");
+    float4 pixel[kQuads];
 #pragma unroll
-    for (int q = 0; q < kPixelLoads; ++q) {
-      const int i = tid + q * kCostThreads;
-      const int kc = i / N, r = i % N, y = r / W, x = r % W, k = kc / 3, c = kc % 3;
-      pixel[q] = anchor_x[k] < 0 ? 0.0f
-               : p.opsin[c * p.pitch + static_cast<size_t>(anchor_y[k] * 8 + y) * p.stride +
-                         anchor_x[k] * 8 + x];
+    for (int q = 0; q < kQuads; ++q) {
+      const int quad = t + q * Lay::kChannelThreads;
+      const int k = quad / (N / 4), r = quad % (N / 4) * 4, y = r / W, x = r % W;
+      pixel[q] = anchor_x[k] < 0 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f)
+                                 : LoadFour(p.opsin + c * p.pitch + pixel_base[k] +
+                                              y * p.stride + x, p.opsin_aligned);
     }
     // ComputeQuantNormUnchecked (ac_strategy.cpp:103-130) and the CfL
     // factors, while the loads above are in flight.
-    if (tid < K && anchor_x[tid] >= 0 && p.batch != nullptr && !p.batch_resident) {
-      const CandidateDesc d = p.batch[blockIdx.x * K + tid];
-      quant_norm[tid] = d.quant_norm;
-      cfl[tid][0] = d.cfl_x;
-      cfl[tid][1] = 0.0f;
-      cfl[tid][2] = d.cfl_b;
-    } else if (tid < K && anchor_x[tid] >= 0) {
-      const int ax = anchor_x[tid], ay = anchor_y[tid];
-      const float qn = QuantNorm<S::CW, S::CH>(p, ax, ay);
-      if (!(IsFinite(qn) && qn > 0.0f)) RaiseError(p.error, kErrorNonFiniteInput);
-      quant_norm[tid] = qn;
-      const int tile_index = (ay / 8) * p.tiles_x + (ax / 8);
-      // ColorCorrelationMap::AcFactors (chroma_from_luma.cpp:412-432).
-      cfl[tid][0] = static_cast<float>(p.y_to_x[tile_index]) / 84.0f;
-      cfl[tid][1] = 0.0f;
-      cfl[tid][2] = 1.0f + static_cast<float>(p.y_to_b[tile_index]) / 84.0f;
+    if (tid < K && anchor_x[tid] >= 0) {
+      float qn, cfl_x, cfl_b;
+      if (p.batch != nullptr && !p.batch_resident) {
+        const CandidateDesc d = p.batch[blockIdx.x * K + tid];
+        qn = d.quant_norm;
+        cfl_x = d.cfl_x;
+        cfl_b = d.cfl_b;
+      } else {
+        const int ax = anchor_x[tid], ay = anchor_y[tid];
+        qn = QuantNorm<S::CW, S::CH>(p, ax, ay);
+        if (!(IsFinite(qn) && qn > 0.0f)) RaiseError(p.error, kErrorNonFiniteInput);
+        const int tile_index = (ay / 8) * p.tiles_x + (ax / 8);
+        // ColorCorrelationMap::AcFactors (chroma_from_luma.cpp:412-432).
+        cfl_x = static_cast<float>(p.y_to_x[tile_index]) / 84.0f;
+        cfl_b = 1.0f + static_cast<float>(p.y_to_b[tile_index]) / 84.0f;
+      }
+      scale[tid][0] = make_float2(cfl_x, qn);
+      scale[tid][1] = make_float2(0.0f, qn);
+      scale[tid][2] = make_float2(cfl_b, qn);
     }
 #pragma unroll
-    for (int q = 0; q < kPixelLoads; ++q) {
-      const int i = tid + q * kCostThreads;
-      const int kc = i / N, r = i % N, y = r / W, x = r % W;
-      if (anchor_x[kc / 3] >= 0) A[kc * Lay::PlanePitch + y * Lay::RowPitch + x] = pixel[q];
+    for (int q = 0; q < kQuads; ++q) {
+      const int quad = t + q * Lay::kChannelThreads;
+      const int k = quad / (N / 4), r = quad % (N / 4) * 4, y = r / W, x = r % W;
+      float* dst = A + (k * 3 + c) * Lay::PlanePitch + y * Lay::RowPitch + x;
+      dst[0] = pixel[q].x;
+      dst[1] = pixel[q].y;
+      dst[2] = pixel[q].z;
+      dst[3] = pixel[q].w;
     }
 #pragma unroll
     for (int q = 0; q < kBasisLoads; ++q) {
@@ -452,13 +515,14 @@ CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_cou
   }
   __syncthreads();
 
-  // Forward DCT (ForwardDctCpu): rows into T, then columns into B.
+  // Forward DCT (ForwardDctCpu): rows into T, then columns into B. The sign
+  // of a zero coefficient never reaches the cost.
   const auto present = [&](int plane) { return anchor_x[plane / 3] >= 0; };
   const double* staged = Lay::kStagedBasis ? basis : nullptr;
   if constexpr (kExact) {
-    BatchRowPass<W, H, KC, true>(A, T, tid, kCostThreads, present, staged);
+    BatchRowPass<W, H, KC, true, true>(A, T, tid, kCostThreads, present, staged);
     __syncthreads();
-    BatchColumnPass<W, H, KC, true>(T, B, tid, kCostThreads, present, staged);
+    BatchColumnPass<W, H, KC, true, true>(T, B, tid, kCostThreads, present, staged);
   } else {
     BatchRowPassF<W, H, KC, true>(A, T, tid, kCostThreads, present);
     __syncthreads();
@@ -468,65 +532,50 @@ CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_cou
 
   // Quantize, coefficient j = coefficient_index(v, u) by coefficient:
   // residual coefficients into A at (v, u), sqrt terms into terms[j]. The
-  // quantization weights of all of a thread's coefficients (and the inverse
-  // length-32 basis, which replaces the forward one) are loaded first.
+  // pixel mask is loaded alongside.
   {
-    constexpr int kPerThread = KC * N / kCostThreads;
-    float inv[kPerThread], dq[kPerThread];
-    double2 table[kBasisLoads > 0 ? kBasisLoads : 1];
-#pragma unroll
-    for (int q = 0; q < kBasisLoads; ++q) {
-      const int i = tid + q * kCostThreads;
-      if (i < Lay::BasisDoubles / 2) table[q] = __ldg(staged_inverse + i);
-    }
-#pragma unroll
-    for (int q = 0; q < kPerThread; ++q) {
-      const int i = tid + q * kCostThreads;
-      const int c = (i / N) % 3, j = i % N;
-      inv[q] = __ldg(p.inverse_dequant + c * N + j);
-      dq[q] = __ldg(p.dequant + c * N + j);
-    }
-#pragma unroll
-    for (int q = 0; q < kPerThread; ++q) {
-      const int i = tid + q * kCostThreads;
-      const int kc = i / N, j = i % N, k = kc / 3, c = kc % 3;
-      if (anchor_x[k] < 0) continue;
-      const int v = H < W ? j / W : j % H, u = H < W ? j % W : j / H;
-      const int at = v * Lay::RowPitch + u;
-      const float decorrelated =
-        B[kc * Lay::PlanePitch + at] - B[(k * 3 + 1) * Lay::PlanePitch + at] * cfl[k][c];
-      const float scaled = decorrelated * inv[q] * quant_norm[k];
-      const float rounded = roundf(scaled);
-      const float difference = scaled - rounded;
-      A[kc * Lay::PlanePitch + at] = dq[q] * difference;
-      terms[kc * Lay::TermPitch + j] = sqrtf(fabsf(rounded));
-      // A warp's 32 consecutive coefficients share (k, c) (N is a multiple
-      // of 32 and every thread runs the same trip count): one count per warp.
-      const unsigned nz = __ballot_sync(0xffffffffu, rounded != 0.0f);
-      if ((tid & 31) == 0 && nz != 0u) {
-        atomicAdd(&nonzero[k][c], static_cast<uint32_t>(__popc(nz)));
+    float4 weight = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    if (tid < K * N / 4) {
+      const int k = tid / (N / 4), r = tid % (N / 4) * 4, y = r / W, x = r % W;
+      if (anchor_x[k] >= 0) {
+        weight = LoadFour(p.pixel_mask + mask_base[k] + y * p.mask_stride + x, p.mask_aligned);
       }
     }
+    float inv[Lay::kPositions], dq[Lay::kPositions];
 #pragma unroll
-    for (int q = 0; q < kBasisLoads; ++q) {
-      const int i = tid + q * kCostThreads;
-      if (i < Lay::BasisDoubles / 2) basis2[i] = table[q];
+    for (int i = 0; i < Lay::kPositions; ++i) {
+      const int j = Lay::Position(t, i);
+      inv[i] = __ldg(p.inverse_dequant + c * N + j);
+      dq[i] = __ldg(p.dequant + c * N + j);
     }
+#pragma unroll
+    for (int q = 0; q < kPerThread; ++q) {
+      const int k = Lay::Candidate(t, q), j = Lay::Position(t, q);
+      constexpr int kPositions = Lay::kPositions;
+      const int i = q % kPositions;
+      if (anchor_x[k] < 0) continue;
+      const int v = H < W ? j / W : j % H, u = H < W ? j % W : j / H;
+      const int at = k * 3 * Lay::PlanePitch + v * Lay::RowPitch + u;
+      const float2 factors = scale[k][c];
+      const float decorrelated =
+        B[c * Lay::PlanePitch + at] - B[Lay::PlanePitch + at] * factors.x;
+      const float scaled = decorrelated * inv[i] * factors.y;
+      const float rounded = roundf(scaled);
+      const float difference = scaled - rounded;
+      A[c * Lay::PlanePitch + at] = dq[i] * difference;
+      // A warp's 32 consecutive coefficients share (k, c): one count and one
+      // choice per warp.
+      const unsigned nz = __ballot_sync(0xffffffffu, rounded != 0.0f);
+      float root = 0.0f;
+      if (nz != 0u) {
+        root = sqrtf(fabsf(rounded));
+        if ((tid & 31) == 0) atomicAdd(&nonzero[k][c], static_cast<uint32_t>(__popc(nz)));
+      }
+      terms[(k * 3 + c) * Lay::TermPitch + j] = root;
+    }
+    if (tid < K * N / 4) reinterpret_cast<float4*>(mask)[tid] = weight;
   }
   __syncthreads();
-
-  // The pixel mask is loaded now and kept in registers until the inverse
-  // row pass has read the residual out of A, where it then goes.
-  constexpr int kMaskLoads = (K * N + kCostThreads - 1) / kCostThreads;
-  float pmask[kMaskLoads];
-#pragma unroll
-  for (int q = 0; q < kMaskLoads; ++q) {
-    const int i = tid + q * kCostThreads;
-    const int k = i / N, r = i % N, y = r / W, x = r % W;
-    pmask[q] = i >= K * N || anchor_x[k] < 0 ? 1.0f
-             : p.pixel_mask[static_cast<size_t>(anchor_y[k] * 8 + y) * p.mask_stride +
-                            anchor_x[k] * 8 + x];
-  }
 
   // The exact mode's ordered magnitude sums (one thread per candidate and
   // channel) wait for the end, where they run beside the loss sums: summing
@@ -539,39 +588,40 @@ CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_cou
 
   // Inverse DCT (InverseDctCpu): rows of the residual into T, columns into B.
   if constexpr (kExact) {
-    BatchRowPass<W, H, KC, false>(A, T, tid, kCostThreads, present, staged);
+    FoldedRowPass<W, H, KC>(A, T, row_magnitude, tid, kCostThreads, present);
+    __syncthreads();
+    const auto plane_of = [&](int plane) { return B + plane * Lay::PlanePitch; };
+    FoldedColumnPass<W, H, KC>(T, plane_of, Lay::RowPitch, row_magnitude, again, tid,
+                               kCostThreads, present);
+    __syncthreads();
+    if (again.count > 0) {
+      FoldedColumnsAgain<W, H, KC>(A, plane_of, Lay::RowPitch, again, tid, kCostThreads);
+      __syncthreads();
+    }
   } else {
     BatchRowPassF<W, H, KC, false>(A, T, tid, kCostThreads, present);
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < kMaskLoads; ++q) {
-    const int i = tid + q * kCostThreads;
-    if (i < K * N && anchor_x[i / N] >= 0) mask[i] = pmask[q];
-  }
-  if constexpr (kExact) {
-    BatchColumnPass<W, H, KC, false>(T, B, tid, kCostThreads, present, staged);
-  } else {
+    __syncthreads();
     BatchColumnPassF<W, H, KC, false>(T, B, tid, kCostThreads, present);
+    __syncthreads();
   }
-  __syncthreads();
 
   // Weighted eighth powers in pixel order; the exact mode keeps them in the
   // row-pass buffer (free once the column pass has read it), as `terms`
   // still holds the magnitude terms.
   float* loss_terms = kExact ? reinterpret_cast<float*>(T) : terms;
   static_assert(!kExact || 2 * Lay::Planes >= KC * Lay::TermPitch, "loss terms fit T");
-  for (int i = tid; i < KC * N; i += kCostThreads) {
-    const int kc = i / N, r = i % N, y = r / W, x = r % W, k = kc / 3, c = kc % 3;
+  const float offset = c == 0 ? 12.0f : c == 1 ? 0.0f : 4.0f;
+#pragma unroll
+  for (int q = 0; q < kPerThread; ++q) {
+    const int k = Lay::Candidate(t, q), r = Lay::Position(t, q), y = r / W, x = r % W;
     if (anchor_x[k] < 0) continue;
     const float m = mask[k * N + r];
-    if (!(IsFinite(m) && m > 0.0f)) RaiseError(p.error, kErrorNonFiniteInput);
-    const float offset = c == 0 ? 12.0f : c == 1 ? 0.0f : 4.0f;
-    float weighted = (m + offset) * B[kc * Lay::PlanePitch + y * Lay::RowPitch + x];
+    if (c == 0 && !(IsFinite(m) && m > 0.0f)) RaiseError(p.error, kErrorNonFiniteInput);
+    float weighted = (m + offset) * B[(k * 3 + c) * Lay::PlanePitch + y * Lay::RowPitch + x];
     weighted *= weighted;
     weighted *= weighted;
     weighted *= weighted;
-    loss_terms[kc * Lay::TermPitch + r] = weighted;
+    loss_terms[(k * 3 + c) * Lay::TermPitch + r] = weighted;
   }
   __syncthreads();
 
@@ -595,8 +645,8 @@ CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_cou
     const float mag[3] = {magnitude[tid][0], magnitude[tid][1], magnitude[tid][2]};
     const uint32_t nz[3] = {nonzero[tid][0], nonzero[tid][1], nonzero[tid][2]};
     const float ls[3] = {loss_sum[tid][0], loss_sum[tid][1], loss_sum[tid][2]};
-    const float result = CandidateCost<N, S::CW * S::CH, kExact>(p, mag, nz, ls, quant_norm[tid],
-                                                                  entropy[tid]);
+    const float result = CandidateCost<N, S::CW * S::CH, kExact>(p, mag, nz, ls,
+                                                                  scale[tid][1].y, entropy[tid]);
     if (p.batch != nullptr) {
       p.batch_costs[blockIdx.x * K + tid] = result;
     } else {
@@ -1081,134 +1131,139 @@ struct SearchParams {
   uint32_t* error;
 };
 
-__device__ __forceinline__ int CoveredW(int s) {
+__host__ __device__ constexpr int CoveredW(int s) {
   return s == kDct16x16 ? 2 : s == kDct32x32 ? 4 : s == kDct8x16 ? 2 : s == kDct32x16 ? 2
        : s == kDct16x32 ? 4 : 1;
 }
-__device__ __forceinline__ int CoveredH(int s) {
+__host__ __device__ constexpr int CoveredH(int s) {
   return s == kDct16x16 ? 2 : s == kDct32x32 ? 4 : s == kDct16x8 ? 2 : s == kDct32x16 ? 4
        : s == kDct16x32 ? 2 : 1;
 }
 
-// One tile's search state, in shared memory.
+// One tile's search state, in shared memory. Per cell: the strategy grid's
+// code, whether its transform starts on this row (bit 0) and column (bit 1),
+// the merge priority and the cost (a transform's at its anchor, else 0).
 struct TileState {
   float family_cost[kFamilyCount][64];  // the tile's candidate costs
   float cost[64];
   uint8_t cell[64];
+  uint8_t starts[64];
   uint8_t priority[64];
-  int tile_w, tile_h;
 };
+
+constexpr uint8_t kRowStart = 1, kColumnStart = 2;
 
 __device__ __forceinline__ uint8_t Encode(int s, bool anchor) {
   return static_cast<uint8_t>((s << 1) | (anchor ? 1 : 0));
 }
 
-__device__ void SetCells(TileState& t, int lx, int ly, int s) {
-  const int cw = CoveredW(s), ch = CoveredH(s);
-  for (int dy = 0; dy < ch; ++dy)
-    for (int dx = 0; dx < cw; ++dx) t.cell[(ly + dy) * 8 + lx + dx] = Encode(s, dx == 0 && dy == 0);
-}
-
-// SearchGrid::CrossesHorizontalBoundary / CrossesVerticalBoundary
-// (ac_strategy.cpp:155-200), restricted to the tile (which they never leave).
-// kAligned: the start lies on its region's first column (row) and no transform
-// reaches into the region from before it, so a start that is no anchor crosses
-// and nothing outside the region is read.
-template <bool kAligned>
-__device__ bool CrossesHorizontal(const TileState& t, int start_x, int y, int end_x) {
-  if (start_x >= t.tile_w || y >= t.tile_h || y % 8 == 0) return false;
-  end_x = min(end_x, t.tile_w);
-  while (!kAligned && start_x != 0 && !(t.cell[y * 8 + start_x] & 1)) --start_x;
-  for (int x = start_x; x < end_x;) {
-    const uint8_t c = t.cell[y * 8 + x];
-    if (!(c & 1)) return true;
-    x += CoveredW(c >> 1);
+// Places a transform of strategy kStrategy with its cost.
+template <int kStrategy>
+__device__ __forceinline__ void Place(TileState& t, int lx, int ly, float cost) {
+  constexpr int kWidth = CoveredW(kStrategy), kHeight = CoveredH(kStrategy);
+#pragma unroll
+  for (int dy = 0; dy < kHeight; ++dy) {
+#pragma unroll
+    for (int dx = 0; dx < kWidth; ++dx) {
+      const int i = (ly + dy) * 8 + lx + dx;
+      t.cell[i] = Encode(kStrategy, dx == 0 && dy == 0);
+      t.starts[i] = (dy == 0 ? kRowStart : 0) | (dx == 0 ? kColumnStart : 0);
+      t.cost[i] = dx == 0 && dy == 0 ? cost : 0.0f;
+    }
   }
-  return false;
 }
 
-template <bool kAligned>
-__device__ bool CrossesVertical(const TileState& t, int x, int start_y, int end_y) {
-  if (x >= t.tile_w || start_y >= t.tile_h || x % 8 == 0) return false;
-  end_y = min(end_y, t.tile_h);
-  while (!kAligned && start_y != 0 && !(t.cell[start_y * 8 + x] & 1)) --start_y;
-  for (int y = start_y; y < end_y;) {
-    const uint8_t c = t.cell[y * 8 + x];
-    if (!(c & 1)) return true;
-    y += CoveredH(c >> 1);
-  }
-  return false;
+// The cells whose transforms start on their row / column, as 64-bit masks
+// over the tile (bit 8 y + x). A transform crosses the boundary above row y
+// (left of column x) where a cell of that row (column) does not start there,
+// which is what SearchGrid::CrossesHorizontalBoundary and
+// CrossesVerticalBoundary (ac_strategy.cpp:155-200) find by walking the row's
+// (column's) anchors.
+struct StartMasks {
+  uint64_t row, column;
+};
+
+template <int kStrategy>
+__device__ __forceinline__ void Mark(StartMasks& m, int lx, int ly) {
+  constexpr int kWidth = CoveredW(kStrategy), kHeight = CoveredH(kStrategy);
+  constexpr uint64_t kRow = (1u << kWidth) - 1u;
+  constexpr uint64_t kColumn = kHeight == 4 ? 0x01010101u : kHeight == 2 ? 0x0101u : 1u;
+  const int at = ly * 8 + lx;
+  m.row = (m.row & ~((kRow * kColumn) << at)) | (kRow << at);
+  m.column = (m.column & ~((kRow * kColumn) << at)) | (kColumn << at);
 }
 
-__device__ float Cost(const SearchParams& p, const TileState& t, int s, int lx, int ly) {
+// Boundary above row y (left of column x) over kCells cells from x (y), which
+// lie inside the tile; the tile's own first row and column are no boundary.
+template <int kCells>
+__device__ __forceinline__ bool CrossesHorizontal(const StartMasks& m, int x, int y, int h) {
+  if (y >= h || y % 8 == 0) return false;
+  return ((~m.row >> (y * 8 + x)) & ((1u << kCells) - 1u)) != 0;
+}
+template <int kCells>
+__device__ __forceinline__ bool CrossesVertical(const StartMasks& m, int x, int y, int w) {
+  if (x >= w || x % 8 == 0) return false;
+  constexpr uint64_t kColumn = kCells == 4 ? 0x01010101u : 0x0101u;
+  return ((~m.column >> (y * 8 + x)) & kColumn) != 0;
+}
+
+__device__ __forceinline__ float Cost(const SearchParams& p, const TileState& t, int s, int lx,
+                                      int ly) {
   const float v = t.family_cost[FamilyOfStrategy(s)][ly * 8 + lx];
   if (!(IsFinite(v) && v >= 0.0f)) RaiseError(p.error, kErrorInternal);
   return v;
 }
 
-__device__ void SetCost(TileState& t, int lx, int ly, int s, float cost) {
-  const int cw = CoveredW(s), ch = CoveredH(s);
-  for (int dy = 0; dy < ch; ++dy)
-    for (int dx = 0; dx < cw; ++dx) t.cost[(ly + dy) * 8 + lx + dx] = 0.0f;
-  t.cost[ly * 8 + lx] = cost;
-}
-
 // TryMerge (ac_strategy.cpp:340-386).
-__device__ void TryMerge(const SearchParams& p, TileState& t, int s, int lx, int ly,
-                         uint8_t priority) {
-  const int cw = CoveredW(s), ch = CoveredH(s);
+template <int kStrategy>
+__device__ void TryMerge(const SearchParams& p, TileState& t, int lx, int ly, uint8_t priority) {
+  constexpr int kWidth = CoveredW(kStrategy), kHeight = CoveredH(kStrategy);
   float current = 0.0f;
-  for (int dy = 0; dy < ch; ++dy) {
-    for (int dx = 0; dx < cw; ++dx) {
+  for (int dy = 0; dy < kHeight; ++dy) {
+    for (int dx = 0; dx < kWidth; ++dx) {
       const int i = (ly + dy) * 8 + lx + dx;
       if (t.priority[i] >= priority) return;
       current += t.cost[i];
     }
   }
-  const float candidate = Cost(p, t, s, lx, ly);
+  const float candidate = Cost(p, t, kStrategy, lx, ly);
   if (!(candidate < current)) return;
-  for (int dy = 0; dy < ch; ++dy) {
-    for (int dx = 0; dx < cw; ++dx) {
-      const int i = (ly + dy) * 8 + lx + dx;
-      t.cost[i] = 0.0f;
-      t.priority[i] = priority;
-    }
+  for (int dy = 0; dy < kHeight; ++dy) {
+    for (int dx = 0; dx < kWidth; ++dx) t.priority[(ly + dy) * 8 + lx + dx] = priority;
   }
-  SetCells(t, lx, ly, s);
-  t.cost[ly * 8 + lx] = candidate;
+  Place<kStrategy>(t, lx, ly, candidate);
 }
 
-// FindBestFirstLevelDivision (ac_strategy.cpp:406-589). kAligned: the square
-// is one of the aligned ones during the aligned passes, whose borders nothing
-// crosses.
-template <bool kAligned>
-__device__ void FirstLevelDivision(const SearchParams& p, TileState& t, int blocks, int lx,
-                                   int ly) {
-  const int half = blocks / 2;
-  if (!kAligned && (CrossesHorizontal<false>(t, lx, ly, lx + blocks) ||
-                    CrossesHorizontal<false>(t, lx, ly + blocks, lx + blocks) ||
-                    CrossesVertical<false>(t, lx, ly, ly + blocks) ||
-                    CrossesVertical<false>(t, lx + blocks, ly, ly + blocks))) {
-    return;
-  }
-  const bool allow_vertical = !CrossesVertical<kAligned>(t, lx + half, ly, ly + blocks);
-  const bool allow_horizontal = !CrossesHorizontal<kAligned>(t, lx, ly + half, lx + blocks);
+// FindBestFirstLevelDivision (ac_strategy.cpp:406-589) of a square of kBlocks
+// blocks whose borders no transform crosses; allow_vertical (_horizontal): no
+// transform crosses its middle column (row) boundary either. placed(strategy,
+// x, y) reports each placement.
+template <int kBlocks, typename Placed>
+__device__ __forceinline__ void FirstLevelDivision(const SearchParams& p, TileState& t, int lx,
+                                                   int ly, bool allow_vertical,
+                                                   bool allow_horizontal, Placed placed) {
+  constexpr int kHalf = kBlocks / 2;
+  constexpr int vs = kBlocks == 2 ? kDct16x8 : kDct32x16;
+  constexpr int hs = kBlocks == 2 ? kDct8x16 : kDct16x32;
+  constexpr int ss = kBlocks == 2 ? kDct16x16 : kDct32x32;
   float quadrant[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
-  for (int dy = 0; dy < blocks; ++dy)
-    for (int dx = 0; dx < blocks; ++dx)
-      quadrant[dy / half][dx / half] += t.cost[(ly + dy) * 8 + lx + dx];
+#pragma unroll
+  for (int dy = 0; dy < kBlocks; ++dy) {
+#pragma unroll
+    for (int dx = 0; dx < kBlocks; ++dx) {
+      quadrant[dy / kHalf][dx / kHalf] += t.cost[(ly + dy) * 8 + lx + dx];
+    }
+  }
   const float kUnavailable = 3.40282347e+38f;
   float vl = kUnavailable, vr = kUnavailable, ht = kUnavailable, hb = kUnavailable;
-  const int vs = blocks == 2 ? kDct16x8 : kDct32x16;
-  const int hs = blocks == 2 ? kDct8x16 : kDct16x32;
-  const int ss = blocks == 2 ? kDct16x16 : kDct32x32;
+  const int strategy = t.cell[ly * 8 + lx] >> 1;
   if (allow_vertical) {
-    if ((t.cell[ly * 8 + lx] >> 1) != vs) vl = Cost(p, t, vs, lx, ly);
-    if ((t.cell[ly * 8 + lx + half] >> 1) != vs) vr = Cost(p, t, vs, lx + half, ly);
+    if (strategy != vs) vl = Cost(p, t, vs, lx, ly);
+    if ((t.cell[ly * 8 + lx + kHalf] >> 1) != vs) vr = Cost(p, t, vs, lx + kHalf, ly);
   }
   if (allow_horizontal) {
-    if ((t.cell[ly * 8 + lx] >> 1) != hs) ht = Cost(p, t, hs, lx, ly);
-    if ((t.cell[(ly + half) * 8 + lx] >> 1) != hs) hb = Cost(p, t, hs, lx, ly + half);
+    if (strategy != hs) ht = Cost(p, t, hs, lx, ly);
+    if ((t.cell[(ly + kHalf) * 8 + lx] >> 1) != hs) hb = Cost(p, t, hs, lx, ly + kHalf);
   }
   const float square = Cost(p, t, ss, lx, ly);
   const float vertical_cost = fminf(vl, quadrant[0][0] + quadrant[1][0]) +
@@ -1217,27 +1272,60 @@ __device__ void FirstLevelDivision(const SearchParams& p, TileState& t, int bloc
                                 fminf(hb, quadrant[1][0] + quadrant[1][1]);
   // ChooseFirstLevelDivision (ac_strategy_search_policy.h:69-83).
   if (square < vertical_cost && square < horizontal_cost) {
-    SetCells(t, lx, ly, ss);
-    SetCost(t, lx, ly, ss, square);
+    Place<ss>(t, lx, ly, square);
+    placed(std::integral_constant<int, ss>(), lx, ly);
   } else if (vertical_cost < horizontal_cost) {
     if (vl < quadrant[0][0] + quadrant[1][0]) {
-      SetCells(t, lx, ly, vs);
-      SetCost(t, lx, ly, vs, vl);
+      Place<vs>(t, lx, ly, vl);
+      placed(std::integral_constant<int, vs>(), lx, ly);
     }
     if (vr < quadrant[0][1] + quadrant[1][1]) {
-      SetCells(t, lx + half, ly, vs);
-      SetCost(t, lx + half, ly, vs, vr);
+      Place<vs>(t, lx + kHalf, ly, vr);
+      placed(std::integral_constant<int, vs>(), lx + kHalf, ly);
     }
   } else {
     if (ht < quadrant[0][0] + quadrant[0][1]) {
-      SetCells(t, lx, ly, hs);
-      SetCost(t, lx, ly, hs, ht);
+      Place<hs>(t, lx, ly, ht);
+      placed(std::integral_constant<int, hs>(), lx, ly);
     }
     if (hb < quadrant[1][0] + quadrant[1][1]) {
-      SetCells(t, lx, ly + half, hs);
-      SetCost(t, lx, ly + half, hs, hb);
+      Place<hs>(t, lx, ly + kHalf, hb);
+      placed(std::integral_constant<int, hs>(), lx, ly + kHalf);
     }
   }
+}
+
+// One aligned square during the aligned passes: nothing crosses its borders,
+// and its middle boundaries are crossed where one of its own cells does not
+// start there.
+template <int kBlocks>
+__device__ __forceinline__ void AlignedDivision(const SearchParams& p, TileState& t, int lx,
+                                                int ly) {
+  constexpr int kHalf = kBlocks / 2;
+  bool allow_vertical = true, allow_horizontal = true;
+#pragma unroll
+  for (int i = 0; i < kBlocks; ++i) {
+    allow_vertical &= (t.starts[(ly + i) * 8 + lx + kHalf] & kColumnStart) != 0;
+    allow_horizontal &= (t.starts[(ly + kHalf) * 8 + lx + i] & kRowStart) != 0;
+  }
+  FirstLevelDivision<kBlocks>(p, t, lx, ly, allow_vertical, allow_horizontal,
+                              [](auto, int, int) {});
+}
+
+// One square of the unaligned passes.
+template <int kBlocks>
+__device__ __forceinline__ void UnalignedDivision(const SearchParams& p, TileState& t,
+                                                  StartMasks& m, int lx, int ly, int w, int h) {
+  if (CrossesHorizontal<kBlocks>(m, lx, ly, h) || CrossesHorizontal<kBlocks>(m, lx, ly + kBlocks, h) ||
+      CrossesVertical<kBlocks>(m, lx, ly, w) || CrossesVertical<kBlocks>(m, lx + kBlocks, ly, w)) {
+    return;
+  }
+  FirstLevelDivision<kBlocks>(p, t, lx, ly,
+                              !CrossesVertical<kBlocks>(m, lx + kBlocks / 2, ly, w),
+                              !CrossesHorizontal<kBlocks>(m, lx, ly + kBlocks / 2, h),
+                              [&](auto strategy, int x, int y) {
+                                Mark<decltype(strategy)::value>(m, x, y);
+                              });
 }
 
 // SearchTile (ac_strategy.cpp:591-773), one warp per tile.
@@ -1251,7 +1339,8 @@ __device__ void FirstLevelDivision(const SearchParams& p, TileState& t, int bloc
 // only, so the order among them does not matter. The unaligned passes
 // overlap their predecessors and stay in raster order on lane 0. One thread
 // per tile with every cost a dependent global load took 241 us at 256x256
-// and 243 us at 2048x1536.
+// and 243 us at 2048x1536; lane 0 walking the grid's cells for every boundary
+// (instead of the two masks it keeps in registers) 86 us.
 constexpr int kSearchWarps = 4;
 
 __global__ void __launch_bounds__(32 * kSearchWarps)
@@ -1276,16 +1365,13 @@ SearchTileKernel(const __grid_constant__ SearchParams p) {
                                     : 0.0f;
     }
   }
-  if (lane == 0) {
-    t.tile_w = w;
-    t.tile_h = h;
-  }
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     const int i = lane + 32 * q;
 #pragma unroll
     for (int f = 0; f < kFamilyCount; ++f) t.family_cost[f][i] = loaded[f][q];
     t.cell[i] = Encode(kDct8, true);
+    t.starts[i] = kRowStart | kColumnStart;
     t.priority[i] = 0;
     t.cost[i] = i % 8 < w && i / 8 < h ? Cost(p, t, kDct8, i % 8, i / 8) * p.baseline_multiplier
                                        : 0.0f;
@@ -1297,11 +1383,11 @@ SearchTileKernel(const __grid_constant__ SearchParams p) {
   if (lane < 16) {
     const int x = (lane % 4) * 2, y = (lane / 4) * 2;
     if (x + 1 < w && y + 1 < h) {
-      FirstLevelDivision<true>(p, t, 2, x, y);
+      AlignedDivision<2>(p, t, x, y);
     } else if (x + 1 == w && y + 1 < h) {
-      TryMerge(p, t, kDct16x8, x, y, 2);
+      TryMerge<kDct16x8>(p, t, x, y, 2);
     } else if (x + 1 < w && y + 1 == h) {
-      TryMerge(p, t, kDct8x16, x, y, 2);
+      TryMerge<kDct8x16>(p, t, x, y, 2);
     }
   }
   __syncwarp();
@@ -1310,21 +1396,28 @@ SearchTileKernel(const __grid_constant__ SearchParams p) {
   if (lane < 4) {
     const int x = (lane % 2) * 4, y = (lane / 2) * 4;
     if (x + 3 < w && y + 3 < h) {
-      FirstLevelDivision<true>(p, t, 4, x, y);
+      AlignedDivision<4>(p, t, x, y);
     } else if (x + 3 < w && y + 1 < h) {
-      TryMerge(p, t, kDct16x32, x, y, 4);
+      TryMerge<kDct16x32>(p, t, x, y, 4);
     } else if (x + 1 < w && y + 3 < h) {
-      TryMerge(p, t, kDct32x16, x, y, 4);
+      TryMerge<kDct32x16>(p, t, x, y, 4);
     }
   }
   __syncwarp();
+  const uint32_t rows_low = __ballot_sync(0xffffffffu, (t.starts[lane] & kRowStart) != 0);
+  const uint32_t rows_high = __ballot_sync(0xffffffffu, (t.starts[lane + 32] & kRowStart) != 0);
+  const uint32_t columns_low = __ballot_sync(0xffffffffu, (t.starts[lane] & kColumnStart) != 0);
+  const uint32_t columns_high =
+    __ballot_sync(0xffffffffu, (t.starts[lane + 32] & kColumnStart) != 0);
   if (lane == 0) {
+    StartMasks m = {(static_cast<uint64_t>(rows_high) << 32) | rows_low,
+                    (static_cast<uint64_t>(columns_high) << 32) | columns_low};
     for (int y = 0; y + 1 < h; ++y)
       for (int x = 0; x + 1 < w; ++x)
-        if ((y | x) % 2 != 0) FirstLevelDivision<false>(p, t, 2, x, y);
+        if ((y | x) % 2 != 0) UnalignedDivision<2>(p, t, m, x, y, w, h);
     for (int y = 0; y + 3 < h; y += p.dct32_step)
       for (int x = 0; x + 3 < w; x += p.dct32_step)
-        if ((y | x) % 4 != 0) FirstLevelDivision<false>(p, t, 4, x, y);
+        if ((y | x) % 4 != 0) UnalignedDivision<4>(p, t, m, x, y, w, h);
   }
   __syncwarp();
 
@@ -1355,6 +1448,8 @@ int LaunchFamily(CostParams p, const DeviceTables& d, int family, cudaStream_t s
                            ? batch_count
                            : static_cast<uint32_t>(p.tiles_x * p.tiles_y * p.local_x * p.local_y);
   if (count == 0) return GJXL_B200_OK;
+  p.opsin_aligned = p.stride % 4 == 0 && p.pitch % 4 == 0 && Aligned16(p.opsin);
+  p.mask_aligned = p.mask_stride % 4 == 0 && Aligned16(p.pixel_mask);
   const size_t smem = CostLayout<W, H, Acc>::SharedBytes;
   int status = CheckCuda(cudaFuncSetAttribute(CandidateCostKernel<W, H, Acc>,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize,

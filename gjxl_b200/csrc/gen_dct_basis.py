@@ -46,6 +46,21 @@ def render() -> str:
     for n in (8, 16, 32):
         b = basis(n, True)
         tables.append((f"kDctForwardT{n}", [b[f * n + s] for s in range(n) for f in range(n)]))
+    # The inverse bases' first halves for the folded passes, [frequency * N / 2
+    # + sample]: the mean of the two table values that mirror one another, and
+    # how far either is from it.
+    folds = []
+    for n in (8, 16, 32):
+        b = basis(n, False)
+        half, error = [], 0.0
+        for u in range(n):
+            for x in range(n // 2):
+                near, far = b[u * n + x], b[u * n + n - 1 - x] * (-1.0 if u % 2 else 1.0)
+                mean = 0.5 * (near + far)
+                half.append(mean)
+                error = max(error, abs(near - mean), abs(far - mean))
+        tables.append((f"kDctInverseHalf{n}", half))
+        folds.append((n, error))
     staged = [(f"kDctStaged{name[4:]}", values) for name, values in tables
               if name in ("kDctForwardT32", "kDctInverse32")]
     for index, (name, values) in enumerate(tables + staged):
@@ -55,6 +70,10 @@ def render() -> str:
             lines.append("  " + ", ".join(v.hex() for v in values[i:i + 4]) + ",")
         lines.append("};")
         lines.append("")
+    lines.append("// Largest distance between an inverse basis value and its half-table entry.")
+    for n, error in folds:
+        lines.append(f"constexpr double kDctInverseHalfError{n} = {error.hex()};")
+    lines.append("")
     # Single-precision copies (each value rounded to nearest float) of the
     # lengths 8 and 16, for the FP32 transform passes of the fast cost mode.
     lines.append("// Rounded to float for the FP32 passes.")
