@@ -80,28 +80,24 @@ __device__ __forceinline__ float QuantBiasR(int32_t quantized, int channel) {
 
 __device__ __forceinline__ int LenIdx(int len) { return len == 1 ? 0 : len == 2 ? 1 : 2; }
 
-// ConvertDcToLowFrequencies for one channel of one transform.
+// ConvertDcToLowFrequencies: LLF coefficient (v, u) of one channel of one
+// transform from its CH x CW DC values.
 template <int W, int H>
-__device__ void DcToLowFrequencies(const float* dc_plane, int blocks_x, int ax, int ay,
-                                   float* plane, int row_pitch) {
+__device__ float DcToLowFrequency(const float* dc, int v, int u) {
   using S = TransformShape<W, H>;
   constexpr int CW = S::CW, CH = S::CH;
   const int lh = LenIdx(CH), lw = LenIdx(CW);
-  // LLF coefficient (v, u) lands at row v, column u of the natural plane.
-  for (int v = 0; v < CH; ++v) {
-    for (int u = 0; u < CW; ++u) {
-      double value = 0.0;
-      for (int y = 0; y < CH; ++y) {
-        for (int x = 0; x < CW; ++x) {
-          value += static_cast<double>(dc_plane[(ay + y) * blocks_x + ax + x]) *
-                   c_dc_recon.forward[lh][v][y] * c_dc_recon.forward[lw][u][x];
-        }
-      }
-      plane[v * row_pitch + u] =
-        static_cast<float>(value * static_cast<double>(c_dc_recon.upsample[lh][v]) *
-                           static_cast<double>(c_dc_recon.upsample[lw][u]));
+  double value = 0.0;
+#pragma unroll
+  for (int y = 0; y < CH; ++y) {
+#pragma unroll
+    for (int x = 0; x < CW; ++x) {
+      value += static_cast<double>(dc[y * CW + x]) * c_dc_recon.forward[lh][v][y] *
+               c_dc_recon.forward[lw][u][x];
     }
   }
+  return static_cast<float>(value * static_cast<double>(c_dc_recon.upsample[lh][v]) *
+                            static_cast<double>(c_dc_recon.upsample[lw][u]));
 }
 
 struct ReconParams {
@@ -124,7 +120,7 @@ struct ReconParams {
 };
 
 // K = 1024 / N transforms (3 channels each) per CTA of 384 threads; the
-// inverse DCT gives every thread one 8-output chunk of one line per pass
+// folded inverse DCT gives every thread 8 outputs of one line per pass
 // (line_dct.cuh). Coefficients sit at their natural (v, u) position of a
 // padded plane.
 constexpr int kReconThreads = 384;
@@ -142,6 +138,9 @@ __global__ void __launch_bounds__(kReconThreads, 2) ReconstructKernel(const __gr
   __shared__ float scales[K][3];
   __shared__ float factors[K][2];
   __shared__ float dc_values[K][3][S::CW * S::CH];  // the transforms' DC blocks
+  __shared__ __align__(16) float row_magnitude[KC * H];
+  __shared__ FoldedAgain<W, KC> again;  // columns to transform again
+  ClearAgain(again, threadIdx.x);
   const uint32_t first = blockIdx.x * K;
   // The anchor loads do not wait for the count: the list index is clamped to
   // the list, and anchors past the count are never used. Every later global
@@ -215,24 +214,27 @@ __global__ void __launch_bounds__(kReconThreads, 2) ReconstructKernel(const __gr
     coef[Batch::At(k * 3 + 2, v, u)] += factors[k][1] * y;
   }
   __syncthreads();
-  // LLF from the (smoothed) DC, one thread per transform channel.
-  if (threadIdx.x < active * 3) {
-    const int k = threadIdx.x / 3, c = threadIdx.x % 3;
-    DcToLowFrequencies<W, H>(dc_values[k][c], S::CW, 0, 0, coef + Batch::At(k * 3 + c, 0, 0),
-                             Batch::RowPitch);
+  // LLF from the (smoothed) DC, one thread per coefficient.
+  constexpr int kLlf = S::CW * S::CH;
+  static_assert(KC * kLlf <= kReconThreads, "one LLF coefficient per thread");
+  if (threadIdx.x < active * 3 * kLlf) {
+    const int plane = threadIdx.x / kLlf, i = threadIdx.x % kLlf;
+    coef[Batch::At(plane, i / S::CW, i % S::CW)] =
+      DcToLowFrequency<W, H>(dc_values[plane / 3][plane % 3], i / S::CW, i % S::CW);
   }
   __syncthreads();
   const auto present = [&](int plane) { return plane < 3 * active; };
-  BatchRowPass<W, H, KC, false>(coef, tmp, threadIdx.x, kReconThreads, present);
+  FoldedRowPass<W, H, KC>(coef, tmp, row_magnitude, threadIdx.x, kReconThreads, present);
   __syncthreads();
-  BatchColumnPass<W, H, KC, false>(tmp, coef, threadIdx.x, kReconThreads, present);
+  // The columns go straight to the image.
+  const auto image = [&](int plane) {
+    const int2 a = anchor[plane / 3];
+    return p.recon + plane % 3 * p.pitch + static_cast<size_t>(a.y) * 8 * p.stride + a.x * 8;
+  };
+  FoldedColumnPass<W, H, KC>(tmp, image, p.stride, row_magnitude, again, threadIdx.x,
+                             kReconThreads, present);
   __syncthreads();
-  for (int i = threadIdx.x; i < active * 3 * N; i += kReconThreads) {
-    const int k = i / (3 * N), r = i % (3 * N), c = r / N, yx = r % N;
-    const int2 a = anchor[k];
-    p.recon[c * p.pitch + static_cast<size_t>(a.y * 8 + yx / W) * p.stride + a.x * 8 + yx % W] =
-      coef[Batch::At(k * 3 + c, yx / W, yx % W)];
-  }
+  FoldedColumnsAgain<W, H, KC>(coef, image, p.stride, again, threadIdx.x, kReconThreads);
 }
 
 __device__ __forceinline__ int MirrorR(int c, int n) {
@@ -477,35 +479,68 @@ __global__ void OpsinToLinearKernel(const __grid_constant__ LinearParams p) {
   OpsinToLinearPixel(p, p.opsin[i], p.opsin[p.n + i], p.opsin[2 * p.n + i], i);
 }
 
-__global__ void BlockReduceKernel(const uint8_t* cells, int blocks_x, int blocks_y,
-                                  const float* map, int w, int h, float* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= blocks_x * blocks_y) return;
-  const uint8_t cell = cells[i];
-  if (!(cell & 1)) return;
-  const int f = StrategyFamily(cell >> 1);
-  const int cw = FamilyCoveredW(f), ch = FamilyCoveredH(f);
-  const int bx = i % blocks_x, by = i / blocks_x;
-  const int x0 = bx * 8, y0 = by * 8;
-  const int x1 = min(w, x0 + cw * 8), y1 = min(h, y0 + ch * 8);
-  float norm = 0.0f;
-  int count = 0;
-  for (int y = y0; y < y1; ++y) {
-    for (int x = x0; x < x1; ++x) {
-      float v = map[static_cast<size_t>(y) * w + x];
-      v *= v;
-      v *= v;
-      v *= v;
-      v *= v;
-      norm += v;
-      ++count;
+// Eight lanes per block: a row segment of eight pixels is loaded and raised to
+// the 16th power by the lanes together and added in raster order through
+// shuffles, four segments' loads in flight; the 32 roots of a CTA are then
+// taken by one warp. Bound: latency (a 32x32 transform is 1024 dependent
+// adds). One thread per block with its pixels' loads one row apart took 43 us
+// at 256x256 and 62 us at 2048x1536.
+constexpr int kReduceBlocks = 32;  // blocks per CTA
+constexpr int kReduceLanes = 8;
+
+__global__ void __launch_bounds__(kReduceBlocks * kReduceLanes)
+BlockReduceKernel(const uint8_t* cells, int blocks_x, int blocks_y, const float* map, int w,
+                  int h, float* out) {
+  __shared__ float means[kReduceBlocks];
+  __shared__ int families[kReduceBlocks];  // -1: no anchor
+  const int slot = threadIdx.x / kReduceLanes, lane = threadIdx.x % kReduceLanes;
+  const int i = blockIdx.x * kReduceBlocks + slot;
+  int f = -1;
+  if (i < blocks_x * blocks_y && (cells[i] & 1)) f = StrategyFamily(cells[i] >> 1);
+  if (lane == 0) families[slot] = f;
+  if (f >= 0) {
+    const unsigned group = 0xFFu << (threadIdx.x % 32 - lane);
+    const int x0 = i % blocks_x * 8, y0 = i / blocks_x * 8;
+    const int columns = FamilyCoveredW(f);
+    const int x1 = min(w, x0 + columns * 8), y1 = min(h, y0 + FamilyCoveredH(f) * 8);
+    // Segments in raster order: segment s is columns 8 (s % columns) .. + 7
+    // of row s / columns. Pixels past the image's right edge count as zeros,
+    // which leave the sum as it is.
+    const int segments = (y1 - y0) * columns;
+    float norm = 0.0f;
+    for (int s0 = 0; s0 < segments; s0 += 4) {
+      float v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int x = x0 + (s0 + k) % columns * 8 + lane, y = y0 + (s0 + k) / columns;
+        v[k] = y < y1 && x < x1 ? map[static_cast<size_t>(y) * w + x] : 0.0f;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        v[k] *= v[k];
+        v[k] *= v[k];
+        v[k] *= v[k];
+        v[k] *= v[k];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+#pragma unroll
+        for (int j = 0; j < kReduceLanes; ++j) {
+          norm += __shfl_sync(group, v[k], j, kReduceLanes);
+        }
+      }
     }
+    if (lane == 0) means[slot] = norm / static_cast<float>((x1 - x0) * (y1 - y0));
   }
+  __syncthreads();
+  if (threadIdx.x >= kReduceBlocks || families[threadIdx.x] < 0) return;
   // std::pow(float, 1/16): evaluated in double and rounded to float.
-  const float mean = norm / static_cast<float>(count);
-  const float d = 1.2f * static_cast<float>(pow(static_cast<double>(mean), 0.0625));
+  const float d =
+    1.2f * static_cast<float>(pow(static_cast<double>(means[threadIdx.x]), 0.0625));
+  const int block = blockIdx.x * kReduceBlocks + threadIdx.x;
+  const int cw = FamilyCoveredW(families[threadIdx.x]), ch = FamilyCoveredH(families[threadIdx.x]);
   for (int dy = 0; dy < ch; ++dy)
-    for (int dx = 0; dx < cw; ++dx) out[(by + dy) * blocks_x + bx + dx] = d;
+    for (int dx = 0; dx < cw; ++dx) out[block + dy * blocks_x + dx] = d;
 }
 
 __global__ void PolicyUpdateKernel(float* field, const float* adjusted_initial,
@@ -701,7 +736,8 @@ int AqOpsinToLinear(const float* opsin, size_t width, size_t height, float inten
 
 int AqBlockReduce(const uint8_t* cells, size_t bx, size_t by, const float* distance_map,
                   size_t width, size_t height, float* block_distance, cudaStream_t stream) {
-  BlockReduceKernel<<<Blocks(bx * by), kThreads, 0, stream>>>(
+  const unsigned ctas = static_cast<unsigned>((bx * by + kReduceBlocks - 1) / kReduceBlocks);
+  BlockReduceKernel<<<ctas, kReduceBlocks * kReduceLanes, 0, stream>>>(
     cells, static_cast<int>(bx), static_cast<int>(by), distance_map, static_cast<int>(width),
     static_cast<int>(height), block_distance);
   return CheckLaunch("aq block reduce");
