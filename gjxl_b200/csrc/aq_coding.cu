@@ -341,13 +341,128 @@ __device__ AqQuantizer MakeQuantizer(float median, float mad, float quant_dc, bo
     q.dc_steps[c] = inverse_quant_dc / kInverseDcQuant[c];
     q.inverse_dc_steps[c] = kInverseDcQuant[c] * q.scale * static_cast<float>(qdc);
   }
+  return q;
+}
+
+__device__ __forceinline__ int32_t RawQuant(float field, float inverse_global_scale) {
+  const float v = field * inverse_global_scale + 0.5f;
+  return static_cast<int32_t>(fminf(fmaxf(v, 1.0f), 256.0f));
+}
+
+__global__ void QuantizerKernel(const SelectState* st, const AqPolicy* policy, AqQuantizer* q,
+                                uint32_t* error) {
+  bool in_range;
+  *q = MakeQuantizer(__uint_as_float(st->median_bits), __uint_as_float(st->mad_bits),
+                     policy->quant_dc, &in_range);
+  if (!in_range) RaiseError(error, kErrorRange);
 }
 
 __global__ void RawQuantKernel(const float* field, int n, const AqQuantizer* q, int32_t* raw) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float v = field[i] * q->inverse_global_scale + 0.5f;
-  raw[i] = static_cast<int32_t>(fminf(fmaxf(v, 1.0f), 256.0f));
+  raw[i] = RawQuant(field[i], q->inverse_global_scale);
+}
+
+// Both selections, the quantizer and the raw field in one launch, for fields
+// that one cluster's shared memory holds.
+//
+// Bound: launch latency (the field is at most 1.6 MB, and every pass but the
+// first counts a fraction of it): as grid-wide histogram and digit kernels
+// the same took 15 launches, 42 us per evaluation at 256x256 (three
+// evaluations an analysis). Each CTA keeps its share of the field; per pass
+// the CTAs of the cluster count into their own histograms, and after one
+// cluster barrier every CTA sums all of them over distributed shared memory
+// and scans the sum itself. The histograms alternate, so that one may be
+// cleared while a slower CTA still reads the other.
+constexpr int kSelectThreads = 1024;
+constexpr int kSelectCluster = 8;          // largest (portable) cluster
+constexpr int kSelectShare = 50 * 1024;    // field values per CTA (200 KB)
+constexpr int kSelectSmallShare = 4096;    // values per CTA below the largest cluster
+static_assert(2 * kSelectThreads == kSelectBins, "two bins per thread");
+
+__global__ void __launch_bounds__(kSelectThreads)
+ClusterQuantizerKernel(const float* field, int n, int share, const AqPolicy* policy,
+                       AqQuantizer* q, int32_t* raw, uint32_t* error) {
+  extern __shared__ float values[];
+  __shared__ uint32_t histogram[2][kSelectBins];
+  __shared__ uint32_t warp_sums[32], chosen_digit, chosen_before;
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int ctas = static_cast<int>(cluster.num_blocks());
+  const int t = threadIdx.x, lane = t % 32, warp = t / 32;
+  const int begin = static_cast<int>(cluster.block_rank()) * share;
+  const int count = max(0, min(share, n - begin));
+  for (int i = t; i < count; i += kSelectThreads) values[i] = field[begin + i];
+  for (int b = t; b < 2 * kSelectBins; b += kSelectThreads) (&histogram[0][0])[b] = 0;
+  __syncthreads();
+  uint32_t selected[2];  // median, then median absolute deviation
+  int buffer = 0;
+#pragma unroll
+  for (int selection = 0; selection < 2; ++selection) {
+    const float center = selection == 0 ? 0.0f : __uint_as_float(selected[0]);
+    uint32_t prefix = 0, mask = 0, k = static_cast<uint32_t>(n / 2);
+    for (int pass = 0; pass < kSelectPasses; ++pass, buffer ^= 1) {
+      const int shift = SelectShift(pass);
+      const uint32_t digit_mask = (1u << SelectBits(pass)) - 1u;
+      for (int i = t; i < count; i += kSelectThreads) {
+        const uint32_t bits = SelectKey(values, i, selection == 1, center);
+        if ((bits & mask) == prefix) atomicAdd(&histogram[buffer][(bits >> shift) & digit_mask], 1u);
+      }
+      cluster.sync();
+      uint32_t h0 = 0, h1 = 0;
+      for (int r = 0; r < ctas; ++r) {
+        const uint2 h =
+          reinterpret_cast<const uint2*>(cluster.map_shared_rank(&histogram[buffer][0], r))[t];
+        h0 += h.x;
+        h1 += h.y;
+      }
+      reinterpret_cast<uint2*>(&histogram[buffer ^ 1][0])[t] = make_uint2(0, 0);
+      uint32_t inclusive = h0 + h1;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inclusive, o);
+        if (lane >= o) inclusive += v;
+      }
+      if (lane == 31) warp_sums[warp] = inclusive;
+      __syncthreads();
+      if (warp == 0) {
+        uint32_t w = warp_sums[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t v = __shfl_up_sync(0xffffffffu, w, o);
+          if (lane >= o) w += v;
+        }
+        warp_sums[lane] = w;
+      }
+      __syncthreads();
+      // Exactly one (thread, bin) has before <= k < before + its count.
+      const uint32_t before = inclusive - (h0 + h1) + (warp ? warp_sums[warp - 1] : 0u);
+      if (k >= before && k < before + h0) {
+        chosen_digit = static_cast<uint32_t>(2 * t);
+        chosen_before = before;
+      } else if (k >= before + h0 && k < before + h0 + h1) {
+        chosen_digit = static_cast<uint32_t>(2 * t + 1);
+        chosen_before = before + h0;
+      }
+      __syncthreads();
+      prefix |= chosen_digit << shift;
+      k -= chosen_before;
+      mask |= digit_mask << shift;
+    }
+    selected[selection] = prefix;
+  }
+  // No CTA leaves while another may still read its histograms.
+  cluster.sync();
+  bool in_range;
+  const AqQuantizer made = MakeQuantizer(__uint_as_float(selected[0]),
+                                         __uint_as_float(selected[1]), policy->quant_dc,
+                                         &in_range);
+  if (begin == 0 && t == 0) {
+    *q = made;
+    if (!in_range) RaiseError(error, kErrorRange);
+  }
+  for (int i = t; i < count; i += kSelectThreads) {
+    raw[begin + i] = RawQuant(values[i], made.inverse_global_scale);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -746,6 +861,7 @@ __device__ float LowFrequencyDc(const float* coef, int y, int x) {
   double value = 0.0;
 #pragma unroll
   for (int v = 0; v < CH; ++v) {
+#pragma unroll
     for (int u = 0; u < CW; ++u) {
       const double scaled = static_cast<double>(coef[S::Index(v, u)]) *
                             static_cast<double>(c_dc_tables.downsample[lh][v]) *
@@ -753,6 +869,7 @@ __device__ float LowFrequencyDc(const float* coef, int y, int x) {
       value += scaled * c_dc_tables.inverse[lh][v][y] * c_dc_tables.inverse[lw][u][x];
     }
   }
+  return static_cast<float>(value);
 }
 
 // AdjustQuantizationBias (quantization.cpp:203-218).
@@ -786,6 +903,34 @@ struct CodingParams {
   const float* matrix_multiplier;  // device, X / Y / B
   uint32_t* error;
 };
+
+// t[0] + t[1] + ... + t[N-1] in order, 16 terms at a time with the next 16
+// loaded during the adds; `t` 16-byte aligned.
+template <int N>
+__device__ __forceinline__ float CodingOrderedSum(const float* t) {
+  static_assert(N % 16 == 0, "whole groups");
+  const float4* v = reinterpret_cast<const float4*>(t);
+  float4 now[4], next[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) now[k] = next[k] = v[k];
+  float sum = 0.0f;
+#pragma unroll 2
+  for (int j = 0; j < N / 4; j += 4) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (j + 4 < N / 4) next[k] = v[j + 4 + k];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      sum += now[k].x;
+      sum += now[k].y;
+      sum += now[k].z;
+      sum += now[k].w;
+      now[k] = next[k];
+    }
+  }
+  return sum;
+}
 
 // ComputeQuantizedCoefficientsImpl's per-transform body
 // (reconstruction.cpp:480-700), one CTA of 64 threads per anchor.
@@ -858,7 +1003,6 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
   using Sh = TransformShape<W, H>;
   constexpr int xsize = Sh::SW / 8, ysize = Sh::SH / 8;
   const float qac = q.scale * static_cast<float>(initial_raw);
-#pragma unroll
   float t0[4];
   AdjustThresholds<W, H>(t0);
   {
@@ -878,7 +1022,6 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
         }
         const int quadrant = (y >= Sh::SH / 2) * 2 + (x >= Sh::SW / 2);
         const float value = coef[c][index] * (inverse_dequant[c][index] * qac * mm);
-  return static_cast<float>(value);
         const float quantized = fabsf(value) < t0[quadrant] ? 0.0f : rintf(value);
         const float err = fabsf(value - quantized);
         adjust_err[c][index] = err;
@@ -898,6 +1041,24 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
       }
       if (sums[c][0] >= (1u << 24)) big = true;
     }
+    for (int i = tid; i < 3 * kBorder; i += kT) {
+      const int c = i / kBorder, j = i % kBorder;
+      constexpr int kColumn = 3 * ysize, kCorner = (ysize - 1) * xsize;
+      int y = Sh::SH - 1, x = 4 * xsize + j - kColumn - kCorner;
+      if (j < kColumn) {
+        y = 4 * ysize + j;
+        x = Sh::SW - 1;
+      } else if (j < kColumn + kCorner) {
+        y = 7 * ysize + (j - kColumn) / xsize;
+        x = 7 * xsize + (j - kColumn) % xsize;
+      }
+      const int index = y * Sh::SW + x;
+      const int quadrant = (y >= Sh::SH / 2) * 2 + (x >= Sh::SW / 2);
+      const float mm = c == 0 ? mm0 : c == 1 ? mm1 : mm2;
+      const float value = coef[c][index] * (inverse_dequant[c][index] * qac * mm);
+      const float quantized = fabsf(value) < t0[quadrant] ? 0.0f : rintf(value);
+      border[c][j] = quantized != 0.0f ? fabsf(value) : 0.0f;
+    }
     const int warp = tid / 32, lane = tid % 32;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -913,34 +1074,6 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
       if (lane == 0) adjust_max[warp][k] = m;
     }
     const bool any_big = __any_sync(0xffffffffu, big);
-// t[0] + t[1] + ... + t[N-1] in order, 16 terms at a time with the next 16
-// loaded during the adds; `t` 16-byte aligned.
-template <int N>
-__device__ __forceinline__ float CodingOrderedSum(const float* t) {
-  static_assert(N % 16 == 0, "whole groups");
-  const float4* v = reinterpret_cast<const float4*>(t);
-  float4 now[4], next[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) now[k] = next[k] = v[k];
-  float sum = 0.0f;
-#pragma unroll 2
-  for (int j = 0; j < N / 4; j += 4) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (j + 4 < N / 4) next[k] = v[j + 4 + k];
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      sum += now[k].x;
-      sum += now[k].y;
-      sum += now[k].z;
-      sum += now[k].w;
-      now[k] = next[k];
-    }
-  }
-  return sum;
-}
-
     if (lane == 0) adjust_big[warp] = any_big ? 1 : 0;
   }
   __syncthreads();
@@ -1024,24 +1157,6 @@ __device__ __forceinline__ float CodingOrderedSum(const float* t) {
 
 // ---------------------------------------------------------------------------
 // Prediction-aware DC quantization with the weighted predictor.
-    for (int i = tid; i < 3 * kBorder; i += kT) {
-      const int c = i / kBorder, j = i % kBorder;
-      constexpr int kColumn = 3 * ysize, kCorner = (ysize - 1) * xsize;
-      int y = Sh::SH - 1, x = 4 * xsize + j - kColumn - kCorner;
-      if (j < kColumn) {
-        y = 4 * ysize + j;
-        x = Sh::SW - 1;
-      } else if (j < kColumn + kCorner) {
-        y = 7 * ysize + (j - kColumn) / xsize;
-        x = 7 * xsize + (j - kColumn) % xsize;
-      }
-      const int index = y * Sh::SW + x;
-      const int quadrant = (y >= Sh::SH / 2) * 2 + (x >= Sh::SW / 2);
-      const float mm = c == 0 ? mm0 : c == 1 ? mm1 : mm2;
-      const float value = coef[c][index] * (inverse_dequant[c][index] * qac * mm);
-      const float quantized = fabsf(value) < t0[quadrant] ? 0.0f : rintf(value);
-      border[c][j] = quantized != 0.0f ? fabsf(value) : 0.0f;
-    }
 //
 // The reference walks each 256x256-block DC group in raster order, channel
 // by channel (Y, X, B), resetting the predictor per channel. A sample at
@@ -1220,43 +1335,36 @@ DcQuantKernel(const __grid_constant__ DcQuantParams p) {
   // The sample of the next position is loaded one wave ahead, so its
   // global-memory latency overlaps this wave's work and barrier.
   const size_t row_index = static_cast<size_t>(gy0 + min(y, gh - 1)) * stride + gx0;
-  const uint32_t* source = (kReplay ? reinterpret_cast<const uint32_t*>(p.replay)
-                                    : reinterpret_cast<const uint32_t*>(p.dc)) +
-                           c * p.pitch + row_index;
-  int32_t* plane = kReplay ? nullptr : p.quantized + c * p.pitch + row_index;
-  uint2* tokens = !kTokens ? nullptr
-                           : p.tokens + DcTokenOffset(blockIdx.x, blockIdx.y, p.width, p.height) +
-                               (static_cast<size_t>(DcChannelRank(c)) * gh + y) * gw;
-  uint32_t* ring = &r.samples[0][threadIdx.x];
-  // The row above at x-1, x, x+1 (zero errors above the group's first row),
-  // this row's last sample, and its sub-predictor errors at x-2. Past the
-  // row's ends the nearest sample stands in, as the reference reads it: the
-  // west side is set up one step before the row starts, and on the east side
-  // the lane above has stopped at its last sample.
-  DcSample above_w = {}, above = {}, above_e = {}, own = {};
-  uint32_t before_own[4] = {0, 0, 0, 0};
-  DcSample next = {};  // lane 0: the predecessor warp's sample of the next step
-  int wide = 0;
-  const int steps = kDcLead + gw + 2 * ((gh - 1) % kDcRows) + (warps - 1) * kDcWarpSkew +
-                    (blockIdx.z == 0 ? 0 : kDcSync);
-  for (int t = 0; t < steps; ++t) {
-    const int first = t - kDcLead - start;  // lane 0's position
-    if (first >= -kDcLead && first < gw + 2 * (kDcRows - 1)) {
-      const int x = first - 2 * lane;
-      // Samples arrive kDcLead steps ahead of their use.
-      if (y < gh && x >= -kDcLead && x + kDcLead < gw) {
-        const uint32_t slot = static_cast<uint32_t>(
-          __cvta_generic_to_shared(ring + ((x + kDcLead) & (kDcSampleSlots - 1)) * kDcThreads));
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(slot),
-                     "l"(source + x + kDcLead)
-                     : "memory");
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      above_w = above;
-      above = above_e;
-      above_e.q = __shfl_up_sync(0xffffffffu, own.q, 1);
-      above_e.e = __shfl_up_sync(0xffffffffu, own.e, 1);
-      above_e.n = __shfl_up_sync(0xffffffffu, own.n, 1);
+  uint32_t pending = y < gh ? source[row_index] : 0u;  // idle threads have y >= gh
+  // This row's previous quantized value and signed error (its west
+  // neighbour), kept in registers.
+  int32_t own_q = 0, own_e = 0;
+  const int waves = (gw - 1) + 2 * (gh - 1) + 2;
+  for (int t = 0; t < waves; ++t) {
+    const int x = t - lag - 2 * y;
+    const int wide = r.wide;
+    if (y < gh && x >= 0 && x < gw) {
+      const uint32_t sample = pending;
+      if (x + 1 < gw) pending = source[row_index + x + 1];
+      const int s = x & 7, sw = (x - 1) & 7, sne = (x + 1 < gw ? x + 1 : x) & 7;
+      const int snw = (x ? x - 1 : x) & 7;
+      const int up = y - 1, up2 = y - 2;
+      const int32_t w = x ? own_q : y ? Q[s][up] : 0;
+      const int32_t n = y ? Q[s][up] : w;
+      const int32_t nw = x && y ? Q[sw][up] : w;
+      const int32_t ne = y && x + 1 < gw ? Q[(x + 1) & 7][up] : n;
+      const int32_t nn = y > 1 ? Q[s][up2] : n;
+      const int32_t ew = x ? own_e : 0;
+      const int32_t en = y ? E[s][up] : 0;
+      const int32_t enw = y ? E[snw][up] : 0;
+      const int32_t ene = y ? E[sne][up] : 0;
+      // Sub-predictor error sums (prediction.h:73-90). The signed errors of
+      // row -1 read as zeros. The error sums of row 0 read the predictor's
+      // other rolling row, which by then holds only row 0's own "+="
+      // updates: its entry j carries the error of (j - 1, 0) once that
+      // sample is done, so north = err(x-1), northwest = err(x-2) and
+      // northeast (not yet written) = 0, or north at the right edge.
+      uint32_t errors[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         if (y) {
@@ -1399,17 +1507,6 @@ unsigned Blocks(size_t n, unsigned threads = kThreads) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-  __syncthreads();
-  // Warps past the group's rows, and X's unused half, have nothing to do.
-  const int warps = (gh + kDcRows - 1) / kDcRows;
-  const int half = static_cast<int>(threadIdx.x) / kDcGroup;
-  const int warp = static_cast<int>(threadIdx.x) % kDcGroup / kDcRows;
-  const int lane = static_cast<int>(threadIdx.x) % kDcRows;
-  if (warp >= warps || (blockIdx.z == 0 && half == 1)) return;
-  const int working = warps * kDcRows * (blockIdx.z == 0 ? 1 : 2);
-  const int c = blockIdx.z == 0 ? 0 : 1 + half;  // X; Y, B
-  const int y = warp * kDcRows + lane;
-  const int start = warp * kDcWarpSkew + (c == 2 ? kDcSync : 0);
 // Host launchers.
 
 void UploadDcTables() {
@@ -1466,7 +1563,8 @@ template <int W, int H>
 int LaunchForward(const float* opsin, size_t stride, size_t pitch, const int2* list,
                   const uint32_t* count, size_t max_count, float* coef, cudaStream_t stream) {
   constexpr int N = W * H, K = 1024 / N;
-  const size_t smem = static_cast<size_t>(PlaneBatch<W, H, 3 * K>::Elements) * 12;
+  constexpr size_t kBasisBytes = W == 32 || H == 32 ? 32 * 32 * sizeof(double) : 0;
+  const size_t smem = kBasisBytes + static_cast<size_t>(PlaneBatch<W, H, 3 * K>::Elements) * 12;
   int status = CheckCuda(cudaFuncSetAttribute(ForwardCoefficientsKernel<W, H>,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               static_cast<int>(smem)),
@@ -1536,6 +1634,32 @@ int AqQuantizer_(const float* field, size_t blocks, const AqPolicy* policy, AqQu
                  int32_t* raw, void* select_state, uint32_t* error, cudaStream_t stream) {
   SelectState* st = static_cast<SelectState*>(select_state);
   const int n = static_cast<int>(blocks);
+  if (blocks <= static_cast<size_t>(kSelectCluster) * kSelectShare) {
+    // The smallest power of two of CTAs with at most kSelectSmallShare values
+    // each, up to the largest cluster: fewer values per CTA gain less than
+    // the wider barrier costs.
+    int ctas = 1;
+    while (ctas < kSelectCluster && n > ctas * kSelectSmallShare) ctas *= 2;
+    const int share = (n + ctas - 1) / ctas;
+    const int status = CheckCuda(
+      cudaFuncSetAttribute(ClusterQuantizerKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           kSelectShare * static_cast<int>(sizeof(float))),
+      "aq quantizer attribute");
+    if (status != GJXL_B200_OK) return status;
+    cudaLaunchAttribute attribute;
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim = {static_cast<unsigned>(ctas), 1, 1};
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(ctas);
+    config.blockDim = dim3(kSelectThreads);
+    config.dynamicSmemBytes = share * sizeof(float);
+    config.stream = stream;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    return CheckCuda(cudaLaunchKernelEx(&config, ClusterQuantizerKernel, field, n, share, policy,
+                                        q, raw, error),
+                     "aq quantizer");
+  }
   const unsigned grid = static_cast<unsigned>(std::min<size_t>(Blocks(blocks), 4 * 148));
   SelectInitKernel<<<1, 1024, 0, stream>>>(st, n);
   for (int selection = 0; selection < 2; ++selection) {
