@@ -9,25 +9,28 @@
 // FindBestMultiplier (:98-151) with CflDerivatives (:22-79), whose four-lane
 // float sums keep the reference's element order, and QuantizeMultiplier.
 //
-// One CTA of four warps per tile; both maps of the tile stay in shared memory.
+// One CTA of seven warps per tile; both maps of the tile stay in shared memory.
 //
-// Phase 1 (all four warps): each warp transforms whole blocks, channel by
+// Phase 1 (all warps): each warp transforms whole blocks, channel by
 // channel. The block's pixels are staged in shared memory as doubles, lane l
 // owns row-pass and column-pass outputs (l >> 3, l & 7) and (l >> 3 + 4,
 // l & 7), and keeps its three rows of the DCT basis in registers. Each map's
 // (a, b) pairs go to shared memory grouped by the reference's lane
 // (element i at [i & 3][i >> 2]).
 //
-// Phase 2 (warps 0-2): the Newton iterations. The derivative sums are twelve
-// sequential float chains per map (3 sums x the reference's 4 lanes), so
-// their additions cannot be spread out; the per-element terms can. Warps 1
-// and 2 (one per map) evaluate the terms of 128-element chunks with all 32
-// lanes into a double buffer; warp 0 adds them, lanes 0-11 for y_to_x and
-// 16-27 for y_to_b, each lane one chain in element order, then takes the
-// Newton step. Named barriers pair the warps: FULL/EMPTY per buffer, and
-// XREADY when a new x is published. All three warps run the same loop
-// counts (the chunk count follows from the tile, the iteration count from
-// flags read after XREADY), so every barrier is met.
+// Phase 2: the Newton iterations. The derivative sums are twelve sequential
+// float chains per map (3 sums x the reference's 4 lanes), so their additions
+// cannot be spread out (1024 dependent adds an iteration: the bound); the
+// per-element terms can. Three producer warps per map take turns: each
+// evaluates the terms of every third 128-element chunk with all 32 lanes into
+// its own buffer of the ring. Warp 0 adds them, lanes 0-11 for y_to_x and
+// 16-27 for y_to_b, each lane one chain in element order, with the next
+// chunk's terms loaded during the adds; then it takes the Newton step. With
+// one producer warp per map the consumer waited for it: 143 us at 256x256,
+// 395 us at 2048x1536. Named barriers pair the warps: FULL/EMPTY per buffer,
+// and XREADY when a new x is published. All warps run the same loop counts
+// (the chunk count follows from the tile, the iteration count from flags read
+// after XREADY), so every barrier is met.
 
 #include <cmath>
 #include <cstring>
@@ -40,21 +43,24 @@ namespace gjxl_b200 {
 namespace {
 
 constexpr int kTileValues = 64 * 64;  // up to 64 blocks of 64 coefficients
-constexpr int kCflThreads = 128;
+constexpr int kSets = 3;                    // producer sets and term buffers
+constexpr int kCflWarps = 1 + 2 * kSets;
+constexpr int kCflThreads = 32 * kCflWarps;
 constexpr int kChunk = 32;           // elements per lane chain in one chunk
 constexpr int kTermStride = kChunk + 4;  // floats per term row (bank spread)
 constexpr int kTermRows = 24;        // 2 maps x 3 sums x 4 lanes
 constexpr size_t kPairBytes = 2 * kTileValues * sizeof(float2);
-constexpr size_t kTermBytes = 2 * kTermRows * kTermStride * sizeof(float);
-constexpr size_t kPhase1Bytes = 4 * (64 * sizeof(double) * 2 + 64 * sizeof(float));
+constexpr size_t kTermBytes = kSets * kTermRows * kTermStride * sizeof(float);
+constexpr size_t kPhase1Bytes = kCflWarps * (64 * sizeof(double) * 2 + 64 * sizeof(float));
 constexpr size_t kScratchBytes = kTermBytes > kPhase1Bytes ? kTermBytes : kPhase1Bytes;
-constexpr size_t kCflSmem = kPairBytes + kScratchBytes + 16;
+constexpr size_t kCflSmem = kPairBytes + kScratchBytes + 32;
 
-// Named barrier ids (0 is __syncthreads) and the phase-2 participants.
-constexpr int kBarFull = 1;    // + buffer
-constexpr int kBarEmpty = 3;   // + buffer
-constexpr int kBarXReady = 5;
-constexpr int kPhase2Threads = 96;
+// Named barrier ids (0 is __syncthreads). FULL and EMPTY pair the consumer
+// with one set's two producers; XREADY has every warp.
+constexpr int kBarFull = 1;                // + buffer
+constexpr int kBarEmpty = kBarFull + kSets;  // + buffer
+constexpr int kBarXReady = kBarEmpty + kSets;
+constexpr int kPairThreads = 96;
 
 struct CflParams {
   const float* opsin;  // Gaborish-inverted padded XYB
@@ -68,25 +74,16 @@ struct CflParams {
   int8_t* y_to_b;
 };
 
-// Barrier ids are immediates, so that the kernel reserves only the six it
-// uses; `id` is warp-uniform.
-__device__ __forceinline__ void BarSync(int id) {
-  switch (id) {
-    case kBarFull: asm volatile("bar.sync 1, %0;" :: "n"(kPhase2Threads) : "memory"); break;
-    case kBarFull + 1: asm volatile("bar.sync 2, %0;" :: "n"(kPhase2Threads) : "memory"); break;
-    case kBarEmpty: asm volatile("bar.sync 3, %0;" :: "n"(kPhase2Threads) : "memory"); break;
-    case kBarEmpty + 1: asm volatile("bar.sync 4, %0;" :: "n"(kPhase2Threads) : "memory"); break;
-    default: asm volatile("bar.sync 5, %0;" :: "n"(kPhase2Threads) : "memory"); break;
-  }
+// Barrier ids and counts are immediates (a round trip between two warps takes
+// 75 cycles so, 118 from registers), and no branch picks them: the buffer is a
+// compile-time constant at every use.
+template <int kId, int kThreads>
+__device__ __forceinline__ void BarSync() {
+  asm volatile("bar.sync %0, %1;" ::"n"(kId), "n"(kThreads) : "memory");
 }
-__device__ __forceinline__ void BarArrive(int id) {
-  switch (id) {
-    case kBarFull: asm volatile("bar.arrive 1, %0;" :: "n"(kPhase2Threads) : "memory"); break;
-    case kBarFull + 1: asm volatile("bar.arrive 2, %0;" :: "n"(kPhase2Threads) : "memory"); break;
-    case kBarEmpty: asm volatile("bar.arrive 3, %0;" :: "n"(kPhase2Threads) : "memory"); break;
-    case kBarEmpty + 1: asm volatile("bar.arrive 4, %0;" :: "n"(kPhase2Threads) : "memory"); break;
-    default: asm volatile("bar.arrive 5, %0;" :: "n"(kPhase2Threads) : "memory"); break;
-  }
+template <int kId, int kThreads>
+__device__ __forceinline__ void BarArrive() {
+  asm volatile("bar.arrive %0, %1;" ::"n"(kId), "n"(kThreads) : "memory");
 }
 
 // QuantizeMultiplier (chroma_from_luma.cpp:81-96).
@@ -101,6 +98,8 @@ __device__ __forceinline__ int8_t QuantizeMultiplier(float x) {
   }
   return static_cast<int8_t>(fminf(fmaxf(roundf(x), -128.0f), 127.0f));
 }
+
+constexpr float kEpsilon = 100.0f;  // step of the finite differences
 
 // The derivative terms of one element for the three sums (center, +eps,
 // -eps) at the current x: d = (2/3 a) (|r| + 1) signed like r, r = a x_k + b,
@@ -121,12 +120,93 @@ __device__ __forceinline__ void Terms(float2 v, float x, float xp, float xm, flo
   t2 = rm < 0.0f ? -dm : dm;
 }
 
+// One chunk per chain out of buffer kBuffer into registers, which frees the
+// buffer; and its terms added in order.
+template <int kBuffer>
+__device__ __forceinline__ void TakeChunk(const float* chain_terms, float4 (&t)[kChunk / 4]) {
+  BarSync<kBarFull + kBuffer, kPairThreads>();
+  const float4* src =
+    reinterpret_cast<const float4*>(chain_terms + kBuffer * kTermRows * kTermStride);
+#pragma unroll
+  for (int q = 0; q < kChunk / 4; ++q) t[q] = src[q];
+  BarArrive<kBarEmpty + kBuffer, kPairThreads>();
+}
+
+__device__ __forceinline__ float AddChunk(const float4 (&t)[kChunk / 4], float sum) {
+#pragma unroll
+  for (int q = 0; q < kChunk / 4; ++q) {
+    sum += t[q].x;
+    sum += t[q].y;
+    sum += t[q].z;
+    sum += t[q].w;
+  }
+  return sum;
+}
+
+// Chunk c (of `chunks`, c % 6 == kStep), already in `now`: its adds, with the
+// next chunk's loads before them. Returns false after the last chunk.
+template <int kStep>
+__device__ __forceinline__ bool AddAndTake(const float* chain_terms, int c, int chunks,
+                                           float4 (&now)[kChunk / 4], float4 (&next)[kChunk / 4],
+                                           float& sum) {
+  const bool more = c + 1 < chunks;
+  if (more) TakeChunk<(kStep + 1) % kSets>(chain_terms, next);
+  sum = AddChunk(now, sum);
+  return more;
+}
+
+// A producer warp of set kSet (chunks kSet, kSet + 3, ... of every iteration)
+// for one map. Lane (slot s, quad q) evaluates elements j = chunk * 32 + 4q ..
+// 4q + 3 of reference lane s; past the end of a ragged tile's last chunk the
+// terms are zeros, which leave the sums as they are. The x of an iteration
+// sits in the half of `xs` that the next one does not write: a set without a
+// chunk in a short tile may still read it while the consumer publishes the
+// next.
+template <int kSet>
+__device__ __forceinline__ void ProduceTerms(const float2* map_pairs, float* terms,
+                                             const float* xs, const int* dones, int map, int lane,
+                                             int js, int chunks, int iterations) {
+  const int s = lane >> 3, q = lane & 7;
+  float* const row = terms + (kSet * kTermRows + map * 12 + s) * kTermStride + 4 * q;
+  bool produced = false;
+  for (int iteration = 0; iteration < iterations; ++iteration) {
+    BarSync<kBarXReady, kCflThreads>();
+    const float* const x_now = xs + (iteration & 1) * 2;
+    const int* const done_now = dones + (iteration & 1) * 2;
+    const float x = x_now[map];
+    const bool skip = done_now[map] != 0;
+    if (done_now[0] != 0 && done_now[1] != 0) break;
+    const float xp = x + kEpsilon, xm = x - kEpsilon;
+    for (int c = kSet; c < chunks; c += kSets) {
+      const int j = c * kChunk + 4 * q;
+      float4 o0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), o1 = o0, o2 = o0;
+      if (!skip && j < js) {
+        const float4* src = reinterpret_cast<const float4*>(map_pairs + s * js + j);
+        const float4 ab01 = src[0], ab23 = src[1];
+        Terms(make_float2(ab01.x, ab01.y), x, xp, xm, o0.x, o1.x, o2.x);
+        Terms(make_float2(ab01.z, ab01.w), x, xp, xm, o0.y, o1.y, o2.y);
+        Terms(make_float2(ab23.x, ab23.y), x, xp, xm, o0.z, o1.z, o2.z);
+        Terms(make_float2(ab23.z, ab23.w), x, xp, xm, o0.w, o1.w, o2.w);
+      }
+      if (produced) BarSync<kBarEmpty + kSet, kPairThreads>();
+      produced = true;
+      *reinterpret_cast<float4*>(row) = o0;
+      *reinterpret_cast<float4*>(row + 4 * kTermStride) = o1;
+      *reinterpret_cast<float4*>(row + 8 * kTermStride) = o2;
+      __syncwarp();
+      BarArrive<kBarFull + kSet, kPairThreads>();
+    }
+  }
+  // Meet the consumer's last EMPTY arrival.
+  if (produced) BarSync<kBarEmpty + kSet, kPairThreads>();
+}
+
 __global__ void __launch_bounds__(kCflThreads, 3) CflTileKernel(const __grid_constant__ CflParams p) {
   extern __shared__ __align__(16) unsigned char cfl_smem[];
   float2* pairs = reinterpret_cast<float2*>(cfl_smem);  // [map][4][js]
   unsigned char* scratch = cfl_smem + kPairBytes;
   float* xs = reinterpret_cast<float*>(cfl_smem + kPairBytes + kScratchBytes);
-  int* dones = reinterpret_cast<int*>(xs + 2);
+  int* dones = reinterpret_cast<int*>(xs + 4);  // both [iteration & 1][map]
 
   const int tile = blockIdx.x;
   const int tx = tile % p.tiles_x, ty = tile / p.tiles_x;
@@ -141,7 +221,7 @@ __global__ void __launch_bounds__(kCflThreads, 3) CflTileKernel(const __grid_con
   {
     double* px = reinterpret_cast<double*>(scratch) + warp * 128;  // 64 pixels
     double* tm = px + 64;                                          // row-pass output
-    float* ycoef = reinterpret_cast<float*>(reinterpret_cast<double*>(scratch) + 4 * 128) +
+    float* ycoef = reinterpret_cast<float*>(reinterpret_cast<double*>(scratch) + kCflWarps * 128) +
                    warp * 64;
     const int y0 = lane >> 3, u = lane & 7;
     double basis_u[8], basis_v0[8], basis_v1[8];
@@ -169,8 +249,8 @@ __global__ void __launch_bounds__(kCflThreads, 3) CflTileKernel(const __grid_con
     };
     float2 current[3], next[3];
     load_block(warp, current);
-    for (int b = warp; b < blocks; b += 4) {
-      load_block(b + 4, next);
+    for (int b = warp; b < blocks; b += kCflWarps) {
+      load_block(b + kCflWarps, next);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const int ch = c == 0 ? 1 : c == 1 ? 0 : 2;  // Y first, then X and B
@@ -228,11 +308,9 @@ __global__ void __launch_bounds__(kCflThreads, 3) CflTileKernel(const __grid_con
     }
   }
   __syncthreads();
-  if (warp == 3) return;
 
   // ---- Phase 2: Newton iterations.
   const float kDistanceMultiplierAc = 1.0e-9f;
-  const float kEpsilon = 100.0f;
   float* terms = reinterpret_cast<float*>(scratch);  // [buffer][row][kTermStride]
   const int chunks = (js + kChunk - 1) / kChunk;
   if (warp == 0) {
@@ -242,48 +320,24 @@ __global__ void __launch_bounds__(kCflThreads, 3) CflTileKernel(const __grid_con
     const int row = map * 12 + (chain ? row_in_map : 0);
     float x = 0.0f;
     bool done = false, all_done = false;
-    int g = 0;
+    const float* const chain_terms = terms + row * kTermStride;
     for (int iteration = 0; iteration < p.iterations; ++iteration) {
       if ((lane & 15) == 0) {
-        xs[map] = x;
-        dones[map] = done ? 1 : 0;
+        xs[(iteration & 1) * 2 + map] = x;
+        dones[(iteration & 1) * 2 + map] = done ? 1 : 0;
       }
-      BarArrive(kBarXReady);
+      BarArrive<kBarXReady, kCflThreads>();
       if (all_done) break;
       float lane_sum = 0.0f;
-      for (int c = 0; c < chunks; ++c, ++g) {
-        const int buffer = g & 1;
-        BarSync(kBarFull + buffer);
-        const float4* src = reinterpret_cast<const float4*>(
-          terms + (buffer * kTermRows + row) * kTermStride);
-        // All of the chunk's terms into registers first (the loads overlap),
-        // which also frees the buffer for the producers before the adds.
-        // A chunk holds 32 terms per chain, or 16 in a ragged tile's last.
-        float4 t[kChunk / 4];
-        const bool half = js - c * kChunk < kChunk;
-#pragma unroll
-        for (int q = 0; q < kChunk / 8; ++q) t[q] = src[q];
-        if (!half) {
-#pragma unroll
-          for (int q = kChunk / 8; q < kChunk / 4; ++q) t[q] = src[q];
-        }
-        BarArrive(kBarEmpty + buffer);
-#pragma unroll
-        for (int q = 0; q < kChunk / 8; ++q) {
-          lane_sum += t[q].x;
-          lane_sum += t[q].y;
-          lane_sum += t[q].z;
-          lane_sum += t[q].w;
-        }
-        if (!half) {
-#pragma unroll
-          for (int q = kChunk / 8; q < kChunk / 4; ++q) {
-            lane_sum += t[q].x;
-            lane_sum += t[q].y;
-            lane_sum += t[q].z;
-            lane_sum += t[q].w;
-          }
-        }
+      float4 even[kChunk / 4], odd[kChunk / 4];
+      TakeChunk<0>(chain_terms, even);
+      for (int c = 0;; c += 6) {
+        if (!AddAndTake<0>(chain_terms, c, chunks, even, odd, lane_sum)) break;
+        if (!AddAndTake<1>(chain_terms, c + 1, chunks, odd, even, lane_sum)) break;
+        if (!AddAndTake<2>(chain_terms, c + 2, chunks, even, odd, lane_sum)) break;
+        if (!AddAndTake<3>(chain_terms, c + 3, chunks, odd, even, lane_sum)) break;
+        if (!AddAndTake<4>(chain_terms, c + 4, chunks, even, odd, lane_sum)) break;
+        if (!AddAndTake<5>(chain_terms, c + 5, chunks, odd, even, lane_sum)) break;
       }
       // Horizontal sums (l0 + l1) + (l2 + l3) for each kind, per map.
       float sums[3];
@@ -313,41 +367,16 @@ __global__ void __launch_bounds__(kCflThreads, 3) CflTileKernel(const __grid_con
     if (lane == 16) p.y_to_b[tile] = QuantizeMultiplier(x);
     return;
   }
-  // Producers: warp 1 for y_to_x, warp 2 for y_to_b. Lane (slot s, quad q)
-  // evaluates elements j = chunk * 32 + 4q .. 4q + 3 of reference lane s.
-  const int map = warp - 1;
+  // Producers: warps 1 + 2 * set + map.
+  const int map = (warp - 1) & 1, set = (warp - 1) >> 1;
   const float2* map_pairs = pairs + map * kTileValues;
-  const int s = lane >> 3, q = lane & 7;
-  int g = 0;
-  for (int iteration = 0; iteration < p.iterations; ++iteration) {
-    BarSync(kBarXReady);
-    const float x = xs[map];
-    const bool skip = dones[map] != 0;
-    if (dones[0] != 0 && dones[1] != 0) break;
-    const float xp = x + kEpsilon, xm = x - kEpsilon;
-    for (int c = 0; c < chunks; ++c, ++g) {
-      const int buffer = g & 1;
-      if (g >= 2) BarSync(kBarEmpty + buffer);
-      const int j = c * kChunk + 4 * q;
-      if (!skip && j < js) {
-        const float4* src = reinterpret_cast<const float4*>(map_pairs + s * js + j);
-        const float4 ab01 = src[0], ab23 = src[1];
-        float4 o0, o1, o2;
-        Terms(make_float2(ab01.x, ab01.y), x, xp, xm, o0.x, o1.x, o2.x);
-        Terms(make_float2(ab01.z, ab01.w), x, xp, xm, o0.y, o1.y, o2.y);
-        Terms(make_float2(ab23.x, ab23.y), x, xp, xm, o0.z, o1.z, o2.z);
-        Terms(make_float2(ab23.z, ab23.w), x, xp, xm, o0.w, o1.w, o2.w);
-        float* dst = terms + (buffer * kTermRows + map * 12 + s) * kTermStride + 4 * q;
-        *reinterpret_cast<float4*>(dst) = o0;
-        *reinterpret_cast<float4*>(dst + 4 * kTermStride) = o1;
-        *reinterpret_cast<float4*>(dst + 8 * kTermStride) = o2;
-      }
-      __syncwarp();
-      BarArrive(kBarFull + buffer);
-    }
+  if (set == 0) {
+    ProduceTerms<0>(map_pairs, terms, xs, dones, map, lane, js, chunks, p.iterations);
+  } else if (set == 1) {
+    ProduceTerms<1>(map_pairs, terms, xs, dones, map, lane, js, chunks, p.iterations);
+  } else {
+    ProduceTerms<2>(map_pairs, terms, xs, dones, map, lane, js, chunks, p.iterations);
   }
-  // Meet the consumer's last two EMPTY arrivals.
-  for (int last = max(0, g - 2); last < g; ++last) BarSync(kBarEmpty + (last & 1));
 }
 
 }  // namespace

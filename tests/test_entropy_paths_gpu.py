@@ -1,0 +1,152 @@
+"""Section writers against a Python restatement of the streams, at the sizes
+where their paths change: ANS batches of 128 tokens, reverse maps in shared
+memory or in the code's own memory, maps that are no ANS code;
+prefix chunks of 2048 tokens and codes too large for shared memory."""
+
+import numpy as np
+import pytest
+import torch
+
+from gjxl_b200.entropy import ANS, PREFIX, EntropyCode, write_sections
+from tests.gpu_util import host
+
+pytestmark = pytest.mark.gpu
+
+
+def hybrid(v: int) -> tuple[int, int, int]:
+    """(symbol, extra bits, count) under {4, 2, 0}."""
+    if v < 16:
+        return v, 0, 0
+    n = v.bit_length() - 1
+    return 16 + ((n - 4) << 2) + ((v - (1 << n)) >> (n - 2)), v & ((1 << (n - 2)) - 1), n - 2
+
+
+def make_tokens(seed: int, n: int, contexts: int):
+    rng = np.random.default_rng(seed)
+    ctx = rng.integers(0, contexts, n).astype(np.uint16)
+    values = (rng.geometric(0.2 + 0.7 * (ctx % 7) / 7.0) - 1).astype(np.uint32)
+    large = rng.random(n) < 0.01
+    values[large] = rng.integers(0, 1 << 20, int(large.sum()))
+    return values, ctx
+
+
+def make_tables(mode: int, seed: int, contexts: int, clusters: int) -> dict:
+    rng = np.random.default_rng(seed)
+    t = {"mode": mode, "context_count": contexts, "cluster_count": clusters,
+         "context_map": (np.arange(contexts) % clusters).astype(np.uint8),
+         "configs": np.tile(np.array([[4, 2, 0]], np.uint8), (clusters, 1))}
+    if mode == ANS:
+        freq = np.ones((clusters, 128), np.int64)
+        for c in range(clusters):  # every frequency from 1 up to most of the table
+            room = 4096 - 128
+            for s in rng.permutation(16):
+                f = int(rng.integers(0, room + 1)) if s else 0
+                freq[c, s] += f
+                room -= f
+            freq[c, 0] += room
+        padded = np.zeros((clusters, 256), np.int64)
+        padded[:, :128] = freq
+        starts = np.cumsum(padded, 1) - padded
+        return t | {"frequencies": padded.astype(np.uint16),
+                    "reverse_offsets": starts.astype(np.uint16),
+                    "reverse_map": np.stack([rng.permutation(4096) for _ in range(clusters)])
+                    .astype(np.uint16)}
+    depths = rng.integers(1, 16, (clusters, 128)).astype(np.uint8)
+    bits = (rng.integers(0, 1 << 15, (clusters, 128)) & ((1 << depths.astype(int)) - 1))
+    degenerate = np.full(clusters, 128, np.uint16)
+    return t | {"depths": depths, "bits": bits.astype(np.uint16), "degenerate": degenerate}
+
+
+def ans_stream(t: dict, values, ctx) -> tuple[int, int]:
+    """(bits, count): the final state, then the chunks in reverse push order."""
+    state, stream, count = 0x130000, 0, 0
+    for v, c in zip(values[::-1].tolist(), ctx[::-1].tolist()):
+        cluster = t["context_map"][c]
+        symbol, extra, n = hybrid(v)
+        f = int(t["frequencies"][cluster, symbol])
+        stream, count = (stream << n) | extra, count + n
+        if (state >> 20) >= f:
+            stream, count, state = (stream << 16) | (state & 0xFFFF), count + 16, state >> 16
+        slot = t["reverse_map"][cluster, int(t["reverse_offsets"][cluster, symbol]) + state % f]
+        state = (state // f << 12) + int(slot)
+    return (stream << 32) | state, count + 32
+
+
+def prefix_stream(t: dict, values, ctx) -> tuple[int, int]:
+    parts, count = [], 0
+    for v, c in zip(values.tolist(), ctx.tolist()):
+        cluster = t["context_map"][c]
+        symbol, extra, n = hybrid(v)
+        d = int(t["depths"][cluster, symbol])
+        parts.append(format((extra << d) | int(t["bits"][cluster, symbol]), f"0{d + n}b"))
+        count += d + n
+    return (int("".join(parts[::-1]), 2) if parts else 0), count
+
+
+def check(t: dict, values, ctx, offsets):
+    code = EntropyCode(t)
+    got = write_sections(code, torch.from_numpy(offsets.astype(np.int32)).cuda(),
+                         values=torch.from_numpy(values.view(np.int32)).cuda(),
+                         contexts=torch.from_numpy(ctx.view(np.int16)).cuda())
+    assert int(host(got["error"])[0]) == 0
+    bits, packed = host(got["bit_counts"]), host(got["packed"]).tobytes()
+    at = 0
+    for s in range(offsets.size - 1):
+        lo, hi = int(offsets[s]), int(offsets[s + 1])
+        stream, count = (ans_stream if t["mode"] == ANS else prefix_stream)(
+            t, values[lo:hi], ctx[lo:hi])
+        assert int(bits[s]) == count, f"section {s}: bit count"
+        size = (count + 7) // 8
+        assert packed[at:at + size] == stream.to_bytes(size, "little"), f"section {s}"
+        at += size
+    assert host(got["byte_offsets"])[-1] == at
+
+
+SIZES = [0, 1, 2, 127, 128, 129, 255, 257, 1000, 3]
+
+
+# 1 and 3 clusters: all maps staged; 30 and 90: some in the code only.
+@pytest.mark.parametrize("clusters", [1, 3, 30, 90])
+def test_ans_sections(cuda, clusters):
+    offsets = np.concatenate([[0], np.cumsum(SIZES + [700] * 3)])
+    values, ctx = make_tokens(clusters, int(offsets[-1]), 200)
+    check(make_tables(ANS, 5 + clusters, 200, clusters), values, ctx, offsets)
+
+
+def test_ans_context_map_beyond_shared_memory(cuda):
+    offsets = np.array([0, 400, 1000])
+    values, ctx = make_tokens(3, 1000, 6000)
+    check(make_tables(ANS, 9, 6000, 20), values, ctx, offsets)
+
+
+def test_ans_map_entry_outside_table_is_reported(cuda):
+    """A used reverse-map entry past the 4096-entry table: error bit 2; an
+    unused one changes nothing."""
+    values, ctx = make_tokens(4, 500, 4)
+    t = make_tables(ANS, 11, 4, 4)
+    used = set()
+    state = 0x130000
+    for v, c in zip(values[::-1].tolist(), ctx[::-1].tolist()):
+        cluster = int(t["context_map"][c])
+        f = int(t["frequencies"][cluster, hybrid(v)[0]])
+        if (state >> 20) >= f:
+            state >>= 16
+        at = int(t["reverse_offsets"][cluster, hybrid(v)[0]]) + state % f
+        used.add((cluster, at))
+        state = (state // f << 12) + int(t["reverse_map"][cluster, at])
+    spare = next((0, i) for i in range(4096) if (0, i) not in used)
+    t["reverse_map"][spare] = 5000
+    check(t, values, ctx, np.array([0, 500]))
+    t["reverse_map"][next(iter(used))] = 5000
+    got = write_sections(EntropyCode(t), torch.tensor([0, 500], dtype=torch.int32).cuda(),
+                         values=torch.from_numpy(values.view(np.int32)).cuda(),
+                         contexts=torch.from_numpy(ctx.view(np.int16)).cuda())
+    assert int(host(got["error"])[0]) & 4
+
+
+# 250 clusters of 129 words exceed the staged size.
+@pytest.mark.parametrize("clusters", [1, 40, 250])
+def test_prefix_sections(cuda, clusters):
+    offsets = np.concatenate([[0], np.cumsum([0, 1, 2047, 2048, 2049, 4100, 7])])
+    values, ctx = make_tokens(50 + clusters, int(offsets[-1]), 300)
+    check(make_tables(PREFIX, 60 + clusters, 300, clusters), values, ctx, offsets)
