@@ -1160,20 +1160,26 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
 //
 // The reference walks each 256x256-block DC group in raster order, channel
 // by channel (Y, X, B), resetting the predictor per channel. A sample at
-// (x, y) depends on row y at x-1 and on row y-1 at x-1..x+1 and row y-2 at x,
-// through the quantized values and the predictor's error state. So all
-// samples on a line x + 2y = t are independent, and the kernel sweeps those
-// lines (waves). Rows y-1 and y-2 are then 2 and 4 samples ahead of row y, so
-// every value a sample reads was written within the last 4 waves. Each row
-// keeps its quantized values, signed errors and the four sub-predictor error
-// sums in an 8-slot ring (slot x & 7) in shared memory; nothing goes to
-// global memory but the quantized output.
+// (x, y) depends on row y at x-1 and x-2 and on row y-1 at x-1..x+1 (and row
+// y-2 at x), through the quantized values and the predictor's error state. So
+// all samples on a line x + 2y = t are independent, and the kernel sweeps
+// those lines: a group takes about W + 2H dependent steps, and the latency of
+// one step is the kernel's bound (8 SMs of the chip hold work at 12 MP).
 //
-// Two CTAs per DC group, one thread per (channel, row): one CTA runs X, the
-// other Y (threads 0-255) and B (256-511). X and Y are independent. B's
-// residual subtracts Y's quantized value at the same position, so B runs one
-// wave behind Y and reads it from Y's ring. Slot x & 7 of a row is rewritten 8 waves later, and
-// a reader needs it at most 4 waves (B: 1 wave) after it was written.
+// A warp owns 32 rows of one channel, a lane one row, two samples behind the
+// lane above it. The sample that a step needs of the row above is the one
+// that the lane above computed in the step before, so it comes by shuffle;
+// a lane keeps the two samples before it, and its own row's last two error
+// vectors, in registers. A warp's last row goes through a small ring in
+// shared memory to the next warp, which runs kDcWarpSkew steps later, so that
+// one barrier every kDcSync steps is enough; B follows Y by kDcSync steps for
+// the same reason. With every row's state in shared memory and a barrier per
+// step, a step took about 700 ns (526 us per pass at 2048x1536, 74 us at
+// 256x256): some 400 instructions of one warp, a quarter of them shared
+// accesses and a third selects at the rows' ends.
+//
+// Two CTAs per DC group on different SMs: X alone, and Y with B, whose
+// residual subtracts Y's quantized value at the same position.
 
 struct DcQuantParams {
   const float* dc;  // 3 planes of blocks
@@ -1193,19 +1199,32 @@ struct DcQuantParams {
 };
 
 constexpr int kDcGroup = 256;
-constexpr int kDcRing = 8;
-// Two CTAs per DC group on different SMs: blockIdx.z == 0 runs X (threads
-// 0-255; 256-511 idle), blockIdx.z == 1 runs Y (0-255) and B (256-511), which
-// reads Y's ring.
+constexpr int kDcRows = 32;                     // rows per warp
+constexpr int kDcWarps = kDcGroup / kDcRows;    // warps per channel
+constexpr int kDcSync = 8;                      // steps between barriers
+// A warp's first lane reads its predecessor's last row two samples ahead
+// (62 steps behind the predecessor's first lane), at least kDcSync steps
+// after they were written.
+constexpr int kDcWarpSkew = 2 * kDcRows + kDcSync;
+// Ring slots: a slot is rewritten kDcSlots steps after it was written, read
+// kDcSync steps after, and warps are less than kDcSync steps apart.
+constexpr int kDcSlots = 32;
+static_assert(kDcSlots >= 2 * kDcSync + 2, "ring slots outlive their readers");
 constexpr int kDcThreads = 2 * kDcGroup;
+// A row's samples are loaded kDcSync at a time, up to two loads ahead.
+constexpr int kDcSampleSlots = 2 * kDcSync;
 
-struct DcRings {
-  int32_t q[3][kDcRing][kDcGroup];        // quantized values
-  int32_t e[3][kDcRing][kDcGroup];        // signed prediction errors (error_)
-  uint32_t pe[3][4][kDcRing][kDcGroup];   // sub-predictor errors (prediction_errors_)
-  uint32_t row0[3][4][kDcRing];           // row 0's own errors, before row 1 adds
-  uint32_t reciprocal[64];                // (1 << 24) / (i + 1)
-  uint8_t contexts[1024];                 // DC tree leaf of 512 + property
+struct DcShared {
+  // Of the row above each warp's first one (entry 0: zeros; entry k: the last
+  // row of warp k - 1): quantized value, signed error (error_) and the value
+  // above it, and its sub-predictor errors (prediction_errors_) before the row
+  // below adds its own.
+  int4 last_values[3][kDcWarps + 1][kDcSlots];
+  uint4 last_errors[3][kDcWarps + 1][kDcSlots];
+  int32_t luma[kDcSlots][kDcGroup];           // Y's quantized values, for B
+  uint32_t samples[kDcSampleSlots][kDcThreads];  // per row, by x
+  uint32_t reciprocal[64];                    // (1 << 24) / (i + 1)
+  uint8_t contexts[1024];                     // DC tree leaf of 512 + property
   int wide;  // set once a stored value leaves the 32-bit bounds below
 };
 
@@ -1223,219 +1242,351 @@ constexpr int32_t kDcNarrowQuantized = 1 << 21;
 constexpr int32_t kDcNarrowError = 1 << 23;
 constexpr float kDcNarrowScaled = 2097152.0f;  // 2^21
 
-// One step of the weighted predictor (prediction.h:73-141) and the residual
-// quantization (dc_quantization.cpp:178-199) in integer type Int: the
-// neighbours' quantized values and signed errors, the four sub-predictor
-// error sums and value * inverse step in; the quantized value, its signed
-// error and the four sub-predictor errors out.
-// In replay form (kReplay) the sample's quantized value comes in through
-// *quantized_out and only the prediction and the update run.
-template <typename Int, bool kWide, bool kReplay = false>
-__device__ __forceinline__ void WeightedPredictorStep(Int w, Int n, Int nw, Int ne, Int nn, Int ew,
-                                                      Int en, Int enw, Int ene,
-                                                      const uint32_t (&errors)[4],
-                                                      const uint32_t* reciprocal,
-                                                      float scaled_value, int32_t* quantized_out,
-                                                      int32_t* error_out,
-                                                      uint32_t (&sub_errors)[4],
-                                                      int64_t* predicted_out) {
-  // WeightedPredictorParameters defaults (prediction.h:36-40).
+// What one predictor step reads: the neighbours' quantized values, their
+// signed errors, the four sub-predictor error sums, and value * inverse step.
+// In replay form the sample's quantized value stands in for the last.
+struct DcStepInput {
+  int32_t w, n, nw, ne, nn, ew, en, enw, ene;
+  uint32_t errors[4];
+  float scaled_value;
+  int32_t replayed;
+};
+struct DcStepOutput {
+  int32_t quantized, error;  // quantized value and its signed error
+  uint32_t sub[4];           // sub-predictor errors
+  int64_t predicted;
+};
+
+// The residual quantization (dc_quantization.cpp:178-199): value * inverse
+// step against the prediction.
+__device__ __forceinline__ float DcResidualSteps(float scaled_value, float predicted) {
+  float residual = scaled_value - predicted;
+  if (residual > -0.62f && residual < 0.62f) residual = 0.0f;
+  const float rounded = roundf(residual);
+  const float coarse = roundf(residual * 0.5f) * 2.0f;
+  return fabsf(rounded) > 2.0f ? coarse : rounded;
+}
+
+// One step of the weighted predictor (prediction.h:73-141, with the default
+// parameters of prediction.h:36-40) in 64-bit integers.
+template <bool kReplay>
+__device__ __noinline__ DcStepOutput WideDcStep(const DcStepInput& in,
+                                                const uint32_t* reciprocal) {
   constexpr int kP0 = 16, kP1 = 10, kP2 = 7, kP3 = 7, kP4 = 7, kP5 = 0, kP6 = 0;
   const uint32_t max_weights[4] = {13, 12, 12, 12};
   uint32_t weights[4];
   uint32_t weight_sum = 0;
-#pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int bits = kWide ? BitWidth64(static_cast<uint64_t>(errors[i]) + 1)
-                           : BitWidth32(errors[i] + 1u);
-    const int shift = max(0, bits - 6);
-    weights[i] = 4 + ((max_weights[i] * reciprocal[errors[i] >> shift]) >> shift);
+    const int shift = max(0, BitWidth64(static_cast<uint64_t>(in.errors[i]) + 1) - 6);
+    weights[i] = 4 + ((max_weights[i] * reciprocal[in.errors[i] >> shift]) >> shift);
     weight_sum += weights[i];
   }
   const int log_weight = BitWidth32(weight_sum) - 1;
   weight_sum = 0;
-#pragma unroll
   for (int i = 0; i < 4; ++i) {
     weights[i] >>= log_weight - 4;
     weight_sum += weights[i];
   }
-  const Int n8 = n * 8, w8 = w * 8, ne8 = ne * 8, nw8 = nw * 8, nn8 = nn * 8;
-  Int predictions[4];
+  const int64_t en = in.en, ew = in.ew, enw = in.enw, ene = in.ene;
+  const int64_t n8 = in.n * int64_t(8), w8 = in.w * int64_t(8), ne8 = in.ne * int64_t(8),
+                nw8 = in.nw * int64_t(8), nn8 = in.nn * int64_t(8);
+  int64_t predictions[4];
   predictions[0] = w8 + ne8 - n8;
-  predictions[1] = n8 - (((en + ew + ene) * Int(kP0)) >> 5);
-  predictions[2] = w8 - (((en + ew + enw) * Int(kP1)) >> 5);
-  predictions[3] = n8 - ((enw * Int(kP2) + en * Int(kP3) + ene * Int(kP4) + (nn8 - n8) * Int(kP5) +
-                          (nw8 - w8) * Int(kP6)) >> 5);
-  Int sum = static_cast<Int>(weight_sum >> 1) - 1;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) sum += predictions[i] * static_cast<Int>(weights[i]);
-  Int prediction = static_cast<Int>(
-    (static_cast<int64_t>(sum) * static_cast<int64_t>(reciprocal[weight_sum - 1])) >> 24);
+  predictions[1] = n8 - (((en + ew + ene) * kP0) >> 5);
+  predictions[2] = w8 - (((en + ew + enw) * kP1) >> 5);
+  predictions[3] = n8 - ((enw * kP2 + en * kP3 + ene * kP4 + (nn8 - n8) * kP5 +
+                          (nw8 - w8) * kP6) >> 5);
+  int64_t sum = static_cast<int64_t>(weight_sum >> 1) - 1;
+  for (int i = 0; i < 4; ++i) sum += predictions[i] * static_cast<int64_t>(weights[i]);
+  int64_t prediction = (sum * static_cast<int64_t>(reciprocal[weight_sum - 1])) >> 24;
   if (((en ^ ew) | (en ^ enw)) <= 0) {
-    const Int lo = min(w8, min(ne8, n8)), hi = max(w8, max(ne8, n8));
+    const int64_t lo = min(w8, min(ne8, n8)), hi = max(w8, max(ne8, n8));
     prediction = min(max(prediction, lo), hi);
   }
-  const Int predicted = (prediction + 3) >> 3;
-  *predicted_out = static_cast<int64_t>(predicted);
-  Int quantized;
-  if (kReplay) {
-    quantized = static_cast<Int>(*quantized_out);
-  } else {
-    float residual = scaled_value;
-    residual -= static_cast<float>(predicted);
-    if (residual > -0.62f && residual < 0.62f) residual = 0.0f;
-    float rounded = roundf(residual);
-    if (rounded > 2.0f || rounded < -2.0f) rounded = roundf(residual * 0.5f) * 2.0f;
-    quantized = predicted + static_cast<Int>(rounded);
-    *quantized_out = static_cast<int32_t>(quantized);
+  DcStepOutput out;
+  out.predicted = (prediction + 3) >> 3;
+  int64_t quantized = in.replayed;
+  if (!kReplay) {
+    quantized = out.predicted + static_cast<int64_t>(DcResidualSteps(
+                                  in.scaled_value, static_cast<float>(out.predicted)));
   }
+  out.quantized = static_cast<int32_t>(quantized);
   // Update (prediction.h:121-141).
-  const Int scaled = quantized * 8;
-  *error_out = static_cast<int32_t>(prediction - scaled);
-#pragma unroll
+  const int64_t scaled = quantized * 8;
+  out.error = static_cast<int32_t>(prediction - scaled);
   for (int i = 0; i < 4; ++i) {
-    const Int d = predictions[i] - scaled;
-    sub_errors[i] = static_cast<uint32_t>(((d < 0 ? -d : d) + 3) >> 3);
+    const int64_t d = predictions[i] - scaled;
+    out.sub[i] = static_cast<uint32_t>(((d < 0 ? -d : d) + 3) >> 3);
   }
+  return out;
 }
 
+__device__ __forceinline__ int HighestBit(uint32_t v) {
+  int r;
+  asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+
+// The same in 32 bits, within the bounds above: the chain that sets the
+// kernel's time, so every value that does not depend on the last sample comes
+// first.
 template <bool kReplay>
+__device__ __forceinline__ DcStepOutput NarrowDcStep(const DcStepInput& in,
+                                                     const uint32_t* reciprocal) {
+  const int32_t max_weights[4] = {13, 12, 12, 12};
+  const int32_t n8 = in.n * 8, ne8 = in.ne * 8, w8 = in.w * 8;
+  uint32_t weights[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int shift = max(HighestBit(in.errors[i] + 1u) - 5, 0);
+    weights[i] = 4 + ((max_weights[i] * reciprocal[in.errors[i] >> shift]) >> shift);
+  }
+  const int drop = HighestBit((weights[0] + weights[1]) + (weights[2] + weights[3])) - 4;
+  int32_t predictions[4];
+  predictions[0] = w8 + (ne8 - n8);
+  predictions[1] = n8 - (((in.en + in.ene + in.ew) * 16) >> 5);
+  predictions[2] = w8 - (((in.en + in.enw + in.ew) * 10) >> 5);
+  predictions[3] = n8 - (((in.enw + in.en + in.ene) * 7) >> 5);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) weights[i] >>= drop;
+  const uint32_t weight_sum = (weights[0] + weights[1]) + (weights[2] + weights[3]);
+  const int32_t sum =
+    (predictions[0] * static_cast<int32_t>(weights[0]) +
+     predictions[1] * static_cast<int32_t>(weights[1])) +
+    (predictions[2] * static_cast<int32_t>(weights[2]) +
+     predictions[3] * static_cast<int32_t>(weights[3])) +
+    (static_cast<int32_t>(weight_sum >> 1) - 1);
+  int32_t prediction = static_cast<int32_t>(
+    (static_cast<int64_t>(sum) * static_cast<int32_t>(reciprocal[weight_sum - 1])) >> 24);
+  const int32_t lo = min(w8, min(ne8, n8)), hi = max(w8, max(ne8, n8));
+  const int32_t clamped = min(max(prediction, lo), hi);
+  if (((in.en ^ in.ew) | (in.en ^ in.enw)) <= 0) prediction = clamped;
+  const int32_t predicted = (prediction + 3) >> 3;
+  DcStepOutput out;
+  out.predicted = predicted;
+  out.quantized = kReplay ? in.replayed
+                          : predicted + static_cast<int32_t>(DcResidualSteps(
+                                          in.scaled_value, static_cast<float>(predicted)));
+  const int32_t scaled = out.quantized * 8;
+  out.error = prediction - scaled;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    out.sub[i] = static_cast<uint32_t>((abs(predictions[i] - scaled) + 3) >> 3);
+  }
+  return out;
+}
+
+// Barrier 1 over the CTA's `threads` working threads.
+__device__ __forceinline__ void DcBarrier(int threads) {
+  asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
+
+template <bool kReplay, bool kTokens>
 __global__ void __launch_bounds__(kDcThreads, 1)
 DcQuantKernel(const __grid_constant__ DcQuantParams p) {
   extern __shared__ __align__(16) unsigned char dc_smem[];
-  DcRings& r = *reinterpret_cast<DcRings*>(dc_smem);
+  DcShared& r = *reinterpret_cast<DcShared*>(dc_smem);
   const int gx0 = blockIdx.x * kDcGroup, gy0 = blockIdx.y * kDcGroup;
   const int gw = min(kDcGroup, p.width - gx0), gh = min(kDcGroup, p.height - gy0);
   const int stride = p.width;
-  const bool idle = blockIdx.z == 0 && threadIdx.x >= kDcGroup;
-  const int c = blockIdx.z == 0 ? 0 : 1 + static_cast<int>(threadIdx.x) / kDcGroup;  // X, Y, B
-  const int y = idle ? kDcGroup : static_cast<int>(threadIdx.x) % kDcGroup;
-  const int lag = c == 2 ? 1 : 0;
   for (int i = threadIdx.x; i < 64; i += blockDim.x) r.reciprocal[i] = (1u << 24) / (i + 1);
-  if (p.tokens != nullptr) {
+  if (kTokens) {
     for (int i = threadIdx.x; i < 1024; i += blockDim.x)
       r.contexts[i] = static_cast<uint8_t>(DcContextOfIndex(i));
   }
+  for (int i = threadIdx.x; i < 3 * kDcSlots; i += blockDim.x) {
+    r.last_values[i / kDcSlots][0][i % kDcSlots] = make_int4(0, 0, 0, 0);
+    r.last_errors[i / kDcSlots][0][i % kDcSlots] = make_uint4(0, 0, 0, 0);
+  }
   if (threadIdx.x == 0) r.wide = 0;
+  __syncthreads();
+  // Warps past the group's rows, and X's unused half, have nothing to do.
+  const int warps = (gh + kDcRows - 1) / kDcRows;
+  const int half = static_cast<int>(threadIdx.x) / kDcGroup;
+  const int warp = static_cast<int>(threadIdx.x) % kDcGroup / kDcRows;
+  const int lane = static_cast<int>(threadIdx.x) % kDcRows;
+  if (warp >= warps || (blockIdx.z == 0 && half == 1)) return;
+  const int working = warps * kDcRows * (blockIdx.z == 0 ? 1 : 2);
+  const int c = blockIdx.z == 0 ? 0 : 1 + half;  // X; Y, B
+  const int y = warp * kDcRows + lane;
+  const int start = warp * kDcWarpSkew + (c == 2 ? kDcSync : 0);
   const AqQuantizer q = kReplay ? AqQuantizer{} : *p.q;
   const float inverse_step = kReplay ? 0.0f : q.inverse_dc_steps[c] * p.precision;
   const float step_y = kReplay ? 0.0f : q.dc_steps[1] / p.precision;
-  int32_t* plane = kReplay ? nullptr : p.quantized + c * p.pitch;
-  // The samples: DC values to quantize, or quantized values to replay, read
-  // as raw 32-bit words.
-  const uint32_t* source = kReplay ? reinterpret_cast<const uint32_t*>(p.replay + c * p.pitch)
-                                   : reinterpret_cast<const uint32_t*>(p.dc + c * p.pitch);
-  uint2* tokens = p.tokens == nullptr
-                    ? nullptr
-                    : p.tokens + DcTokenOffset(blockIdx.x, blockIdx.y, p.width, p.height) +
-                        static_cast<size_t>(DcChannelRank(c)) * gw * gh;
-  int32_t (*Q)[kDcGroup] = r.q[c];
-  int32_t (*E)[kDcGroup] = r.e[c];
-  __syncthreads();
-  // The sample of the next position is loaded one wave ahead, so its
-  // global-memory latency overlaps this wave's work and barrier.
+  // This row's samples (DC values to quantize, or quantized values to replay,
+  // read as raw 32-bit words) and outputs.
   const size_t row_index = static_cast<size_t>(gy0 + min(y, gh - 1)) * stride + gx0;
-  uint32_t pending = y < gh ? source[row_index] : 0u;  // idle threads have y >= gh
-  // This row's previous quantized value and signed error (its west
-  // neighbour), kept in registers.
-  int32_t own_q = 0, own_e = 0;
-  const int waves = (gw - 1) + 2 * (gh - 1) + 2;
-  for (int t = 0; t < waves; ++t) {
-    const int x = t - lag - 2 * y;
-    const int wide = r.wide;
-    if (y < gh && x >= 0 && x < gw) {
-      const uint32_t sample = pending;
-      if (x + 1 < gw) pending = source[row_index + x + 1];
-      const int s = x & 7, sw = (x - 1) & 7, sne = (x + 1 < gw ? x + 1 : x) & 7;
-      const int snw = (x ? x - 1 : x) & 7;
-      const int up = y - 1, up2 = y - 2;
-      const int32_t w = x ? own_q : y ? Q[s][up] : 0;
-      const int32_t n = y ? Q[s][up] : w;
-      const int32_t nw = x && y ? Q[sw][up] : w;
-      const int32_t ne = y && x + 1 < gw ? Q[(x + 1) & 7][up] : n;
-      const int32_t nn = y > 1 ? Q[s][up2] : n;
-      const int32_t ew = x ? own_e : 0;
-      const int32_t en = y ? E[s][up] : 0;
-      const int32_t enw = y ? E[snw][up] : 0;
-      const int32_t ene = y ? E[sne][up] : 0;
-      // Sub-predictor error sums (prediction.h:73-90). The signed errors of
-      // row -1 read as zeros. The error sums of row 0 read the predictor's
-      // other rolling row, which by then holds only row 0's own "+="
-      // updates: its entry j carries the error of (j - 1, 0) once that
-      // sample is done, so north = err(x-1), northwest = err(x-2) and
-      // northeast (not yet written) = 0, or north at the right edge.
-      uint32_t errors[4];
+  const uint32_t* source = (kReplay ? reinterpret_cast<const uint32_t*>(p.replay)
+                                    : reinterpret_cast<const uint32_t*>(p.dc)) +
+                           c * p.pitch + row_index;
+  int32_t* plane = kReplay ? nullptr : p.quantized + c * p.pitch + row_index;
+  uint2* tokens = !kTokens ? nullptr
+                           : p.tokens + DcTokenOffset(blockIdx.x, blockIdx.y, p.width, p.height) +
+                               (static_cast<size_t>(DcChannelRank(c)) * gh + y) * gw;
+  uint32_t* ring = &r.samples[0][threadIdx.x];
+  // The row above the warp's first one: its predecessor's last, or zeros.
+  const int4* previous_values = r.last_values[c][warp];
+  const uint4* previous_errors = r.last_errors[c][warp];
+  // The row above at x-1, x, x+1 (`west`, `here`, `east`: values; zero errors
+  // above the group's first row) and this row's last sample. Past the row's
+  // ends the nearest sample stands in, as the reference reads it: the west
+  // side is set up one step before the row starts, and on the east side the
+  // lane above has stopped at its last sample.
+  int32_t west_q = 0, west_e = 0, here_q = 0, here_e = 0, here_n = 0;
+  int32_t own_q = 0, own_e = 0, own_n = 0;
+  // Sub-predictor errors: the row above's at x, this row's at x-1, and the
+  // sum of the row above's at x-1 and x and this row's at x-2.
+  uint32_t here_pe[4] = {0, 0, 0, 0}, own_pe[4] = {0, 0, 0, 0}, sum_pe[4] = {0, 0, 0, 0};
+  int4 next_values = make_int4(0, 0, 0, 0);  // lane 0: the next step's `east`
+  uint4 next_errors = make_uint4(0, 0, 0, 0);
+  const unsigned row_width = y < gh ? static_cast<unsigned>(gw) : 0u;
+  int wide = 0;
+  const int steps = kDcSync + gw + 2 * ((gh - 1) % kDcRows) + (warps - 1) * kDcWarpSkew +
+                    (blockIdx.z == 0 ? 0 : kDcSync);
+  for (int t = 0; t < steps; ++t) {
+    const int first = t - kDcSync - start;  // lane 0's position
+    if (first >= -kDcSync && first < gw + 2 * (kDcRows - 1)) {
+      const int x = first - 2 * lane;
+      if (t % kDcSync == 0) {
+        // The samples of the kDcSync steps after these; those of these steps
+        // were requested kDcSync steps ago.
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (y) {
-          errors[i] = r.pe[c][i][s][up] + r.pe[c][i][sne][up] + r.pe[c][i][snw][up];
-        } else {
-          const uint32_t north = x ? r.row0[c][i][sw] : 0u;
-          const uint32_t northeast = x + 1 < gw ? 0u : north;
-          const uint32_t northwest = x >= 2 ? r.row0[c][i][(x - 2) & 7] : 0u;
-          errors[i] = north + northeast + northwest;
+        for (int i = 0; i < kDcSync; ++i) {
+          const int ahead = x + kDcSync + i;
+          if (static_cast<unsigned>(ahead) < row_width) {
+            const uint32_t slot = static_cast<uint32_t>(
+              __cvta_generic_to_shared(ring + (ahead & (kDcSampleSlots - 1)) * kDcThreads));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(slot),
+                         "l"(source + ahead)
+                         : "memory");
+          }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      }
+      int32_t east_q = __shfl_up_sync(0xffffffffu, own_q, 1);
+      int32_t east_e = __shfl_up_sync(0xffffffffu, own_e, 1);
+      int32_t east_n = __shfl_up_sync(0xffffffffu, own_n, 1);
+      uint32_t east_pe[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) east_pe[i] = __shfl_up_sync(0xffffffffu, own_pe[i], 1);
+      if (lane == 0) {
+        east_q = next_values.x;
+        east_e = next_values.y;
+        east_n = next_values.z;
+        east_pe[0] = next_errors.x;
+        east_pe[1] = next_errors.y;
+        east_pe[2] = next_errors.z;
+        east_pe[3] = next_errors.w;
+      }
+      const int next_slot = min(first + 2, gw - 1) & (kDcSlots - 1);
+      next_values = previous_values[next_slot];
+      next_errors = previous_errors[next_slot];
+      // The group's first row: its west neighbour stands in for the row above.
+      if (y == 0) west_q = here_q = east_q = here_n = own_q;
+      if (first < 2 * kDcRows && x == -1) {
+        here_q = own_q = east_q;
+        here_e = east_e;
+        here_n = east_n;
+        own_e = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          here_pe[i] = east_pe[i];
+          own_pe[i] = 0;
         }
       }
-      float scaled_value = 0.0f;
-      int32_t quantized = 0, error_value;
-      bool narrow;
-      if (kReplay) {
-        quantized = static_cast<int32_t>(sample);
-        narrow = quantized > -kDcNarrowQuantized && quantized < kDcNarrowQuantized;
-      } else {
-        float value = __uint_as_float(sample);
-        if (c == 2) value = fmaf(-static_cast<float>(r.q[1][s][y]), step_y, value);
-        scaled_value = value * inverse_step;
-        narrow = fabsf(scaled_value) < kDcNarrowScaled;
-      }
-      uint32_t sub[4];
-      int64_t predicted;
-      if (!wide && narrow) {
-        WeightedPredictorStep<int32_t, false, kReplay>(w, n, nw, ne, nn, ew, en, enw, ene,
-                                                       errors, r.reciprocal, scaled_value,
-                                                       &quantized, &error_value, sub,
-                                                       &predicted);
-      } else {
-        WeightedPredictorStep<int64_t, true, kReplay>(w, n, nw, ne, nn, ew, en, enw, ene,
-                                                      errors, r.reciprocal, scaled_value,
-                                                      &quantized, &error_value, sub,
-                                                      &predicted);
-      }
-      // Later steps read this value: past the 32-bit bounds, every later
-      // step of the CTA takes the 64-bit form.
-      if (static_cast<uint32_t>(quantized) + static_cast<uint32_t>(kDcNarrowQuantized) >
+      uint32_t sub[4] = {own_pe[0], own_pe[1], own_pe[2], own_pe[3]};
+      bool exceeds = false;
+      if (static_cast<unsigned>(x) < row_width) {
+        const uint32_t sample = ring[(x & (kDcSampleSlots - 1)) * kDcThreads];
+        DcStepInput in;
+        in.w = own_q;
+        in.n = here_q;
+        in.nw = west_q;
+        in.ne = east_q;
+        in.nn = here_n;
+        in.ew = own_e;
+        in.en = here_e;
+        in.enw = west_e;
+        in.ene = east_e;
+        // Sub-predictor error sums (prediction.h:73-90): north, northeast and
+        // northwest. Each of this row's samples adds its errors to the entry
+        // above its east neighbour, so north carries the last sample's and
+        // northwest those of the one before; at the right edge north counts
+        // for northeast. Above the first row there are only those additions:
+        // the reference's rolling rows hold row 0's own errors there, one
+        // entry late.
+        const uint32_t repeat = x + 1 < gw ? 1u : 2u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) in.errors[i] = sum_pe[i] + east_pe[i] + own_pe[i] * repeat;
+        in.scaled_value = 0.0f;
+        in.replayed = static_cast<int32_t>(sample);
+        bool narrow;
+        if (kReplay) {
+          narrow = in.replayed > -kDcNarrowQuantized && in.replayed < kDcNarrowQuantized;
+        } else {
+          float value = __uint_as_float(sample);
+          if (c == 2) {
+            value = fmaf(-static_cast<float>(r.luma[x & (kDcSlots - 1)][y]), step_y, value);
+          }
+          in.scaled_value = value * inverse_step;
+          narrow = fabsf(in.scaled_value) < kDcNarrowScaled;
+        }
+        const DcStepOutput out = !wide && narrow ? NarrowDcStep<kReplay>(in, r.reciprocal)
+                                                 : WideDcStep<kReplay>(in, r.reciprocal);
+        // Later steps read this value: past the 32-bit bounds, every step
+        // that can see it takes the 64-bit form.
+        exceeds =
+          static_cast<uint32_t>(out.quantized) + static_cast<uint32_t>(kDcNarrowQuantized) >
             static_cast<uint32_t>(2 * kDcNarrowQuantized) ||
-          static_cast<uint32_t>(error_value) + static_cast<uint32_t>(kDcNarrowError) >
-            static_cast<uint32_t>(2 * kDcNarrowError)) {
-        r.wide = 1;
+          static_cast<uint32_t>(out.error) + static_cast<uint32_t>(kDcNarrowError) >
+            static_cast<uint32_t>(2 * kDcNarrowError);
+        if (!kReplay) plane[x] = out.quantized;
+        if (kTokens) {
+          // The weighted predictor's context property: of ew, en, enw, ene the
+          // first with the largest magnitude (prediction.h:95-99); the token is
+          // the packed residual against the prediction (weighted_dc.cpp:67-80).
+          int64_t property = in.ew;
+          if (llabs(static_cast<int64_t>(in.en)) > llabs(property)) property = in.en;
+          if (llabs(static_cast<int64_t>(in.enw)) > llabs(property)) property = in.enw;
+          if (llabs(static_cast<int64_t>(in.ene)) > llabs(property)) property = in.ene;
+          const int64_t index = property < -512 ? 0 : property > 511 ? 1023 : 512 + property;
+          const int64_t residual = static_cast<int64_t>(out.quantized) - out.predicted;
+          if (residual < INT32_MIN || residual > INT32_MAX) RaiseError(p.error, kErrorRange);
+          tokens[x] = make_uint2(r.contexts[index], PackSigned(static_cast<int32_t>(residual)));
+        }
+        own_q = out.quantized;
+        own_e = out.error;
+        own_n = y == 0 ? out.quantized : in.n;  // row 1's second row above is row 0 itself
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sub[i] = out.sub[i];
+        const int slot = x & (kDcSlots - 1);
+        if (!kReplay && c == 1) r.luma[slot][y] = out.quantized;
+        if (lane == kDcRows - 1) {
+          r.last_values[c][warp + 1][slot] = make_int4(own_q, own_e, own_n, 0);
+          r.last_errors[c][warp + 1][slot] = make_uint4(sub[0], sub[1], sub[2], sub[3]);
+        }
       }
-      if (!kReplay) plane[row_index + x] = quantized;
-      if (tokens != nullptr) {
-        // The weighted predictor's context property: of ew, en, enw, ene the
-        // first with the largest magnitude (prediction.h:95-99); the token is
-        // the packed residual against the prediction (weighted_dc.cpp:67-80).
-        int64_t property = ew;
-        if (llabs(static_cast<int64_t>(en)) > llabs(property)) property = en;
-        if (llabs(static_cast<int64_t>(enw)) > llabs(property)) property = enw;
-        if (llabs(static_cast<int64_t>(ene)) > llabs(property)) property = ene;
-        const int64_t index = property < -512 ? 0 : property > 511 ? 1023 : 512 + property;
-        const int64_t residual = static_cast<int64_t>(quantized) - predicted;
-        if (residual < INT32_MIN || residual > INT32_MAX) RaiseError(p.error, kErrorRange);
-        tokens[y * gw + x] = make_uint2(r.contexts[index],
-                                        PackSigned(static_cast<int32_t>(residual)));
-      }
-      Q[s][y] = quantized;
-      E[s][y] = error_value;
-      own_q = quantized;
-      own_e = error_value;
+      west_q = here_q;
+      west_e = here_e;
+      here_q = east_q;
+      here_e = east_e;
+      here_n = east_n;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        r.pe[c][i][s][y] = sub[i];
-        if (y && x + 1 < gw) r.pe[c][i][(x + 1) & 7][up] += sub[i];
-        if (!y) r.row0[c][i][s] = sub[i];
+        sum_pe[i] = here_pe[i] + east_pe[i] + own_pe[i];
+        here_pe[i] = east_pe[i];
+        own_pe[i] = sub[i];
+      }
+      if (__any_sync(0xffffffffu, exceeds)) {
+        wide = 1;
+        if (lane == 0) r.wide = 1;
       }
     }
-    __syncthreads();
+    if (t % kDcSync == kDcSync - 1) {
+      DcBarrier(working);
+      wide |= *const_cast<volatile int*>(&r.wide);
+    }
   }
 }
 
@@ -1768,16 +1919,16 @@ int AqCoding(const int2* lists, const uint32_t* counts, size_t bx, size_t by, co
 
 namespace {
 
-template <bool kReplay>
+template <bool kReplay, bool kTokens>
 int LaunchDcQuant(const DcQuantParams& p, size_t bx, size_t by, cudaStream_t stream) {
-  const int smem = static_cast<int>(sizeof(DcRings));
-  int status = CheckCuda(cudaFuncSetAttribute(DcQuantKernel<kReplay>,
+  const int smem = static_cast<int>(sizeof(DcShared));
+  int status = CheckCuda(cudaFuncSetAttribute(DcQuantKernel<kReplay, kTokens>,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                          "dc predictor attribute");
   if (status != GJXL_B200_OK) return status;
   dim3 grid(static_cast<unsigned>((bx + kDcGroup - 1) / kDcGroup),
             static_cast<unsigned>((by + kDcGroup - 1) / kDcGroup), 2);
-  DcQuantKernel<kReplay><<<grid, kDcThreads, smem, stream>>>(p);
+  DcQuantKernel<kReplay, kTokens><<<grid, kDcThreads, smem, stream>>>(p);
   return CheckLaunch("dc predictor");
 }
 
@@ -1798,7 +1949,8 @@ int AqDcQuantize(const float* dc, size_t bx, size_t by, const AqQuantizer* q, in
   p.precision = static_cast<float>(1u << extra_precision);
   p.tokens = tokens;
   p.error = error;
-  int status = LaunchDcQuant<false>(p, bx, by, stream);
+  int status = tokens != nullptr ? LaunchDcQuant<false, true>(p, bx, by, stream)
+                                 : LaunchDcQuant<false, false>(p, bx, by, stream);
   if (status != GJXL_B200_OK) return status;
   DcDequantKernel<<<Blocks(bx * by), kThreads, 0, stream>>>(
     quantized, reconstructed, static_cast<int>(bx * by), bx * by, q, p.precision);
@@ -1815,7 +1967,7 @@ int DcWeightedTokens(const int32_t* quantized, size_t pitch, size_t bx, size_t b
   p.replay = quantized;
   p.tokens = tokens;
   p.error = error;
-  return LaunchDcQuant<true>(p, bx, by, stream);
+  return LaunchDcQuant<true, true>(p, bx, by, stream);
 }
 
 int AqInverseSigma(const uint8_t* cells, size_t bx, size_t by, const int32_t* raw,
