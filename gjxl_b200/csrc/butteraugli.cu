@@ -188,7 +188,15 @@ constexpr int kRowSegment = kThreads * kRowRun;
 constexpr int kBlurRows = 2;
 
 template <int R>
-__global__ void __launch_bounds__(kThreads)
+__device__ __forceinline__ void BlurRowBorders(const float* in, float* out, int w, int h,
+                                               size_t in_pitch, size_t out_pitch,
+                                               const Kernel17& k);
+
+template <int R>
+// The CTAs per SM bound the registers to what the row pass needs: the ends'
+// unrolled sums would take a third more and cost every CTA its occupancy (26 us
+// for a 2048x1536 plane triple and its half scale at R = 7 against 16).
+__global__ void __launch_bounds__(kThreads, R > 8 ? 4 : 6)
 BlurRowsKernel(const float* in, float* out, int w, int h, size_t in_pitch, size_t out_pitch,
                const __grid_constant__ Kernel17 k) {
   constexpr int kWindow = kRowRun + 2 * R;
@@ -198,6 +206,10 @@ BlurRowsKernel(const float* in, float* out, int w, int h, size_t in_pitch, size_
   __shared__ __align__(16) float segment[kBlurRows][kPitch];
   const int plane = blockIdx.z;
   const int x0 = blockIdx.x * kRowSegment;
+  if (x0 >= w) {
+    BlurRowBorders<R>(in, out, w, h, in_pitch, out_pitch, k);
+    return;
+  }
   const float* base = in + plane * in_pitch;
   // Rows beyond the grid's y extent (65535 row groups) are taken in further
   // rounds.
@@ -259,24 +271,28 @@ BlurRowsKernel(const float* in, float* out, int w, int h, size_t in_pitch, size_
 }
 
 // The outputs within R of either row end (ConvolveLine's renormalized border
-// sum), for the rows of the row-blur CTAs: one thread per row and border
-// position, so that the row-blur CTAs run no divergent border code. The
+// sum): the work of the CTAs past a row's last segment, one thread per row
+// and border position, so that the others run no divergent border code. The
 // positions are x = 0..R-1 and x = w-2R+R..w-1, the latter kept only where
-// x >= R (narrow rows).
+// x >= R (narrow rows). As a launch of its own it took 3 us per blur of a
+// 256x256 image.
 template <int R>
-__global__ void __launch_bounds__(kThreads)
-BlurRowBordersKernel(const float* in, float* out, int w, int h, size_t in_pitch,
-                     size_t out_pitch, const __grid_constant__ Kernel17 k) {
+__device__ __forceinline__ void BlurRowBorders(const float* in, float* out, int w, int h,
+                                               size_t in_pitch, size_t out_pitch,
+                                               const Kernel17& k) {
   constexpr int kPerRow = 2 * R;
   constexpr int kRowsPerCta = kThreads / kPerRow;
-  const int plane = blockIdx.y;
+  const int plane = blockIdx.z;
   const int r = threadIdx.x / kPerRow, item = threadIdx.x % kPerRow;
-  const int y = blockIdx.x * kRowsPerCta + r;
-  if (r >= kRowsPerCta || y >= h) return;
+  if (r >= kRowsPerCta) return;
   const int x = item < R ? item : w - kPerRow + item;
   if (item < R ? x >= w : (x < R || x >= w)) return;
-  const float* row = in + plane * in_pitch + static_cast<size_t>(y) * w;
-  out[plane * out_pitch + static_cast<size_t>(y) * w + x] = ConvolveBorder<R>(row, 1, x, w, k);
+  for (int64_t y = static_cast<int64_t>(blockIdx.y) * kRowsPerCta + r; y < h;
+       y += static_cast<int64_t>(gridDim.y) * kRowsPerCta) {
+    const float* row = in + plane * in_pitch + static_cast<size_t>(y) * w;
+    out[plane * out_pitch + static_cast<size_t>(y) * w + x] =
+      ConvolveBorder<R>(row, 1, x, w, k);
+  }
 }
 
 template <int R>
@@ -489,113 +505,204 @@ __device__ __forceinline__ float MaltaScaledValue(const MaltaScale& p, float v0,
   return scaled;
 }
 
-// After the 33-tap blur of all three XYB planes into psycho LF: MF = xyb - LF
-// and the LF scaling (butteraugli_internal.cpp:750-776).
-__global__ void __launch_bounds__(kThreads)
-FrequencyLowKernel(const float* xyb, float* psycho, int n, size_t pitch, uint32_t* error) {
-  const int i = blockIdx.x * kThreads + threadIdx.x;
-  if (i >= n) return;
-  // All loads first: `psycho` is read and written, so loads after a store
-  // could not be moved ahead of it.
-  float lf[3], v[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    lf[c] = psycho[(kLF + c) * pitch + i];
-    v[c] = xyb[c * pitch + i];
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) psycho[(kMF + c) * pitch + i] = v[c] - lf[c];
-  const float l2 = (-0.362267051518f * lf[1] + lf[2]) * 49.87984651440f;
-  const float l0 = lf[0] * 33.832837186260f;
-  const float l1 = lf[1] * 14.458268100570f;
-  psycho[(kLF + 2) * pitch + i] = l2;
-  psycho[(kLF + 0) * pitch + i] = l0;
-  psycho[(kLF + 1) * pitch + i] = l1;
-  if (!(IsFinite(l0) && IsFinite(l1) && IsFinite(l2))) RaiseError(error, kErrorNonFiniteOutput);
-}
-
-// After the 15-tap blur of MF into `blurred` (3 planes): HF = MF - blurred
-// (X, Y), MF ranges, MF_B = blurred, then X suppression by Y
-// (butteraugli_internal.cpp:778-810).
-// The Malta stages' scaled differences of the distorted image against the
-// reference, written beside the final planes they are taken from (plane k of
-// `malta` for stage k: MF_Y, MF_X, HF_Y, HF_X, UHF_Y, UHF_X), so that each
-// is computed once per pixel instead of once per Malta tile that reads it.
+// The steps of the frequency separation that follow a blur, each given pixel
+// i's blurred samples. `ref` set (the distorted image): also the Malta stages'
+// scaled differences against the reference, beside the final planes they are
+// taken from (plane k of `malta` for stage k: MF_Y, MF_X, HF_Y, HF_X, UHF_Y,
+// UHF_X), so that each is computed once per pixel instead of once per Malta
+// tile that reads it.
 struct MaltaPlanes {
   const float* ref;  // reference psycho planes; null: the reference itself
   float* malta;      // 6 planes
   MaltaScale scale[6];
 };
 
-__global__ void __launch_bounds__(kThreads)
-FrequencyHighKernel(const float* blurred, float* psycho, int n, size_t pitch, uint32_t* error,
-                    const __grid_constant__ MaltaPlanes m) {
-  const int i = blockIdx.x * kThreads + threadIdx.x;
-  if (i >= n) return;
-  const float mv0 = blurred[i], mv1 = blurred[pitch + i], mf_b = blurred[2 * pitch + i];
-  float ref_mf0 = 0.0f, ref_mf1 = 0.0f;
-  if (m.ref != nullptr) {
-    ref_mf0 = m.ref[(kMF + 0) * pitch + i];
-    ref_mf1 = m.ref[(kMF + 1) * pitch + i];
+// After the 33-tap blur of all three XYB planes: MF = xyb - LF and the LF
+// scaling (butteraugli_internal.cpp:750-776).
+struct FrequencyLow {
+  static constexpr int kPlanes = 3;
+  static constexpr bool kPreload = true;
+  const float* xyb;
+  float* psycho;
+  size_t pitch;
+  uint32_t* error;
+  struct Loaded {
+    float v[3];
+  };
+  __device__ __forceinline__ Loaded Load(size_t i) const {
+    Loaded l;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) l.v[c] = xyb[c * pitch + i];
+    return l;
   }
-  const float hf0 = psycho[(kMF + 0) * pitch + i] - mv0;
-  const float hf1 = psycho[(kMF + 1) * pitch + i] - mv1;
-  const float mf0 = RemoveRangeAroundZero(mv0, 0.29f);
-  const float mf1 = AmplifyRangeAroundZero(mv1, 0.1f);
-  psycho[(kMF + 0) * pitch + i] = mf0;
-  psycho[(kMF + 1) * pitch + i] = mf1;
-  psycho[(kMF + 2) * pitch + i] = mf_b;
-  constexpr float kSuppress = 46.0f, kMinimumScale = 0.653020556257f;
-  const float scaler =
-    kSuppress / (hf1 * hf1 + kSuppress) * (1.0f - kMinimumScale) + kMinimumScale;
-  psycho[(kHF + 0) * pitch + i] = scaler * hf0;
-  psycho[(kHF + 1) * pitch + i] = hf1;
-  if (m.ref != nullptr) {
-    m.malta[0 * pitch + i] = MaltaScaledValue(m.scale[0], ref_mf1, mf1);
-    m.malta[1 * pitch + i] = MaltaScaledValue(m.scale[1], ref_mf0, mf0);
+  __device__ __forceinline__ void operator()(size_t i, const Loaded& l,
+                                             const float (&lf)[3]) const {
+    const float (&v)[3] = l.v;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) psycho[(kMF + c) * pitch + i] = v[c] - lf[c];
+    const float l2 = (-0.362267051518f * lf[1] + lf[2]) * 49.87984651440f;
+    const float l0 = lf[0] * 33.832837186260f;
+    const float l1 = lf[1] * 14.458268100570f;
+    psycho[(kLF + 2) * pitch + i] = l2;
+    psycho[(kLF + 0) * pitch + i] = l0;
+    psycho[(kLF + 1) * pitch + i] = l1;
+    if (!(IsFinite(l0) && IsFinite(l1) && IsFinite(l2))) RaiseError(error, kErrorNonFiniteOutput);
   }
-  // Finiteness of the final MF planes (the HF planes are rewritten, and
-  // checked, by FrequencyUltraKernel).
-  if (!(IsFinite(mf0) & IsFinite(mf1) & IsFinite(mf_b))) RaiseError(error, kErrorNonFiniteOutput);
-}
+};
 
-// After the 7-tap blur of HF into `blurred` (2 planes): UHF and final HF
+// After the 15-tap blur of MF (3 planes): HF = MF - blurred (X, Y), MF ranges,
+// MF_B = blurred, then X suppression by Y (butteraugli_internal.cpp:778-810).
+struct FrequencyHigh {
+  static constexpr int kPlanes = 3;
+  static constexpr bool kPreload = true;
+  float* psycho;
+  size_t pitch;
+  uint32_t* error;
+  MaltaPlanes m;
+  struct Loaded {
+    float mf0, mf1, ref_mf0, ref_mf1;
+  };
+  __device__ __forceinline__ Loaded Load(size_t i) const {
+    Loaded l = {psycho[(kMF + 0) * pitch + i], psycho[(kMF + 1) * pitch + i], 0.0f, 0.0f};
+    if (m.ref != nullptr) {
+      l.ref_mf0 = m.ref[(kMF + 0) * pitch + i];
+      l.ref_mf1 = m.ref[(kMF + 1) * pitch + i];
+    }
+    return l;
+  }
+  __device__ __forceinline__ void operator()(size_t i, const Loaded& l,
+                                             const float (&blurred)[3]) const {
+    const float mv0 = blurred[0], mv1 = blurred[1], mf_b = blurred[2];
+    const float ref_mf0 = l.ref_mf0, ref_mf1 = l.ref_mf1;
+    const float hf0 = l.mf0 - mv0;
+    const float hf1 = l.mf1 - mv1;
+    const float mf0 = RemoveRangeAroundZero(mv0, 0.29f);
+    const float mf1 = AmplifyRangeAroundZero(mv1, 0.1f);
+    psycho[(kMF + 0) * pitch + i] = mf0;
+    psycho[(kMF + 1) * pitch + i] = mf1;
+    psycho[(kMF + 2) * pitch + i] = mf_b;
+    constexpr float kSuppress = 46.0f, kMinimumScale = 0.653020556257f;
+    const float scaler =
+      kSuppress / (hf1 * hf1 + kSuppress) * (1.0f - kMinimumScale) + kMinimumScale;
+    psycho[(kHF + 0) * pitch + i] = scaler * hf0;
+    psycho[(kHF + 1) * pitch + i] = hf1;
+    if (m.ref != nullptr) {
+      m.malta[0 * pitch + i] = MaltaScaledValue(m.scale[0], ref_mf1, mf1);
+      m.malta[1 * pitch + i] = MaltaScaledValue(m.scale[1], ref_mf0, mf0);
+    }
+    // Finiteness of the final MF planes (the HF planes are rewritten, and
+    // checked, by FrequencyUltra).
+    if (!(IsFinite(mf0) & IsFinite(mf1) & IsFinite(mf_b))) {
+      RaiseError(error, kErrorNonFiniteOutput);
+    }
+  }
+};
+
+// After the 7-tap blur of HF (2 planes): UHF and final HF
 // (butteraugli_internal.cpp:812-849).
-__global__ void __launch_bounds__(kThreads)
-FrequencyUltraKernel(const float* blurred, float* psycho, int n, size_t pitch,
-                     uint32_t* error, const __grid_constant__ MaltaPlanes m) {
-  const int i = blockIdx.x * kThreads + threadIdx.x;
-  if (i >= n) return;
-  float ref_hf0 = 0.0f, ref_hf1 = 0.0f, ref_uhf0 = 0.0f, ref_uhf1 = 0.0f;
-  if (m.ref != nullptr) {
-    ref_hf0 = m.ref[(kHF + 0) * pitch + i];
-    ref_hf1 = m.ref[(kHF + 1) * pitch + i];
-    ref_uhf0 = m.ref[(kUHF + 0) * pitch + i];
-    ref_uhf1 = m.ref[(kUHF + 1) * pitch + i];
+struct FrequencyUltra {
+  static constexpr int kPlanes = 2;
+  static constexpr bool kPreload = false;  // six values of four pixels: too many registers
+  float* psycho;
+  size_t pitch;
+  uint32_t* error;
+  MaltaPlanes m;
+  __device__ __forceinline__ void operator()(size_t i, const float (&blurred)[2]) const {
+    float ref_hf0 = 0.0f, ref_hf1 = 0.0f, ref_uhf0 = 0.0f, ref_uhf1 = 0.0f;
+    if (m.ref != nullptr) {
+      ref_hf0 = m.ref[(kHF + 0) * pitch + i];
+      ref_hf1 = m.ref[(kHF + 1) * pitch + i];
+      ref_uhf0 = m.ref[(kUHF + 0) * pitch + i];
+      ref_uhf1 = m.ref[(kUHF + 1) * pitch + i];
+    }
+    const float hv0 = blurred[0];
+    const float ultra0 = psycho[(kHF + 0) * pitch + i];
+    const float uhf0 = RemoveRangeAroundZero(ultra0 - hv0, 0.04f);
+    const float hf0 = RemoveRangeAroundZero(hv0, 1.5f);
+    const float hv1 = MaximumClamp(blurred[1], 28.4691806922f);
+    const float ultra1 = psycho[(kHF + 1) * pitch + i];
+    const float uv1 = MaximumClamp(ultra1 - hv1, 5.19175294647f);
+    const float uhf1 = uv1 * 2.69313763794f;
+    const float hf1 = AmplifyRangeAroundZero(hv1 * 2.155f, 0.132f);
+    psycho[(kUHF + 0) * pitch + i] = uhf0;
+    psycho[(kHF + 0) * pitch + i] = hf0;
+    psycho[(kUHF + 1) * pitch + i] = uhf1;
+    psycho[(kHF + 1) * pitch + i] = hf1;
+    if (m.ref != nullptr) {
+      m.malta[2 * pitch + i] = MaltaScaledValue(m.scale[2], ref_hf1, hf1);
+      m.malta[3 * pitch + i] = MaltaScaledValue(m.scale[3], ref_hf0, hf0);
+      m.malta[4 * pitch + i] = MaltaScaledValue(m.scale[4], ref_uhf1, uhf1);
+      m.malta[5 * pitch + i] = MaltaScaledValue(m.scale[5], ref_uhf0, uhf0);
+    }
+    // Finiteness of the final HF and UHF planes; FrequencyLow and
+    // FrequencyHigh check the final LF and MF planes as they write them.
+    if (!(IsFinite(uhf0) && IsFinite(hf0) && IsFinite(uhf1) && IsFinite(hf1))) {
+      RaiseError(error, kErrorNonFiniteOutput);
+    }
   }
-  const float hv0 = blurred[i];
-  const float ultra0 = psycho[(kHF + 0) * pitch + i];
-  const float uhf0 = RemoveRangeAroundZero(ultra0 - hv0, 0.04f);
-  const float hf0 = RemoveRangeAroundZero(hv0, 1.5f);
-  const float hv1 = MaximumClamp(blurred[pitch + i], 28.4691806922f);
-  const float ultra1 = psycho[(kHF + 1) * pitch + i];
-  const float uv1 = MaximumClamp(ultra1 - hv1, 5.19175294647f);
-  const float uhf1 = uv1 * 2.69313763794f;
-  const float hf1 = AmplifyRangeAroundZero(hv1 * 2.155f, 0.132f);
-  psycho[(kUHF + 0) * pitch + i] = uhf0;
-  psycho[(kHF + 0) * pitch + i] = hf0;
-  psycho[(kUHF + 1) * pitch + i] = uhf1;
-  psycho[(kHF + 1) * pitch + i] = hf1;
-  if (m.ref != nullptr) {
-    m.malta[2 * pitch + i] = MaltaScaledValue(m.scale[2], ref_hf1, hf1);
-    m.malta[3 * pitch + i] = MaltaScaledValue(m.scale[3], ref_hf0, hf0);
-    m.malta[4 * pitch + i] = MaltaScaledValue(m.scale[4], ref_uhf1, uhf1);
-    m.malta[5 * pitch + i] = MaltaScaledValue(m.scale[5], ref_uhf0, uhf0);
-  }
-  // Finiteness of the final HF and UHF planes; FrequencyLowKernel and
-  // FrequencyHighKernel check the final LF and MF planes as they write them.
-  if (!(IsFinite(uhf0) && IsFinite(hf0) && IsFinite(uhf1) && IsFinite(hf1))) {
-    RaiseError(error, kErrorNonFiniteOutput);
+};
+
+// Column blur of Op::kPlanes planes and the frequency step that follows it, on
+// a tile of 32 columns x 32 rows: a warp blurs one plane's run of 8 rows (the
+// tile's 12 or 8 warps share the 32 + 2R rows they read through L1, where
+// runs in separate CTAs read each row (8 + 2R) / 8 times from L2), then all
+// threads take the tile's pixels. Bound: HBM (R = 16: 12 bytes read and 24
+// written per pixel beside the blurred planes, which no longer pass through
+// memory). A column blur and a kernel for the step took, per map of a
+// 2048x1536 image and its half scale, 46 us (R = 16), 36 us (R = 7) and 37 us
+// (R = 3); this takes 39, 32 and 36 us. The CTAs per SM hold the registers to
+// what keeps 24 (R = 16), 36 or 48 warps resident: left to itself the compiler
+// takes 150 for R = 16 (44 us), and 62 for R = 3 when told one CTA (41 us).
+constexpr int kTileColumns = 32, kTileRuns = 4, kTileRowsB = kTileRuns * kRun;
+
+template <int R, typename Op>
+__global__ void __launch_bounds__(32 * kTileRuns * Op::kPlanes, R > 8 ? 2 : R > 4 ? 3 : 6)
+BlurColumnsThenKernel(const float* in, int w, int h, size_t in_pitch,
+                      const __grid_constant__ Kernel17 k, const __grid_constant__ Op op) {
+  constexpr int P = Op::kPlanes;
+  __shared__ float blurred[P][kTileRowsB][kTileColumns];
+  const int tiles_x = (w + kTileColumns - 1) / kTileColumns;
+  const int x0 = (blockIdx.x % tiles_x) * kTileColumns, y0 = (blockIdx.x / tiles_x) * kTileRowsB;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int plane = warp % P, run = warp / P;
+  const int x = x0 + lane;
+  constexpr int kWarps = kTileRuns * P, kRows = (kTileRowsB + kWarps - 1) / kWarps;
+  const auto blur = [&]() {
+    if (x < w && y0 + run * kRun < h) {
+      const int y = y0 + run * kRun;
+      ConvolveRun<R>(in + plane * in_pitch + x, w, y, h, k, &blurred[plane][run * kRun][lane],
+                     kTileColumns, min(kRun, h - y));
+    }
+    __syncthreads();
+  };
+  const auto inside = [&](int row) { return row < kTileRowsB && x < w && y0 + row < h; };
+  const auto at = [&](int row) { return static_cast<size_t>(y0 + row) * w + x; };
+  float v[P];
+  if constexpr (Op::kPreload) {
+    // A warp takes every kWarps-th row of the tile, kRows at most.
+    typename Op::Loaded loaded[kRows];
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+      if (inside(warp + q * kWarps)) loaded[q] = op.Load(at(warp + q * kWarps));
+    }
+    blur();
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+      const int row = warp + q * kWarps;
+      if (!inside(row)) continue;
+#pragma unroll
+      for (int c = 0; c < P; ++c) v[c] = blurred[c][row][lane];
+      op(at(row), loaded[q], v);
+    }
+  } else {
+    blur();
+    for (int i = threadIdx.x; i < kTileRowsB * kTileColumns; i += 32 * kWarps) {
+      const int row = i / kTileColumns;
+      if (!inside(row)) continue;
+#pragma unroll
+      for (int c = 0; c < P; ++c) v[c] = blurred[c][row][lane];
+      op(at(row), v);
+    }
   }
 }
 
@@ -1235,7 +1342,6 @@ struct Scale {
   float* ref_mask = nullptr;     // FuzzyErosion(blur13(pre0))
   float* ref_blurred = nullptr;  // blur13(pre0)
   float* linear_tmp = nullptr;   // 3 planes: expanded/subsampled input
-  float* blur3 = nullptr;        // 3 planes
   float* xyb = nullptr;          // 3 planes
   float* tmp = nullptr;          // 3 planes (row-pass outputs)
   float* ac = nullptr;           // 3 planes
@@ -1251,8 +1357,10 @@ struct Scale {
   CUtensorMap malta_map[6];
 };
 
+// 47 planes, and one more so that the half scale's planes, which follow the
+// full scale's, start on a 16-byte boundary whatever the image's size.
 size_t ScaleFloats(size_t n) {
-  return n * (10 + 10 + 1 + 1 + 3 + 3 + 3 + 3 + 3 + 3 + 1 + 1 + 1 + 1 + 6);
+  return n * (10 + 10 + 1 + 1 + 3 + 3 + 3 + 3 + 3 + 1 + 1 + 1 + 1 + 6 + 1);
 }
 
 void AssignScale(Scale& s, float* base) {
@@ -1267,7 +1375,6 @@ void AssignScale(Scale& s, float* base) {
   s.ref_mask = take(1);
   s.ref_blurred = take(1);
   s.linear_tmp = take(3);
-  s.blur3 = take(3);
   s.xyb = take(3);
   s.tmp = take(3);
   s.ac = take(3);
@@ -1313,18 +1420,34 @@ struct ButteraugliState {
 
 namespace {
 
+// Row pass of a blur; one more CTA column takes the rows' ends.
+template <int R>
+void BlurRows(const float* in, float* out, int w, int h, size_t pitch, int planes,
+              const Kernel17& k, cudaStream_t stream) {
+  static_assert(kThreads / (2 * R) >= kBlurRows, "the end CTAs cover their rows");
+  const int row_groups = std::min((h + kBlurRows - 1) / kBlurRows, 65535);
+  BlurRowsKernel<R><<<dim3((w + kRowSegment - 1) / kRowSegment + 1, row_groups, planes), kThreads,
+                      0, stream>>>(in, out, w, h, pitch, pitch, k);
+}
+
 template <int R>
 void BlurPlanes(const float* in, float* tmp, float* out, int w, int h, size_t pitch, int planes,
                 const Kernel17& k, cudaStream_t stream) {
   const size_t column_runs = static_cast<size_t>(w) * ((h + kRun - 1) / kRun);
-  const int row_groups = std::min((h + kBlurRows - 1) / kBlurRows, 65535);
-  BlurRowsKernel<R><<<dim3((w + kRowSegment - 1) / kRowSegment, row_groups, planes), kThreads, 0,
-                      stream>>>(in, tmp, w, h, pitch, pitch, k);
-  constexpr int kBorderRows = kThreads / (2 * R);
-  BlurRowBordersKernel<R><<<dim3((h + kBorderRows - 1) / kBorderRows, planes), kThreads, 0,
-                            stream>>>(in, tmp, w, h, pitch, pitch, k);
+  BlurRows<R>(in, tmp, w, h, pitch, planes, k, stream);
   BlurColumnsKernel<R><<<dim3(Blocks(column_runs), planes), kThreads, 0, stream>>>(
     tmp, out, w, h, pitch, pitch, k);
+}
+
+// Row pass into `tmp`, then the column pass with the frequency step `op`.
+template <int R, typename Op>
+void BlurPlanesThen(const float* in, float* tmp, int w, int h, size_t pitch, const Kernel17& k,
+                    const Op& op, cudaStream_t stream) {
+  BlurRows<R>(in, tmp, w, h, pitch, Op::kPlanes, k, stream);
+  const size_t tiles = static_cast<size_t>((w + kTileColumns - 1) / kTileColumns) *
+                       ((h + kTileRowsB - 1) / kTileRowsB);
+  BlurColumnsThenKernel<R, Op><<<static_cast<unsigned>(tiles), 32 * kTileRuns * Op::kPlanes, 0,
+                                 stream>>>(tmp, w, h, pitch, k, op);
 }
 
 // Constants of the six Malta stages (MaltaDiffMap calls of
@@ -1384,18 +1507,14 @@ void Psycho(ButteraugliState& st, Scale& s, const float* linear, size_t stride, 
                         dim3(kB5W, kB5Rows), 0, stream>>>(dense, s.xyb, s.w, s.h, n,
                                                           st.k_opsin, st.intensity_target,
                                                           st.error);
-  // LF: 33-tap blur of the three XYB planes straight into the LF planes.
-  BlurPlanes<16>(s.xyb, s.tmp, psycho + kLF * n, s.w, s.h, n, 3, st.k_low, stream);
-  FrequencyLowKernel<<<Blocks(n), kThreads, 0, stream>>>(s.xyb, psycho, static_cast<int>(n), n,
-                                                         st.error);
-  // 15-tap blur of MF (3 planes) into blur3.
-  BlurPlanes<7>(psycho + kMF * n, s.tmp, s.blur3, s.w, s.h, n, 3, st.k_high, stream);
-  FrequencyHighKernel<<<Blocks(n), kThreads, 0, stream>>>(s.blur3, psycho, static_cast<int>(n), n,
-                                                          st.error, mp);
-  // 7-tap blur of HF (2 planes) into blur3.
-  BlurPlanes<3>(psycho + kHF * n, s.tmp, s.blur3, s.w, s.h, n, 2, st.k_ultra, stream);
-  FrequencyUltraKernel<<<Blocks(n), kThreads, 0, stream>>>(s.blur3, psycho, static_cast<int>(n),
-                                                           n, st.error, mp);
+  // LF: 33-tap blur of the three XYB planes; MF: 15-tap blur of what it
+  // leaves; HF: 7-tap blur of what that leaves of X and Y.
+  BlurPlanesThen<16>(s.xyb, s.tmp, s.w, s.h, n, st.k_low,
+                     FrequencyLow{s.xyb, psycho, n, st.error}, stream);
+  BlurPlanesThen<7>(psycho + kMF * n, s.tmp, s.w, s.h, n, st.k_high,
+                    FrequencyHigh{psycho, n, st.error, mp}, stream);
+  BlurPlanesThen<3>(psycho + kHF * n, s.tmp, s.w, s.h, n, st.k_ultra,
+                    FrequencyUltra{psycho, n, st.error, mp}, stream);
 }
 
 // Difference stages of one scale into s.final_map; with `reference_side`
