@@ -122,11 +122,12 @@ struct ReconParams {
 // K = 1024 / N transforms (3 channels each) per CTA of 384 threads; the
 // folded inverse DCT gives every thread 8 outputs of one line per pass
 // (line_dct.cuh). Coefficients sit at their natural (v, u) position of a
-// padded plane.
+// padded plane. Three CTAs per SM (56 registers, no spills) against two (72):
+// 32x32 53 against 65 us at 2048x1536, 226 against 283 us at 4032x3024.
 constexpr int kReconThreads = 384;
 
 template <int W, int H>
-__global__ void __launch_bounds__(kReconThreads, 2) ReconstructKernel(const __grid_constant__ ReconParams p) {
+__global__ void __launch_bounds__(kReconThreads, 3) ReconstructKernel(const __grid_constant__ ReconParams p) {
   constexpr int N = W * H, K = 1024 / N, KC = 3 * K;
   using Batch = PlaneBatch<W, H, KC>;
   static_assert(Batch::Items == kReconThreads, "one chunk per thread and pass");
