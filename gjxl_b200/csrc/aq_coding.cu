@@ -500,12 +500,22 @@ __device__ __forceinline__ int8_t QuantizeMultiplierF(float x) {
 // reference's element order (anchors in raster order, coefficients in
 // storage order); then lanes 0-3 (y_to_x) and 4-7 (y_to_b) of warp 0 run the
 // four ordered fused multiply-add chains per problem from shared memory.
-constexpr int kFinalCflThreads = 128;
+//
+// Bound: latency of the term loads and of the chains (1024 dependent
+// multiply-adds and their shared loads). Chains that read one term at a time
+// (two loads each, 128 threads preparing): 61 us at 2048x1536, 189 us at
+// 4032x3024; four at a time with 256 threads 43 and 130 us. 512 threads of 72
+// registers leave one CTA per SM and gain nothing.
+constexpr int kFinalCflThreads = 256;
 constexpr int kFinalCflTerms = 64 * 64;  // coefficients of one 64x64 tile
+// Terms of one kind lie by the reference's lane (e % 4), each lane's in its
+// order, so that a chain reads four at a time.
+constexpr int kFinalCflLane = kFinalCflTerms / 4 + 4;
+constexpr int kFinalCflPlane = 4 * kFinalCflLane + 8;  // the two problems' reads miss each other's banks
 
 __global__ void __launch_bounds__(kFinalCflThreads)
 FinalCflKernel(const __grid_constant__ CflFinalParams p) {
-  extern __shared__ __align__(16) float terms[];  // [a_x, b_x, a_b, b_b][kFinalCflTerms]
+  extern __shared__ __align__(16) float terms[];  // [a_x, b_x, a_b, b_b][kFinalCflPlane]
   __shared__ int block_terms[64], offsets[64], total_terms;
   __shared__ uint8_t group_block[64];  // anchor block of each 64-term group
   // Per anchor block: covered width and height, inverse-dequant table
@@ -610,10 +620,11 @@ FinalCflKernel(const __grid_constant__ CflFinalParams p) {
       const float chroma_x = x_v[j] * inv_x[j] * quant_scale;
       const float luma_b = luma_v[j] * inv_b[j] * quant_scale;
       const float chroma_b = b_v[j] * inv_b[j] * quant_scale;
-      terms[e] = luma_x / 84.0f;
-      terms[kFinalCflTerms + e] = base_x * luma_x - chroma_x;
-      terms[2 * kFinalCflTerms + e] = luma_b / 84.0f;
-      terms[3 * kFinalCflTerms + e] = base_b * luma_b - chroma_b;
+      float* out = terms + (e & 3) * kFinalCflLane + (e >> 2);
+      out[0] = luma_x / 84.0f;
+      out[kFinalCflPlane] = base_x * luma_x - chroma_x;
+      out[2 * kFinalCflPlane] = luma_b / 84.0f;
+      out[3 * kFinalCflPlane] = base_b * luma_b - chroma_b;
     }
   }
   __syncthreads();
@@ -621,32 +632,37 @@ FinalCflKernel(const __grid_constant__ CflFinalParams p) {
   const int problem = lane / 4, slot = lane % 4;  // problem 0: X, 1: B
   float quadratic = 0.0f, linear = 0.0f;
   if (problem < 2) {
-    const float* A = terms + 2 * problem * kFinalCflTerms;
-    const float* B = A + kFinalCflTerms;
+    const float4* A = reinterpret_cast<const float4*>(terms + 2 * problem * kFinalCflPlane +
+                                                      slot * kFinalCflLane);
+    const float4* B = A + kFinalCflPlane / 4;
     // count is a multiple of 64: batches of 8 elements per lane; the next
     // batch is loaded while the current one goes through the ordered
     // multiply-adds.
-    float a[8], b[8];
+    const int batches = count / 32;
+    float4 a[2], b[2];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      a[j] = count > 0 ? A[slot + 4 * j] : 0.0f;
-      b[j] = count > 0 ? B[slot + 4 * j] : 0.0f;
+    for (int j = 0; j < 2; ++j) {
+      a[j] = batches > 0 ? A[j] : make_float4(0, 0, 0, 0);
+      b[j] = batches > 0 ? B[j] : make_float4(0, 0, 0, 0);
     }
-    for (int e0 = slot; e0 < count; e0 += 32) {
-      float na[8], nb[8];
-      const int next = e0 + 32 < count ? e0 + 32 : slot;
+    for (int n = 0; n < batches; ++n) {
+      float4 na[2], nb[2];
+      const int next = n + 1 < batches ? 2 * n + 2 : 0;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        na[j] = A[next + 4 * j];
-        nb[j] = B[next + 4 * j];
+      for (int j = 0; j < 2; ++j) {
+        na[j] = A[next + j];
+        nb[j] = B[next + j];
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        quadratic = fmaf(a[j], a[j], quadratic);
-        linear = fmaf(a[j], b[j], linear);
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < 2; ++j) {
+        quadratic = fmaf(a[j].x, a[j].x, quadratic);
+        linear = fmaf(a[j].x, b[j].x, linear);
+        quadratic = fmaf(a[j].y, a[j].y, quadratic);
+        linear = fmaf(a[j].y, b[j].y, linear);
+        quadratic = fmaf(a[j].z, a[j].z, quadratic);
+        linear = fmaf(a[j].z, b[j].z, linear);
+        quadratic = fmaf(a[j].w, a[j].w, quadratic);
+        linear = fmaf(a[j].w, b[j].w, linear);
         a[j] = na[j];
         b[j] = nb[j];
       }
@@ -1848,7 +1864,7 @@ int AqFinalCfl(const uint8_t* cells, size_t bx, size_t by, const float* coef, si
   }
   p.y_to_x = y_to_x;
   p.y_to_b = y_to_b;
-  const size_t smem = 4 * kFinalCflTerms * sizeof(float);
+  const size_t smem = 4 * kFinalCflPlane * sizeof(float);
   status = CheckCuda(cudaFuncSetAttribute(FinalCflKernel,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           static_cast<int>(smem)),
