@@ -480,26 +480,42 @@ __global__ void OpsinToLinearKernel(const __grid_constant__ LinearParams p) {
   OpsinToLinearPixel(p, p.opsin[i], p.opsin[p.n + i], p.opsin[2 * p.n + i], i);
 }
 
-// Eight lanes per block: a row segment of eight pixels is loaded and raised to
-// the 16th power by the lanes together and added in raster order through
-// shuffles, four segments' loads in flight; the 32 roots of a CTA are then
-// taken by one warp. Bound: latency (a 32x32 transform is 1024 dependent
-// adds). One thread per block with its pixels' loads one row apart took 43 us
-// at 256x256 and 62 us at 2048x1536.
+// Eight lanes per transform: a row segment of eight pixels is loaded and
+// raised to the 16th power by the lanes together and added in raster order
+// through shuffles, the next eight segments' loads in flight; the roots of a
+// CTA's anchors are then taken by one warp. Bound: latency at small sizes (a
+// 32x32 transform is 1024 dependent adds), the shuffles at large ones, so that
+// the CTA's anchors are gathered first: a warp with one anchor among its four
+// groups issues as much as one with four. One evaluation at 256x256 /
+// 2048x1536 / 4032x3024: one thread per block 43 / 62 / - us; eight lanes per
+// block, anchor or not, with four loads at a time 26 / 46 / 107; this 15 / 25
+// / 61.
 constexpr int kReduceBlocks = 32;  // blocks per CTA
 constexpr int kReduceLanes = 8;
+constexpr int kReduceAhead = 8;    // segments per load
 
 __global__ void __launch_bounds__(kReduceBlocks * kReduceLanes)
 BlockReduceKernel(const uint8_t* cells, int blocks_x, int blocks_y, const float* map, int w,
                   int h, float* out) {
   __shared__ float means[kReduceBlocks];
-  __shared__ int families[kReduceBlocks];  // -1: no anchor
+  // The CTA's anchors, so that a warp's four groups of lanes all hold one.
+  __shared__ int anchors[kReduceBlocks], families[kReduceBlocks], anchor_count;
+  if (threadIdx.x < kReduceBlocks) {
+    const int block = blockIdx.x * kReduceBlocks + threadIdx.x;
+    const uint8_t cell = block < blocks_x * blocks_y ? cells[block] : 0;
+    const int family = cell & 1 ? StrategyFamily(cell >> 1) : -1;
+    const unsigned held = __ballot_sync(0xffffffffu, family >= 0);
+    if (family >= 0) {
+      const int rank = __popc(held & ((1u << threadIdx.x) - 1u));
+      anchors[rank] = block;
+      families[rank] = family;
+    }
+    if (threadIdx.x == 0) anchor_count = __popc(held);
+  }
+  __syncthreads();
   const int slot = threadIdx.x / kReduceLanes, lane = threadIdx.x % kReduceLanes;
-  const int i = blockIdx.x * kReduceBlocks + slot;
-  int f = -1;
-  if (i < blocks_x * blocks_y && (cells[i] & 1)) f = StrategyFamily(cells[i] >> 1);
-  if (lane == 0) families[slot] = f;
-  if (f >= 0) {
+  if (slot < anchor_count) {
+    const int i = anchors[slot], f = families[slot];
     const unsigned group = 0xFFu << (threadIdx.x % 32 - lane);
     const int x0 = i % blocks_x * 8, y0 = i / blocks_x * 8;
     const int columns = FamilyCoveredW(f);
@@ -507,38 +523,45 @@ BlockReduceKernel(const uint8_t* cells, int blocks_x, int blocks_y, const float*
     // Segments in raster order: segment s is columns 8 (s % columns) .. + 7
     // of row s / columns. Pixels past the image's right edge count as zeros,
     // which leave the sum as it is.
+    const int shift = columns == 4 ? 2 : columns - 1, mask = columns - 1;
     const int segments = (y1 - y0) * columns;
-    float norm = 0.0f;
-    for (int s0 = 0; s0 < segments; s0 += 4) {
-      float v[4];
+    const auto load = [&](int s0, float (&v)[kReduceAhead]) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int x = x0 + (s0 + k) % columns * 8 + lane, y = y0 + (s0 + k) / columns;
+      for (int k = 0; k < kReduceAhead; ++k) {
+        const int x = x0 + ((s0 + k) & mask) * 8 + lane, y = y0 + ((s0 + k) >> shift);
         v[k] = y < y1 && x < x1 ? map[static_cast<size_t>(y) * w + x] : 0.0f;
       }
+    };
+    float norm = 0.0f;
+    float v[kReduceAhead], next[kReduceAhead];
+    load(0, v);
+    for (int s0 = 0; s0 < segments; s0 += kReduceAhead) {
+      load(s0 + kReduceAhead, next);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < kReduceAhead; ++k) {
         v[k] *= v[k];
         v[k] *= v[k];
         v[k] *= v[k];
         v[k] *= v[k];
       }
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < kReduceAhead; ++k) {
 #pragma unroll
         for (int j = 0; j < kReduceLanes; ++j) {
           norm += __shfl_sync(group, v[k], j, kReduceLanes);
         }
       }
+#pragma unroll
+      for (int k = 0; k < kReduceAhead; ++k) v[k] = next[k];
     }
     if (lane == 0) means[slot] = norm / static_cast<float>((x1 - x0) * (y1 - y0));
   }
   __syncthreads();
-  if (threadIdx.x >= kReduceBlocks || families[threadIdx.x] < 0) return;
+  if (threadIdx.x >= anchor_count) return;
   // std::pow(float, 1/16): evaluated in double and rounded to float.
   const float d =
     1.2f * static_cast<float>(pow(static_cast<double>(means[threadIdx.x]), 0.0625));
-  const int block = blockIdx.x * kReduceBlocks + threadIdx.x;
+  const int block = anchors[threadIdx.x];
   const int cw = FamilyCoveredW(families[threadIdx.x]), ch = FamilyCoveredH(families[threadIdx.x]);
   for (int dy = 0; dy < ch; ++dy)
     for (int dx = 0; dx < cw; ++dx) out[block + dy * blocks_x + dx] = d;
