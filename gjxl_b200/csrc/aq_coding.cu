@@ -818,12 +818,12 @@ __device__ void AdjustFinish(int channel, int strategy, const AdjustSums& sums,
     ++*raw_quant;
     if (*raw_quant >= 256) *raw_quant = 255;
   }
-  const double kFirst[4][3] = {
+  constexpr double kFirst[4][3] = {
     {0.22080615753848404, 0.45797479824262011, 0.29859235095977965},
     {0.70109486510286834, 0.16185281305512639, 0.14387691730035473},
     {0.114985964456218638, 0.44656840441027695, 0.10587658215149048},
     {0.46849665264409396, 0.41239077937781954, 0.088667407767185444}};
-  const double kSecond[4][3] = {
+  constexpr double kSecond[4][3] = {
     {0.27450281941822197, 1.1255766549984996, 0.98950459134128388},
     {0.4652168675598285, 0.40945807983455818, 0.36581899811751367},
     {0.28034972424715715, 0.9182653201929738, 1.5581531543057416},
@@ -832,17 +832,17 @@ __device__ void AdjustFinish(int channel, int strategy, const AdjustSums& sums,
   error_sum = static_cast<float>(static_cast<double>(error_sum) * kQuantNormalizer);
   value_sum = static_cast<float>(static_cast<double>(value_sum) * kQuantNormalizer);
   if (strategy >= kStrategyDct16x16) {
-    int cls = 3;
-    if (strategy == kStrategyDct32x16 || strategy == kStrategyDct16x32) {
-      cls = 1;
-    } else if (strategy == kStrategyDct16x16) {
-      cls = 0;
-    } else if (strategy == kStrategyDct32x32) {
-      cls = 2;
-    }
+    constexpr int cls = W == 16 && H == 16 ? 0 : W == 32 && H == 32 ? 2 : W * H == 512 ? 1 : 3;
+    // (Selected by channel: an index would put the tables on the stack.)
+    const double first = channel == 0   ? kFirst[cls][0]
+                         : channel == 1 ? kFirst[cls][1]
+                                        : kFirst[cls][2];
+    const double second = channel == 0   ? kSecond[cls][0]
+                          : channel == 1 ? kSecond[cls][1]
+                                         : kSecond[cls][2];
     const double threshold =
-      kFirst[cls][channel] * static_cast<double>(xsize) * static_cast<double>(ysize) * 8.0 * 8.0 +
-      kSecond[cls][channel] * static_cast<double>(value_sum);
+      first * static_cast<double>(xsize) * static_cast<double>(ysize) * 8.0 * 8.0 +
+      second * static_cast<double>(value_sum);
     int step = static_cast<int>(static_cast<double>(error_sum) / threshold);
     step = min(max(step, 0), 2);
     if (static_cast<double>(error_sum) > threshold) {
@@ -949,15 +949,26 @@ __device__ __forceinline__ float CodingOrderedSum(const float* t) {
 }
 
 // ComputeQuantizedCoefficientsImpl's per-transform body
-// (reconstruction.cpp:480-700), one CTA of 64 threads per anchor.
-// Threads per anchor.
+// (reconstruction.cpp:480-700), one CTA per anchor.
+//
+// Bound: latency (its loads, the ordered error sums of up to 1024 dependent
+// adds, the few double operations of the decisions), so that what counts is
+// how many CTAs an SM holds and how short the stretches between are. Threads
+// per anchor: about four coefficients of each channel a thread from 16x16 on
+// (32x32 one evaluation, 64 against 256 threads: 22 against 17 us at 256x256,
+// 66 against 59 at 2048x1536, the same at 4032x3024); 256 threads for the 512
+// coefficients of 32x16 cost 24 against 17 us at 4032x3024, where most CTAs
+// find no anchor. Sums per quadrant and the decisions' tables are selected,
+// not indexed, which would put them in local memory (32x32 / 8x8 at
+// 4032x3024: 271 / 161 against 248 / 152 us).
 template <int W, int H>
 __host__ __device__ constexpr int CodingThreads() {
-  return 64;
+  return W * H >= 1024 ? 256 : W * H >= 256 ? 128 : 64;
 }
 
 template <int W, int H>
-__global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __grid_constant__ CodingParams p) {
+__global__ void __launch_bounds__(CodingThreads<W, H>(), W * H >= 1024 ? 4 : W * H >= 512 ? 8 : 1)
+CodingKernel(const __grid_constant__ CodingParams p) {
   using S = TransformShape<W, H>;
   constexpr int N = S::N;
   constexpr int strategy = W == 8 && H == 8     ? kStrategyDct8
@@ -968,7 +979,8 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
                          : W == 16              ? kStrategyDct32x16
                                                 : kStrategyDct16x32;
   constexpr int covered = S::CW * S::CH;
-  constexpr int kT = CodingThreads<W, H>();
+  constexpr int kT = CodingThreads<W, H>(), kWarps = kT / 32;
+  static_assert(kWarps >= 2, "two roles");
   __shared__ float coef[3][N];
   // The family's inverse-dequant weights, staged so that the serial
   // threshold passes below read shared memory instead of waiting on L2.
@@ -981,11 +993,10 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
   constexpr int kBorder = 3 * (S::SH / 8) + (S::SH / 8 - 1) * (S::SW / 8) + 4 * (S::SW / 8);
   __shared__ __align__(16) float adjust_err[3][N];
   __shared__ float border[3][kBorder];
-  __shared__ uint32_t adjust_sum[2][3][5];  // per warp and channel: sum |q|, per quadrant
-  __shared__ uint32_t adjust_max[2][4];     // per warp: Y max error per quadrant (float bits)
-  __shared__ int adjust_big[2];             // per warp: a |q| sum reached 2^24
+  __shared__ uint32_t adjust_sum[kWarps][3][5];  // per warp and channel: sum |q|, per quadrant
+  __shared__ uint32_t adjust_max[kWarps][4];     // per warp: Y max error per quadrant (float bits)
+  __shared__ int adjust_big[kWarps];             // per warp: a |q| sum reached 2^24
   __shared__ float dequant_y[N];            // the family's Y dequant weights
-  static_assert(kT == 64, "two warps");
   const uint32_t anchor_index = blockIdx.x;
   // The grid is the anchor list's capacity, so the anchor load is in bounds;
   // it is issued beside the count load instead of after it.
@@ -1038,23 +1049,27 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
         }
         const int quadrant = (y >= Sh::SH / 2) * 2 + (x >= Sh::SW / 2);
         const float value = coef[c][index] * (inverse_dequant[c][index] * qac * mm);
-        const float quantized = fabsf(value) < t0[quadrant] ? 0.0f : rintf(value);
+        const float quantized =
+          fabsf(value) < (quadrant == 0 ? t0[0] : t0[1]) ? 0.0f : rintf(value);
         const float err = fabsf(value - quantized);
         adjust_err[c][index] = err;
         const float magnitude = fabsf(quantized);
         if (magnitude < 16777216.0f) {
           const uint32_t m = static_cast<uint32_t>(magnitude);
-          sums[c][0] += m;
-          sums[c][1 + quadrant] += m;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) sums[c][1 + k] += quadrant == k ? m : 0u;
         } else {
           big = true;
         }
         if (c == 1 && quantized == 0.0f) {
           // Non-negative floats order like their bit patterns; NaN errors are
           // skipped, as fmaxf skips them.
-          if (err == err) max_bits[quadrant] = max(max_bits[quadrant], __float_as_uint(err));
+          const uint32_t bits = err == err ? __float_as_uint(err) : 0u;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) max_bits[k] = max(max_bits[k], quadrant == k ? bits : 0u);
         }
       }
+      sums[c][0] = (sums[c][1] + sums[c][2]) + (sums[c][3] + sums[c][4]);
       if (sums[c][0] >= (1u << 24)) big = true;
     }
     for (int i = tid; i < 3 * kBorder; i += kT) {
@@ -1072,7 +1087,8 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
       const int quadrant = (y >= Sh::SH / 2) * 2 + (x >= Sh::SW / 2);
       const float mm = c == 0 ? mm0 : c == 1 ? mm1 : mm2;
       const float value = coef[c][index] * (inverse_dequant[c][index] * qac * mm);
-      const float quantized = fabsf(value) < t0[quadrant] ? 0.0f : rintf(value);
+      const float quantized =
+        fabsf(value) < (quadrant == 0 ? t0[0] : t0[1]) ? 0.0f : rintf(value);
       border[c][j] = quantized != 0.0f ? fabsf(value) : 0.0f;
     }
     const int warp = tid / 32, lane = tid % 32;
@@ -1098,8 +1114,16 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
     float t[4] = {t0[0], t0[1], t0[2], t0[3]};
     int candidate = initial_raw;
     AdjustSums sums;
-    const uint32_t total = adjust_sum[0][c][0] + adjust_sum[1][c][0];
-    if (adjust_big[0] | adjust_big[1] || total >= (1u << 24)) {
+    uint32_t totals[5] = {0, 0, 0, 0, 0};
+    int any_big = 0;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) {
+      any_big |= adjust_big[i];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) totals[k] += adjust_sum[i][c][k];
+    }
+    const uint32_t total = totals[0];
+    if (any_big || total >= (1u << 24)) {
       AdjustSumsSerial<W, H>(qac, c, c == 0 ? mm0 : c == 1 ? mm1 : mm2, coef[c],
                              inverse_dequant[c], t, &sums);
     } else {
@@ -1113,9 +1137,11 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
       sums.border_sum = border_sum;
       sums.value_sum = static_cast<float>(total);
       for (int k = 0; k < 4; ++k) {
-        sums.nonzeros[k] = static_cast<float>(adjust_sum[0][c][1 + k] + adjust_sum[1][c][1 + k]);
-        sums.max_error[k] =
-          c == 1 ? __uint_as_float(max(adjust_max[0][k], adjust_max[1][k])) : 0.0f;
+        sums.nonzeros[k] = static_cast<float>(totals[1 + k]);
+        uint32_t most = 0;
+#pragma unroll
+        for (int i = 0; i < kWarps; ++i) most = max(most, adjust_max[i][k]);
+        sums.max_error[k] = c == 1 ? __uint_as_float(most) : 0.0f;
       }
     }
     AdjustFinish<W, H>(c, strategy, sums, t, &candidate);
@@ -1152,7 +1178,7 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
     coef[2][j] -= f2 * coef[1][j];
   }
   __syncthreads();
-  if (tid % 32 < covered) {
+  if (tid < 64 && tid % 32 < covered) {
     const int c = tid < 32 ? 0 : 2, dy = tid % 32 / S::CW, dx = tid % 32 % S::CW;
     p.dc[c * p.dc_pitch + static_cast<size_t>(a.y + dy) * p.blocks_x + a.x + dx] =
       LowFrequencyDc<W, H>(coef[c], dy, dx);
@@ -1165,7 +1191,8 @@ __global__ void __launch_bounds__(CodingThreads<W, H>()) CodingKernel(const __gr
     const int ti = (y >= S::SH / 2) * 2 + (x >= S::SW / 2);
     const float qs = q.scale * static_cast<float>(raw) * (c == 0 ? mm0 : mm2);
     const float value = inverse_dequant[c][j] * qs * coef[c][j];
-    const int32_t quantized = fabsf(value) < t[ti] ? 0 : static_cast<int32_t>(rintf(value));
+    const int32_t quantized =
+      fabsf(value) < (ti == 0 ? t[0] : t[1]) ? 0 : static_cast<int32_t>(rintf(value));
     p.qac[c * p.pitch + static_cast<size_t>(a.y * 8 + j / W) * p.stride + a.x * 8 + j % W] =
       quantized;
   }
