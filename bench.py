@@ -170,7 +170,8 @@ def candidate_cost_fp64_ops(blocks_x: int, blocks_y: int) -> int:
     image: every candidate transforms 3 channels forward and back, each
     separable DCT costs (W + H) multiply-adds per coefficient, and the
     bit-exact restatement rounds every multiply and every add separately
-    (2 FP64 operations per multiply-add)."""
+    (2 FP64 operations per multiply-add). This counts the sequential sums: the
+    kernels' folded inverse passes execute a quarter of theirs."""
     total = 0
     for w, h, cw, ch, step in FAMILIES:
         anchors = 0
@@ -362,7 +363,8 @@ def run_gpu(args) -> dict:
             "bound": "fp64",
             "achieved": round(achieved, 3),
             "peak": round(peak, 3),
-            "unit": "TFLOP/s (FP64, multiply and add rounded and counted separately)",
+            "unit": ("TFLOP/s (FP64 multiplies and adds of the sequential sums; the folded "
+                     "inverse passes execute a quarter of theirs)"),
             "frac": round(achieved / peak, 4),
             "traffic": COST_KERNEL_DRAM_BYTES,
             "algorithmic_ops": fp64_ops,
