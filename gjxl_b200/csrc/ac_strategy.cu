@@ -385,6 +385,12 @@ CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_cou
   constexpr bool kExact = sizeof(Acc) == 8;
   constexpr int N = S::N, K = Lay::K, KC = Lay::KC;
   constexpr int kPerThread = Lay::kPerThread;
+  // Of the element stages. Unrolled eight times their code and the transforms'
+  // outgrew the instruction cache (ncu: 2.8 cycles of "no instruction" per issue
+  // for 16x16); twice for 16x16 1303 -> 1216 us at 4032x3024, four times for
+  // 16x32 941 -> 915 and 8x16 611 -> 597. 8x8 is best unrolled (295 against 299),
+  // and a 32x32 thread's eight positions hold their weights in registers.
+  constexpr int kUnroll = N == 256 ? 2 : N == 128 || N == 512 ? 4 : kPerThread;
   static_assert(K == S::K, "candidates per CTA");
   static_assert(kExact || (W <= 16 && H <= 16), "FP32 passes cover lengths 8 and 16");
   extern __shared__ __align__(16) unsigned char smem[];
@@ -548,7 +554,7 @@ CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_cou
       inv[i] = __ldg(p.inverse_dequant + c * N + j);
       dq[i] = __ldg(p.dequant + c * N + j);
     }
-#pragma unroll
+#pragma unroll kUnroll
     for (int q = 0; q < kPerThread; ++q) {
       const int k = Lay::Candidate(t, q), j = Lay::Position(t, q);
       constexpr int kPositions = Lay::kPositions;
@@ -611,7 +617,7 @@ CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_cou
   float* loss_terms = kExact ? reinterpret_cast<float*>(T) : terms;
   static_assert(!kExact || 2 * Lay::Planes >= KC * Lay::TermPitch, "loss terms fit T");
   const float offset = c == 0 ? 12.0f : c == 1 ? 0.0f : 4.0f;
-#pragma unroll
+#pragma unroll kUnroll
   for (int q = 0; q < kPerThread; ++q) {
     const int k = Lay::Candidate(t, q), r = Lay::Position(t, q), y = r / W, x = r % W;
     if (anchor_x[k] < 0) continue;
