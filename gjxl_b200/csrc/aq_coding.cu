@@ -380,11 +380,17 @@ constexpr int kSelectShare = 50 * 1024;    // field values per CTA (200 KB)
 constexpr int kSelectSmallShare = 4096;    // values per CTA below the largest cluster
 static_assert(2 * kSelectThreads == kSelectBins, "two bins per thread");
 
+// Read two bins at a time.
+struct __align__(8) SelectHistogram {
+  uint32_t bins[kSelectBins];
+};
+static_assert(alignof(SelectHistogram) >= alignof(uint2), "two bins per load");
+
 __global__ void __launch_bounds__(kSelectThreads)
 ClusterQuantizerKernel(const float* field, int n, int share, const AqPolicy* policy,
                        AqQuantizer* q, int32_t* raw, uint32_t* error) {
   extern __shared__ float values[];
-  __shared__ uint32_t histogram[2][kSelectBins];
+  __shared__ SelectHistogram histogram[2];
   __shared__ uint32_t warp_sums[32], chosen_digit, chosen_before;
   const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int ctas = static_cast<int>(cluster.num_blocks());
@@ -392,7 +398,9 @@ ClusterQuantizerKernel(const float* field, int n, int share, const AqPolicy* pol
   const int begin = static_cast<int>(cluster.block_rank()) * share;
   const int count = max(0, min(share, n - begin));
   for (int i = t; i < count; i += kSelectThreads) values[i] = field[begin + i];
-  for (int b = t; b < 2 * kSelectBins; b += kSelectThreads) (&histogram[0][0])[b] = 0;
+  for (int b = t; b < 2 * kSelectBins; b += kSelectThreads) {
+    histogram[b / kSelectBins].bins[b % kSelectBins] = 0;
+  }
   __syncthreads();
   uint32_t selected[2];  // median, then median absolute deviation
   int buffer = 0;
@@ -405,17 +413,19 @@ ClusterQuantizerKernel(const float* field, int n, int share, const AqPolicy* pol
       const uint32_t digit_mask = (1u << SelectBits(pass)) - 1u;
       for (int i = t; i < count; i += kSelectThreads) {
         const uint32_t bits = SelectKey(values, i, selection == 1, center);
-        if ((bits & mask) == prefix) atomicAdd(&histogram[buffer][(bits >> shift) & digit_mask], 1u);
+        if ((bits & mask) == prefix) {
+          atomicAdd(&histogram[buffer].bins[(bits >> shift) & digit_mask], 1u);
+        }
       }
       cluster.sync();
       uint32_t h0 = 0, h1 = 0;
       for (int r = 0; r < ctas; ++r) {
         const uint2 h =
-          reinterpret_cast<const uint2*>(cluster.map_shared_rank(&histogram[buffer][0], r))[t];
+          reinterpret_cast<const uint2*>(cluster.map_shared_rank(histogram[buffer].bins, r))[t];
         h0 += h.x;
         h1 += h.y;
       }
-      reinterpret_cast<uint2*>(&histogram[buffer ^ 1][0])[t] = make_uint2(0, 0);
+      reinterpret_cast<uint2*>(histogram[buffer ^ 1].bins)[t] = make_uint2(0, 0);
       uint32_t inclusive = h0 + h1;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
