@@ -1029,32 +1029,44 @@ DeviceLimits Limits() {
   return l;
 }
 
+const DeviceLimits& CachedLimits() {
+  static const DeviceLimits limits = Limits();
+  return limits;
+}
+
+// Reverse maps that fit in `bytes` of shared memory beside the ANS kernel's
+// static arrays.
+int MapsWithin(int bytes) {
+  constexpr int kStatic = kAnsPairs * static_cast<int>(sizeof(AnsStage)) + 2 * 256 * 4 + 256 +
+                          static_cast<int>(kAnsContexts) +
+                          kMaxHotClusters + 64;
+  return std::max(0, std::min((bytes - kStatic) / static_cast<int>(kAnsTable * 2),
+                              static_cast<int>(kMaxHotClusters)));
+}
+
 // Reverse maps staged per CTA: as many as fit in the shared memory one CTA
 // may take while all sections still run in one wave (up to four CTAs per
 // SM), at most the code's clusters. Maps must be 16-byte aligned.
 uint32_t HotClusters(const EmitParams& p) {
   if (reinterpret_cast<uintptr_t>(p.code.reverse_map) % 16 != 0) return 0;
-  static const DeviceLimits limits = Limits();
+  const DeviceLimits& limits = CachedLimits();
   if (limits.sms <= 0 || limits.smem_per_sm <= 0) return 0;
   const int ctas = static_cast<int>((p.tokens.count + kAnsPairs - 1) / kAnsPairs);
   const int per_sm = std::min(4, std::max(1, (ctas + limits.sms - 1) / limits.sms));
-  constexpr int kStatic = kAnsPairs * static_cast<int>(sizeof(AnsStage)) + 2 * 256 * 4 + 256 +
-                          static_cast<int>(kAnsContexts) +
-                          kMaxHotClusters + 64;
-  const int budget = std::min(limits.smem_per_block, limits.smem_per_sm / per_sm - 1024) -
-                     kStatic;
-  const int maps = budget / static_cast<int>(kAnsTable * 2);
-  return static_cast<uint32_t>(std::max(0, std::min<int>(
-    {maps, static_cast<int>(kMaxHotClusters), static_cast<int>(p.code.cluster_count)})));
+  const int maps = MapsWithin(std::min(limits.smem_per_block, limits.smem_per_sm / per_sm - 1024));
+  return std::min(static_cast<uint32_t>(maps), p.code.cluster_count);
 }
 
+// Both writers raise their kernel's shared-memory limit to the most that any
+// call asks for, not to this call's need: the limit belongs to the kernel, and
+// calls from several host threads share it.
 template <bool kCount>
 void LaunchAns(EmitParams p, cudaStream_t stream) {
   p.hot_clusters = HotClusters(p);
-  const int bytes = static_cast<int>(p.hot_clusters * kAnsTable * 2);
-  if (bytes > 0 &&
+  const int most = MapsWithin(CachedLimits().smem_per_block) * static_cast<int>(kAnsTable * 2);
+  if (p.hot_clusters > 0 &&
       cudaFuncSetAttribute(AnsSectionKernel<kCount>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           bytes) != cudaSuccess) {
+                           most) != cudaSuccess) {
     cudaGetLastError();
     p.hot_clusters = 0;
   }
@@ -1073,7 +1085,7 @@ void LaunchSections(const EmitParams& p, cudaStream_t stream) {
     bool staged = bytes <= kPrefixStagedBytes;
     if (staged && cudaFuncSetAttribute(PrefixSectionKernel<kCount>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(bytes)) != cudaSuccess) {
+                                       static_cast<int>(kPrefixStagedBytes)) != cudaSuccess) {
       cudaGetLastError();
       staged = false;
     }

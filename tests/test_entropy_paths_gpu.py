@@ -3,11 +3,15 @@ where their paths change: ANS batches of 128 tokens, reverse maps in shared
 memory or in the code's own memory, maps that are no ANS code;
 prefix chunks of 2048 tokens and codes too large for shared memory."""
 
+import ctypes
+import threading
+
 import numpy as np
 import pytest
 import torch
 
-from gjxl_b200.entropy import ANS, PREFIX, EntropyCode, write_sections
+from gjxl_b200 import _lib
+from gjxl_b200.entropy import ANS, PREFIX, EntropyCode, _sections, write_sections
 from tests.gpu_util import host
 
 pytestmark = pytest.mark.gpu
@@ -150,3 +154,48 @@ def test_prefix_sections(cuda, clusters):
     offsets = np.concatenate([[0], np.cumsum([0, 1, 2047, 2048, 2049, 4100, 7])])
     values, ctx = make_tokens(50 + clusters, int(offsets[-1]), 300)
     check(make_tables(PREFIX, 60 + clusters, 300, clusters), values, ctx, offsets)
+
+
+@pytest.mark.parametrize("mode", [ANS, PREFIX])
+def test_threads_with_codes_of_different_sizes(cuda, mode):
+    """Two host threads, each with its own stream and code: neither call's
+    shared-memory size may limit the other's launch."""
+    work = []
+    for clusters in (3, 150 if mode == PREFIX else 25):
+        offsets = torch.tensor([0, 300, 1000], dtype=torch.int32).cuda()
+        values, ctx = make_tokens(70 + clusters, 1000, 300)
+        work.append((EntropyCode(make_tables(mode, 80 + clusters, 300, clusters)), offsets,
+                     torch.from_numpy(values.view(np.int32)).cuda(),
+                     torch.from_numpy(ctx.view(np.int16)).cuda()))
+    want = [write_sections(code, o, values=v, contexts=c, tokens=1000)["packed"]
+            for code, o, v, c in work]
+    torch.cuda.synchronize()
+    start, failed = threading.Barrier(2), []
+
+    def run(k: int) -> None:
+        code, o, v, c = work[k]
+        stream = torch.cuda.Stream()
+        try:
+            with torch.cuda.stream(stream):
+                # Most of the time inside the library, where threads run at once.
+                struct, sections = code.struct(), _sections(o, v, c)
+                bits = torch.zeros(2, dtype=torch.int64, device="cuda")
+                error = torch.zeros(1, dtype=torch.int32, device="cuda")
+                count = _lib.load().gjxl_b200_entropy_count_sections
+                call = (ctypes.addressof(struct), 1, ctypes.addressof(sections), bits.data_ptr(),
+                        error.data_ptr(), stream.cuda_stream)
+                start.wait()
+                for _ in range(20000):
+                    assert count(*call) == 0, "launch failed"
+                got = write_sections(code, o, values=v, contexts=c, tokens=1000)
+                assert torch.equal(got["packed"], want[k])
+                assert torch.equal(got["bit_counts"], bits) and int(error) == 0
+        except Exception as exception:
+            failed.append(exception)
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed[0]
