@@ -21,6 +21,9 @@
 // loads per sample, or else from constant memory.
 #pragma once
 
+#include <cstdint>
+#include <cstring>
+
 #include "dct_basis.inc"
 
 namespace gjxl_b200 {
@@ -327,7 +330,8 @@ namespace gjxl_b200 {
 // differ by at most E = FoldBound<W, H>() * S (both lines' bounds times the
 // other pass's sqrt(2)). The float is the same unless a rounding boundary (a
 // tie between neighbouring floats) lies within E of the folded result; a
-// column with such an output is transformed again by the sequential sums. For
+// column with an output for which FoldedSettled cannot rule that out is
+// transformed again by the sequential sums. For
 // the residuals of ordinary images E is about 2^9 (8x8) to 2^13 (32x32) units
 // in the last place of the double, against 2^28 from a float to the tie: less
 // than one plane in 1000 (8x8) and one in five (32x32) has such a column.
@@ -401,28 +405,56 @@ __device__ __forceinline__ void FoldedRow(const float* __restrict__ in, double* 
   }
 }
 
+__host__ __device__ __forceinline__ int HighWord(double v) {
+#ifdef __CUDA_ARCH__
+  return __double2hiint(v);
+#else
+  uint64_t bits;
+  memcpy(&bits, &v, sizeof(bits));
+  return static_cast<int>(bits >> 32);
+#endif
+}
+
+// Whether each of several values v rounds to the same float f as any value
+// within `bound` of v. For |v| in [2^e, 2^(e+1)) the ties next to f are at
+// least 2^(e-24) from it, but for the one below f = 2^e, at 2^(e-25); as |v|
+// is not below that f, the bound alone has to stay under it. So the distance to f
+// plus the bound is held below 2^(e-24) and the bound below 2^(e-25), compared
+// by the high words, which errs towards false. (Subnormal floats' ties are
+// further apart than this takes them to be.)
+struct FoldedSettled {
+  int worst = static_cast<int>(0x80000000u);
+  int lowest = 0x7FFFFFFF;
+
+  __host__ __device__ __forceinline__ void Add(double v, float f, double bound) {
+    const int exponent = HighWord(v) & 0x7FF00000;
+    const double reach = fabs(v - static_cast<double>(f)) + bound;
+    const int over = HighWord(reach) - exponent;
+    worst = worst > over ? worst : over;
+    lowest = lowest < exponent ? lowest : exponent;
+  }
+  __host__ __device__ __forceinline__ bool All(double bound) const {
+    return worst < -(24 << 20) && HighWord(bound) < lowest - (25 << 20);
+  }
+};
+
 // The outputs rounded to float; returns whether every one is the float of
-// any value within `bound` of it. The tie next to a value s in [2^e, 2^(e+1))
-// is 2^(e-24) from the float that s rounds to, so the distance plus the bound
-// has to stay below that; compared by the high words, which errs towards
-// false.
+// any value within `bound` of it.
 template <int L, int C, int Step>
 __device__ __forceinline__ bool FoldedColumn(const double* __restrict__ in,
                                              float* __restrict__ out, size_t out_step,
                                              double bound) {
   double v[8];
   FoldedLine<L, C, Step, false>(in, v, nullptr);
-  int worst = static_cast<int>(0x80000000u);
+  FoldedSettled settled;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const float f = static_cast<float>(v[j]);
-    const double reach = fabs(v[j] - static_cast<double>(f)) + bound;
-    worst = max(worst, __double2hiint(reach) + (24 << 20) -
-                         (__double2hiint(v[j]) & 0x7FF00000));
+    settled.Add(v[j], f, bound);
     const int x = j < 4 ? C * 4 + j : L - 1 - C * 4 - (j - 4);
     out[x * out_step] = f;
   }
-  return worst < 0;
+  return settled.All(bound);
 }
 
 // Row pass of the folded inverse over all KC * H rows (as BatchRowPass), with
