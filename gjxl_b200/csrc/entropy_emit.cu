@@ -8,7 +8,7 @@
 // bits, then, when (state >> 20) >= frequency, the low 16 state bits, and the
 // state becomes (state / f << 12) + reverse_map[offset + state % f]. The
 // stream is the final 32-bit state followed by the pushed chunks in reverse
-// push order. Two sections per CTA, three warps each: a producer warp turns
+// push order. Two sections per CTA, four warps each: two producer warps turn
 // batches of tokens into encoder records (hybrid-uint extra bits, frequency,
 // exact division factor, reverse-map offset), one thread runs the state
 // recurrence, which is serial by the format, over the previous batch, and an
@@ -49,11 +49,9 @@ constexpr int kAnsThreads = kSectionThreads * kAnsPairs;
 constexpr uint32_t kAnsContexts = 4096;  // largest context map kept in shared memory
 constexpr uint32_t kMaxHotClusters = 32;
 constexpr int kAnsBatch = 128;    // tokens per record batch
-constexpr int kPrefixThreads = 512;
 constexpr int kPrefixPerThread = 4;
-constexpr int kPrefixChunk = kPrefixThreads * kPrefixPerThread;
-// Words a chunk can touch: its bits plus the partial word it starts in.
-constexpr int kPrefixWindow = (kPrefixTokenBits * kPrefixChunk + 63) / 64 + 2;
+constexpr int kPrefixThreads = 512;
+constexpr int kPrefixSmallThreads = 256;  // for small sections
 
 struct Code {
   int mode;
@@ -430,7 +428,9 @@ __device__ __forceinline__ uint32_t TakeAnsStep(AnsStep& step, const uint4& next
 }
 
 // One section's four warps (role 0 recurrence, 1 and 2 records, 3 bits).
-template <bool kCount>
+// kSmall: no map is staged or known to be a code's; an entry past the table
+// enters the recurrence cut to the table's size, and is reported at the end.
+template <bool kCount, bool kSmall>
 __device__ __forceinline__ void AnsSection(const EmitParams& p, AnsStage& st, const AnsMaps& where,
                                            bool checked, uint32_t s, int section, int role,
                                            int lane, int st_thread, uint32_t begin, uint32_t end,
@@ -483,7 +483,8 @@ __device__ __forceinline__ void AnsSection(const EmitParams& p, AnsStage& st, co
   uint32_t q = kAnsInitialState >> kAnsLogTable, m = kAnsInitialState & (kAnsTable - 1);
   uint32_t map_bits = 0;
   uint64_t top = slot_end * 64, carry = 0;
-  const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(where.staged_maps));
+  const uint32_t base =
+    kSmall ? 0 : static_cast<uint32_t>(__cvta_generic_to_shared(where.staged_maps));
   const bool records = role == 1 || role == 2;
   if (records && batches > 0) {
     fetch(0);
@@ -499,7 +500,17 @@ __device__ __forceinline__ void AnsSection(const EmitParams& p, AnsStage& st, co
         const uint4* records = st.records[buffer];
         uint32_t* chunks = st.chunks[buffer];
         const int count = batch_count(k);
-        if (!checked) {
+        if constexpr (kSmall) {
+          AnsStep step = PrepareAnsStep(q, records[count - 1]);
+          uint4 next = records[max(count - 2, 0)];
+          for (int i = count - 1; i >= 0; --i) {
+            const uint4 following = records[max(i - 2, 0)];
+            chunks[i] = TakeAnsStep<false>(step, next, code.reverse_map, base, q, m);
+            map_bits |= m;
+            m &= kAnsTable - 1;
+            next = following;
+          }
+        } else if (!checked) {
           // Runs of tokens whose maps are here, by plain shared loads; a token
           // between them leaves the run's loop (a choice inside the loop costs
           // every token 35 cycles, leaving it costs those that do).
@@ -582,6 +593,26 @@ __device__ __forceinline__ void AnsSection(const EmitParams& p, AnsStage& st, co
     if (k < words) slot[k] = v;
     SectionBarrier(section);
   }
+}
+
+// Whether a lane's share of a reverse map has an entry past the table. A warp
+// takes a map, all its loads under way at once: with the CTA on one map after
+// another, sections of 200 tokens spent 10 of 86 us here. Not inlined: inside the
+// kernel it lengthened the counting recurrence by 2% (48 sections of 31 K tokens:
+// 5285 us against 5078).
+__device__ __noinline__ bool MapLeavesTable(const uint16_t* map, bool aligned, int lane) {
+  uint32_t bits = 0;
+  if (aligned) {
+#pragma unroll
+    for (uint32_t i = 0; i < kAnsTable / 8; i += 32) {
+      const uint4 v = reinterpret_cast<const uint4*>(map)[i + lane];
+      bits |= (v.x | v.y | v.z | v.w) & 0xF000F000u;
+    }
+  } else {
+#pragma unroll 16
+    for (uint32_t i = lane; i < kAnsTable; i += 32) bits |= map[i] & 0xF000u;
+  }
+  return bits != 0;
 }
 
 template <bool kCount>
@@ -668,20 +699,11 @@ __global__ void __launch_bounds__(kAnsThreads) AnsSectionKernel(const __grid_con
     hot_storage[i] = v;
   }
   const bool aligned = reinterpret_cast<uintptr_t>(maps) % 16 == 0;
-  for (uint32_t c = 0; c < code.cluster_count; ++c) {
+  for (uint32_t c = warp; c < code.cluster_count; c += kAnsThreads / 32) {
     // Without copies, the first map stands in for a bad token's.
     const bool needed = cluster_tokens[c] != 0 || (c == 0 && hot == 0);
     if (!needed || slot_of[c] != kSlotNone) continue;
-    if (aligned) {
-      for (uint32_t i = threadIdx.x; i < kVectors; i += kAnsThreads) {
-        outside |= out_of_table(maps[c * kVectors + i]);
-      }
-    } else {
-#pragma unroll 4
-      for (uint32_t i = threadIdx.x; i < kAnsTable; i += kAnsThreads) {
-        outside |= code.reverse_map[c * kAnsTable + i] >= kAnsTable;
-      }
-    }
+    outside |= MapLeavesTable(code.reverse_map + c * kAnsTable, aligned, lane);
   }
   const bool checked = __syncthreads_or(outside) != 0;
   if (checked) {
@@ -695,8 +717,47 @@ __global__ void __launch_bounds__(kAnsThreads) AnsSectionKernel(const __grid_con
   where.staged_maps = reinterpret_cast<const uint16_t*>(hot_storage);
   where.staged = hot > 0 && !checked;
   if (active) {
-    AnsSection<kCount>(p, st, where, checked, s, section, role, lane, st_thread, begin, end,
-                       slot_begin, slot_end);
+    AnsSection<kCount, false>(p, st, where, checked, s, section, role, lane, st_thread, begin,
+                              end, slot_begin, slot_end);
+  }
+}
+
+// The same for small sections: nothing is staged but the clusters'
+// configurations. The kernel above counts each CTA's clusters, copies maps and
+// looks the others through before the first token, 8 KB a map, which a few
+// hundred tokens don't repay; and its copies leave room for four CTAs per SM.
+template <bool kCount>
+__global__ void __launch_bounds__(kAnsThreads, 5)
+AnsSmallKernel(const __grid_constant__ EmitParams p) {
+  __shared__ AnsStage stage[kAnsPairs];
+  __shared__ uint32_t configs[256];
+  __shared__ __align__(4) uint8_t slot_of[256];
+  const Code& code = p.code;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int section = warp / 4, role = (warp + 2 * section) % 4;
+  const int st_thread = threadIdx.x - kSectionThreads * section;
+  AnsStage& st = stage[section];
+  const uint32_t s = blockIdx.x * kAnsPairs + section;
+  uint32_t begin = 0, end = 0;
+  uint64_t slot_begin = 0, slot_end = 0;
+  const bool active = s < p.tokens.count && SectionBounds(p, s, !kCount, &begin, &end,
+                                                         &slot_begin, &slot_end,
+                                                         st_thread == 0);
+  for (uint32_t c = threadIdx.x; c < code.cluster_count; c += kAnsThreads) {
+    configs[c] = PackedConfig(code, c);
+    slot_of[c] = kSlotNone;
+  }
+  if (st_thread == 0) st.bad_token = 0;
+  __syncthreads();
+  AnsMaps where;
+  where.slot_of = slot_of;
+  where.configs = configs;
+  where.contexts = code.context_map;
+  where.staged_maps = nullptr;
+  where.staged = false;
+  if (active) {
+    AnsSection<kCount, true>(p, st, where, false, s, section, role, lane, st_thread, begin, end,
+                             slot_begin, slot_end);
   }
 }
 
@@ -778,12 +839,17 @@ __device__ __forceinline__ bool PrefixToken(const Code& code, const PrefixTables
 // memory where they fit kPrefixStagedBytes, and the next chunk's tokens are
 // loaded while this one is placed. With 256 threads and the lookups in global
 // memory, 192 sections of 31 K tokens took 353 us.
-template <bool kCount>
-__global__ void __launch_bounds__(kPrefixThreads, 2)
+template <bool kCount, bool kSmall>
+__global__ void __launch_bounds__(kSmall ? kPrefixSmallThreads : kPrefixThreads,
+                                  kSmall ? (kCount ? 8 : 6) : 2)
 PrefixSectionKernel(const __grid_constant__ EmitParams p, bool staged) {
+  constexpr int kThreads = kSmall ? kPrefixSmallThreads : kPrefixThreads;
+  constexpr int kChunk = kThreads * kPrefixPerThread;
+  // Words a chunk can touch: its bits plus the partial word it starts in.
+  constexpr int kWindow = (kPrefixTokenBits * kChunk + 63) / 64 + 2;
   extern __shared__ uint32_t prefix_tables[];
-  __shared__ unsigned long long window[kPrefixWindow];
-  __shared__ uint32_t warp_bits[2][kPrefixThreads / 32];
+  __shared__ unsigned long long window[kWindow];
+  __shared__ uint32_t warp_bits[2][kThreads / 32];
   __shared__ uint32_t bad_token;
   uint32_t begin, end;
   uint64_t slot_begin, slot_end;
@@ -802,20 +868,21 @@ PrefixSectionKernel(const __grid_constant__ EmitParams p, bool staged) {
       if (t < end) FetchToken(p.tokens, t, &context[k], &value[k]);
     }
   };
-  fetch(begin);
+  if constexpr (!kSmall) fetch(begin);
   PrefixTables tables = {nullptr, nullptr, nullptr};
-  if (staged) tables = StagePrefixTables(code, prefix_tables);
+  if (!kSmall && staged) tables = StagePrefixTables(code, prefix_tables);
   if (threadIdx.x == 0) bad_token = 0;
   // window[0] holds the partial word a chunk starts in; the rest is zero.
-  for (int i = threadIdx.x; i < kPrefixWindow; i += kPrefixThreads) window[i] = 0;
+  for (int i = threadIdx.x; i < kWindow; i += kThreads) window[i] = 0;
   __syncthreads();
   uint64_t position = 0;  // bits written so far
   int parity = 0;
-  for (uint32_t first = begin; first < end; first += kPrefixChunk, parity ^= 1) {
+  for (uint32_t first = begin; first < end; first += kChunk, parity ^= 1) {
     uint64_t data[kPrefixPerThread];
     uint32_t length[kPrefixPerThread];
     uint32_t mine = 0;
     bool bad = false;
+    if constexpr (kSmall) fetch(first);
 #pragma unroll
     for (int k = 0; k < kPrefixPerThread; ++k) {
       const uint32_t t = first + threadIdx.x * kPrefixPerThread + k;
@@ -827,7 +894,7 @@ PrefixSectionKernel(const __grid_constant__ EmitParams p, bool staged) {
       mine += length[k];
     }
     if (bad) bad_token = 1;
-    if (end - first > kPrefixChunk) fetch(first + kPrefixChunk);
+    if (!kSmall && end - first > kChunk) fetch(first + kChunk);
     // Exclusive scan of the threads' bit counts.
     uint32_t inclusive = mine;
 #pragma unroll
@@ -839,7 +906,7 @@ PrefixSectionKernel(const __grid_constant__ EmitParams p, bool staged) {
     __syncthreads();
     uint32_t before = inclusive - mine, chunk_bits = 0;
 #pragma unroll
-    for (int i = 0; i < kPrefixThreads / 32; ++i) {
+    for (int i = 0; i < kThreads / 32; ++i) {
       const uint32_t v = warp_bits[parity][i];
       if (i < warp) before += v;
       chunk_bits += v;
@@ -860,7 +927,7 @@ PrefixSectionKernel(const __grid_constant__ EmitParams p, bool staged) {
       const int full = static_cast<int>((end_bit >> 6) - w0);
       unsigned long long partial = 0;
       if (threadIdx.x == 0) partial = window[full];
-      for (int i = threadIdx.x; i < full; i += kPrefixThreads) {
+      for (int i = threadIdx.x; i < full; i += kThreads) {
         slot[w0 + i] = window[i];
         window[i] = 0;
       }
@@ -880,6 +947,9 @@ PrefixSectionKernel(const __grid_constant__ EmitParams p, bool staged) {
   }
 }
 
+// ------------------------------------------------------------ packing ----
+
+// byte_offsets[s] = sum over earlier sections of ceil(bits / 8); one CTA.
 __global__ void __launch_bounds__(1024) SectionByteOffsetsKernel(const uint64_t* bit_counts,
                                                                  uint32_t count,
                                                                  uint64_t* byte_offsets) {
@@ -912,7 +982,10 @@ __global__ void __launch_bounds__(1024) SectionByteOffsetsKernel(const uint64_t*
   if (threadIdx.x == 0) byte_offsets[count] = carry;
 }
 
-constexpr unsigned kPackSplit = 4;  // CTAs per section
+// CTAs per section, and the tokens per section that take one only (5000
+// sections of 100 tokens: 4 CTAs each cost 8 us of 51).
+constexpr unsigned kPackSplit = 4;
+constexpr uint32_t kPackOne = 1024;
 
 __global__ void __launch_bounds__(256) PackSectionsKernel(const uint64_t* slots,
                                                           size_t slot_capacity,
@@ -1057,11 +1130,40 @@ uint32_t HotClusters(const EmitParams& p) {
   return std::min(static_cast<uint32_t>(maps), p.code.cluster_count);
 }
 
+// Whether the sections are too small to repay what the full kernels stage for
+// each of them, by the tokens per section that the arrays hold. Sections x
+// tokens, us a call with packing (and counting only), full against small:
+//   ANS     300 x 20: 27 (19) / 23 (15)      5000 x 100: 172 (148) / 123 (99)
+//           600 x 100: 50 (43) / 57 (48)     2000 x 500: 303 (294) / 248 (235)
+//           300 x 200: 76 (70) / 99 (90)     1000 x 1000: 428 (424) / 409 (402)
+//   prefix  48 x 500: 14.5 (6.5) / 14.7 (6.4)    5000 x 100: 93 (58) / 43 (15)
+//           300 x 500: 16.6 (9.2) / 14.7 (6.5)   2000 x 2000: 60 (35) / 54 (27)
+//           500 x 2000: 25 (14.5) / 29 (14.5)    2000 x 5000: 100 (58) / 109 (59)
+// The small ANS kernel takes more CTAs an SM, so that it gains where the
+// sections fill the chip several times; below, only tokens that are fewer than
+// the full kernel's preparation. Prefix sections cost a staging each, which a
+// chip full of them pays once per turn: the more turns, the larger a section
+// has to be.
+bool SmallAnsSections(const Tokens& t) {
+  const uint32_t tokens = t.capacity / t.count;
+  return tokens < 64 || (tokens < 512 && t.count / 8 > static_cast<uint32_t>(CachedLimits().sms));
+}
+
+bool SmallPrefixSections(const Tokens& t) {
+  const uint64_t sms = std::max(1, CachedLimits().sms);
+  return t.capacity / t.count < std::min<uint64_t>(4096, 512 * (t.count / sms));
+}
+
 // Both writers raise their kernel's shared-memory limit to the most that any
 // call asks for, not to this call's need: the limit belongs to the kernel, and
 // calls from several host threads share it.
 template <bool kCount>
 void LaunchAns(EmitParams p, cudaStream_t stream) {
+  const unsigned ctas = (p.tokens.count + kAnsPairs - 1) / kAnsPairs;
+  if (SmallAnsSections(p.tokens)) {
+    AnsSmallKernel<kCount><<<ctas, kAnsThreads, 0, stream>>>(p);
+    return;
+  }
   p.hot_clusters = HotClusters(p);
   const int most = MapsWithin(CachedLimits().smem_per_block) * static_cast<int>(kAnsTable * 2);
   if (p.hot_clusters > 0 &&
@@ -1070,8 +1172,8 @@ void LaunchAns(EmitParams p, cudaStream_t stream) {
     cudaGetLastError();
     p.hot_clusters = 0;
   }
-  AnsSectionKernel<kCount><<<(p.tokens.count + kAnsPairs - 1) / kAnsPairs, kAnsThreads,
-                             p.hot_clusters * kAnsTable * 2, stream>>>(p);
+  AnsSectionKernel<kCount>
+    <<<ctas, kAnsThreads, p.hot_clusters * kAnsTable * 2, stream>>>(p);
 }
 
 template <bool kCount>
@@ -1079,17 +1181,22 @@ void LaunchSections(const EmitParams& p, cudaStream_t stream) {
   if (p.code.mode == GJXL_B200_ENTROPY_ANS) {
     LaunchAns<kCount>(p, stream);
   } else {
+    if (SmallPrefixSections(p.tokens)) {
+      PrefixSectionKernel<kCount, true>
+        <<<p.tokens.count, kPrefixSmallThreads, 0, stream>>>(p, false);
+      return;
+    }
     // The tables are staged where two CTAs of them fit an SM; a larger code is
     // looked up in global memory.
     const size_t bytes = PrefixTableBytes(p.code.context_count, p.code.cluster_count);
     bool staged = bytes <= kPrefixStagedBytes;
-    if (staged && cudaFuncSetAttribute(PrefixSectionKernel<kCount>,
+    if (staged && cudaFuncSetAttribute(PrefixSectionKernel<kCount, false>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(kPrefixStagedBytes)) != cudaSuccess) {
       cudaGetLastError();
       staged = false;
     }
-    PrefixSectionKernel<kCount>
+    PrefixSectionKernel<kCount, false>
       <<<p.tokens.count, kPrefixThreads, staged ? bytes : 0, stream>>>(p, staged);
   }
 }
@@ -1131,10 +1238,10 @@ extern "C" int gjxl_b200_entropy_write_sections(const gjxl_b200_entropy_code* co
   int status = CheckLaunch("entropy sections");
   if (status != GJXL_B200_OK || packed == nullptr) return status;
   SectionByteOffsetsKernel<<<1, 1024, 0, s>>>(bit_counts, sections->count, byte_offsets);
-  PackSectionsKernel<<<dim3(sections->count, kPackSplit), 256, 0, s>>>(slot_words, slot_word_capacity,
-                                                     sections->offsets, code->mode,
-                                                     bit_counts, byte_offsets, packed,
-                                                     packed_capacity, device_error);
+  const unsigned split = sections->capacity / sections->count < kPackOne ? 1 : kPackSplit;
+  PackSectionsKernel<<<dim3(sections->count, split), 256, 0, s>>>(
+    slot_words, slot_word_capacity, sections->offsets, code->mode, bit_counts, byte_offsets, packed,
+    packed_capacity, device_error);
   return CheckLaunch("entropy section packing");
 }
 

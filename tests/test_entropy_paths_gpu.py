@@ -156,6 +156,63 @@ def test_prefix_sections(cuda, clusters):
     check(make_tables(PREFIX, 60 + clusters, 300, clusters), values, ctx, offsets)
 
 
+def small_offsets(seed: int, sections: int, most: int, first: list[int]) -> np.ndarray:
+    sizes = np.random.default_rng(seed).integers(0, most + 1, sections)
+    sizes[:len(first)] = first
+    return np.concatenate([[0], np.cumsum(sizes)])
+
+
+# The kernels for small sections, with a few that are not: fewer than 64 tokens
+# a section (ANS); 400 sections of fewer than 1024 (prefix, chunks of 1024).
+@pytest.mark.parametrize("clusters", [1, 40])
+def test_small_sections(cuda, clusters):
+    offsets = small_offsets(1, 150, 90, [0, 1, 128, 129, 400, 257])
+    values, ctx = make_tokens(90 + clusters, int(offsets[-1]), 300)
+    check(make_tables(ANS, 91 + clusters, 300, clusters), values, ctx, offsets)
+    offsets = small_offsets(2, 400, 90, [0, 1, 1023, 1024, 1025, 2500])
+    values, ctx = make_tokens(92 + clusters, int(offsets[-1]), 300)
+    check(make_tables(PREFIX, 93 + clusters, 300, clusters), values, ctx, offsets)
+
+
+def test_many_sections(cuda):
+    """More sections than eight times the SMs: the small ANS kernel below 512 tokens a
+    section, the small prefix kernel below 4096."""
+    offsets = small_offsets(3, 1200, 130, [700])
+    values, ctx = make_tokens(94, int(offsets[-1]), 300)
+    check(make_tables(ANS, 95, 300, 40), values, ctx, offsets)
+    check(make_tables(PREFIX, 96, 300, 40), values, ctx, offsets)
+
+
+def test_ans_map_entry_outside_table_in_a_small_section(cuda):
+    values, ctx = make_tokens(99, 50, 1)
+    t = make_tables(ANS, 100, 1, 1)
+    t["reverse_map"][:] = 65535
+    got = write_sections(EntropyCode(t), torch.tensor([0, 50], dtype=torch.int32).cuda(),
+                         values=torch.from_numpy(values.view(np.int32)).cuda(),
+                         contexts=torch.from_numpy(ctx.view(np.int16)).cuda())
+    assert int(host(got["error"])[0]) & 4
+
+
+def test_ans_reverse_map_off_16_bytes(cuda):
+    """A map that no 16-byte load may read: looked through and used in place."""
+    offsets = np.array([0, 400, 1000])
+    values, ctx = make_tokens(97, 1000, 30)
+    t = make_tables(ANS, 98, 30, 3)
+    expected = [ans_stream(t, values[a:b], ctx[a:b]) for a, b in ((0, 400), (400, 1000))]
+    code = EntropyCode(t)
+    shifted = torch.empty(3 * 4096 + 1, dtype=torch.int16, device="cuda")[1:]
+    shifted.copy_(code._keep["reverse_map"].reshape(-1))
+    code._keep["reverse_map"] = shifted
+    got = write_sections(code, torch.from_numpy(offsets.astype(np.int32)).cuda(),
+                         values=torch.from_numpy(values.view(np.int32)).cuda(),
+                         contexts=torch.from_numpy(ctx.view(np.int16)).cuda())
+    assert int(host(got["error"])[0]) == 0
+    assert host(got["bit_counts"]).tolist() == [count for _, count in expected]
+    data = host(got["packed"]).tobytes()
+    size = (expected[0][1] + 7) // 8
+    assert data[:size] == expected[0][0].to_bytes(size, "little")
+
+
 @pytest.mark.parametrize("mode", [ANS, PREFIX])
 def test_threads_with_codes_of_different_sizes(cuda, mode):
     """Two host threads, each with its own stream and code: neither call's
