@@ -872,19 +872,25 @@ int LaunchConvWeights(const float* dz, const __nv_bfloat16* x, int layer, int n,
   return CheckLaunch("cnn weight gradients");
 }
 
+// Of the gradient planes' vector loads and stores. The caller's scratch may
+// start anywhere a float may; the bytes asked for leave room to round up.
+constexpr size_t kTrainAlignment = 16;
+
 size_t CnnTrainScratchBytes(int n) {
   // dhead, two gradient planes of the largest activation, partials.
   const size_t dhead = static_cast<size_t>(n) * 64 * kCnnHead * 4;
   const size_t plane = static_cast<size_t>(n) * 40 * 40 * kCnnC * 4;
   const size_t partial = ConvPartialRows(n) * (kCnnC * 9 * kCnnC + kCnnC) * 4;
   const size_t loss = ((static_cast<size_t>(n) * 64 + 255) / 256 + 1) * 4;
-  return Align(dhead, 256) + 2 * Align(plane, 256) + Align(partial, 256) + Align(loss, 256);
+  return Align(dhead, 256) + 2 * Align(plane, 256) + Align(partial, 256) + Align(loss, 256) +
+         kTrainAlignment;
 }
 
 int CnnTrainStep(const float* params, const CnnActivations& a, int n, const uint8_t* labels,
                  const float* targets, const float* weights, float qf_weight, float* grads,
                  void* scratch, float* loss, cudaStream_t stream) {
-  unsigned char* p = static_cast<unsigned char*>(scratch);
+  unsigned char* p = reinterpret_cast<unsigned char*>(
+    Align(reinterpret_cast<uintptr_t>(scratch), kTrainAlignment));
   float* dhead = reinterpret_cast<float*>(p);
   p += Align(static_cast<size_t>(n) * 64 * kCnnHead * 4, 256);
   const size_t plane = static_cast<size_t>(n) * 40 * 40 * kCnnC * 4;

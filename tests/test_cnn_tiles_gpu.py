@@ -31,3 +31,18 @@ def test_gradients_match_oracle(cuda, n):
         size = int(np.prod(shape))
         g, w = got[offset:offset + size].astype(np.float64), want[offset:offset + size]
         assert np.linalg.norm(g - w) <= 2e-2 * np.linalg.norm(w) + 1e-9, name
+
+
+def test_scratch_off_16_bytes(cuda):
+    """A scratch that starts at any float: the same gradients."""
+    x0, labels, targets, weights = random_batch(2, 5)
+    grads = []
+    for offset in (0, 4, 12):
+        net = ProposalNetwork(params(4))
+        load_batch(net, x0)
+        whole = torch.empty(net.scratch.numel() + offset, dtype=torch.uint8, device="cuda")
+        net.scratch = whole[offset:]
+        net.train_step(2, torch.from_numpy(labels).cuda(), torch.from_numpy(targets).cuda(),
+                       torch.from_numpy(weights).cuda(), lr=0.0, weight_decay=0.0)
+        grads.append(host(net.grads))
+    assert np.array_equal(grads[0], grads[1]) and np.array_equal(grads[0], grads[2])
