@@ -170,9 +170,23 @@ def candidate_cost_fp64_ops(blocks_x: int, blocks_y: int) -> int:
     image: every candidate transforms 3 channels forward and back, each
     separable DCT costs (W + H) multiply-adds per coefficient, and the
     bit-exact restatement rounds every multiply and every add separately
-    (2 FP64 operations per multiply-add). This counts the sequential sums: the
-    kernels' folded inverse passes execute a quarter of theirs."""
-    total = 0
+    (2 FP64 operations per multiply-add)."""
+    return sum(anchors * 3 * 2 * (w * h) * (w + h) * 2
+               for (w, h), anchors in candidate_anchors(blocks_x, blocks_y))
+
+
+def candidate_cost_executed_ops(blocks_x: int, blocks_y: int) -> int:
+    """FP64 instructions that the candidate-cost kernels issue for them: the
+    forward passes' sequential sums, and the folded inverse passes' 4 L + 8
+    per 8 outputs of a line of length L (columns transformed again, which few
+    planes have, are not counted)."""
+    return sum(anchors * 3 * (w * h) * (2 * (w + h) + (w + h) // 2 + 2)
+               for (w, h), anchors in candidate_anchors(blocks_x, blocks_y))
+
+
+def candidate_anchors(blocks_x: int, blocks_y: int) -> list[tuple[tuple[int, int], int]]:
+    """((W, H), number of candidates) of each family."""
+    out = []
     for w, h, cw, ch, step in FAMILIES:
         anchors = 0
         for ty in range(0, blocks_y, 8):
@@ -181,8 +195,8 @@ def candidate_cost_fp64_ops(blocks_x: int, blocks_y: int) -> int:
                 nx = len([x for x in range(0, 8 - cw + 1, step) if x + cw <= tw])
                 ny = len([y for y in range(0, 8 - ch + 1, step) if y + ch <= th])
                 anchors += nx * ny
-        total += anchors * 3 * 2 * (w * h) * (w + h) * 2
-    return total
+        out.append(((w, h), anchors))
+    return out
 
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of the seven
@@ -340,7 +354,8 @@ def run_gpu(args) -> dict:
     o = prof.outputs
     cost_ms = stage_ms.get("ac_strategy_costs", float("nan"))
     fp64_ops = candidate_cost_fp64_ops(o.blocks_x, o.blocks_y)
-    achieved = fp64_ops / (cost_ms / 1e3) / 1e12
+    executed_ops = candidate_cost_executed_ops(o.blocks_x, o.blocks_y)
+    achieved = executed_ops / (cost_ms / 1e3) / 1e12
     peak = fp64_peak_tflops(stream)
     launches = session.kernel_count(d_img.data_ptr(), row, 3)
     result = {
@@ -363,11 +378,12 @@ def run_gpu(args) -> dict:
             "bound": "fp64",
             "achieved": round(achieved, 3),
             "peak": round(peak, 3),
-            "unit": ("TFLOP/s (FP64 multiplies and adds of the sequential sums; the folded "
-                     "inverse passes execute a quarter of theirs)"),
+            "unit": "TFLOP/s (FP64 instructions issued; multiply, add and fused one each)",
             "frac": round(achieved / peak, 4),
             "traffic": COST_KERNEL_DRAM_BYTES,
+            "executed_ops": executed_ops,
             "algorithmic_ops": fp64_ops,
+            "sequential_equivalent": round(fp64_ops / (cost_ms / 1e3) / 1e12, 3),
             "peak_source": ("measured live: gjxl_b200_fp64_throughput (independent DMUL/DADD "
                             "chains on every SM); MEASURED_PEAKS.json has no FP64 figure"),
             "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum summed over "
@@ -436,10 +452,22 @@ class ReferencePool:
         self.pool.join()
 
 
+def reference_missing() -> str | None:
+    """Why the reference's library cannot run, or None."""
+    from oracle import ref
+    if not ref.LIBRARY_PATH.exists():
+        return (f"oracle/_ref/{ref.LIBRARY_PATH.name} is not built: it needs the reference's "
+                f"sources")
+    return None
+
+
 def run_reference(args) -> dict:
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return {}
+    missing = reference_missing()
+    if missing:
+        return {"impl": "reference", "unavailable": missing}
     pool = ReferencePool()
     for _ in range(args.warmup):
         pool.step()
@@ -656,8 +684,19 @@ def learned_leg(images: "BatchImages | None", precision: int, steps: int, warmup
                           "lanes": lanes}
         b.close()
         del dev
+    out |= or_unavailable("bd_rate", learned_bd_rate)
+    torch.cuda.empty_cache()
+    return out
+
+
+def learned_bd_rate() -> dict:
+    """The BD-rate part of the learned leg, through the encoder binding."""
+    from gjxl_b200 import learned
     from gjxl_b200.synthetic import generate_srgb8, workload_seed
+    if not learned.ENCODER_PATH.exists():
+        raise FileNotFoundError(f"{learned.ENCODER_PATH.name} not built")
     held = [generate_srgb8(2048, 2048, workload_seed(5, 1000 + i)) for i in range(4)]
+    out = {}
     ev = learned.evaluate(learned.WEIGHTS_PATH, held, learned_iterations=1)
     out["bd_rate_max"] = round(ev["bd_rate_mean"], 5)
     out["bd_rate_pnorm"] = round(ev["bd_rate_pnorm_mean"], 5)
@@ -670,8 +709,16 @@ def learned_leg(images: "BatchImages | None", precision: int, steps: int, warmup
     out["two_updates"] = {"bd_rate_max": round(ev2["bd_rate_mean"], 5),
                           "bd_rate_pnorm": round(ev2["bd_rate_pnorm_mean"], 5),
                           "analysis_speedup_4mp": round(ev2["speedup_mean"], 3)}
-    torch.cuda.empty_cache()
     return out
+
+
+def or_unavailable(name: str, part, *args) -> dict:
+    """part(*args), or {name: {"unavailable": why}}: what stands on files that
+    may be missing is reported, never fatal to the values already measured."""
+    try:
+        return part(*args)
+    except Exception as exc:
+        return {name: {"unavailable": f"{type(exc).__name__}: {exc}"[:200]}}
 
 
 def main():
@@ -709,7 +756,7 @@ def main():
     # The CPU leg's worker processes start before any CUDA work (spawn).
     pool = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline and not args.launch_list:
-        pool = ReferencePool()
+        pool = ReferencePool() if reference_missing() is None else None
     batch_images = None
     if rank == 0 and world == 1 and not args.no_batched and not args.launch_list:
         batch_images = BatchImages()
@@ -729,13 +776,12 @@ def main():
                     out["learned_form"]["batched"]["value"] / base, 3)
             out["learned_form"]["vs_plain_12mp"] = round(
                 out["learned_form"]["value_12mp"] / out["value"], 3)
+        if pool is None and not args.no_cpu_baseline and not args.launch_list and world == 1:
+            out["cpu_baseline"] = {"unavailable": reference_missing()}
         if pool is not None:
-            out["cpu_baseline"] = cpu_baseline_leg(pool)
+            out |= or_unavailable("cpu_baseline", lambda: {"cpu_baseline": cpu_baseline_leg(pool)})
         if world == 1 and not args.launch_list and not args.no_reference_gpu:
-            try:
-                out["reference_gpu"] = reference_gpu_leg()
-            except Exception as exc:  # reported, never fatal to our own line
-                out["reference_gpu"] = {"unavailable": str(exc)[:200]}
+            out |= or_unavailable("reference_gpu", lambda: {"reference_gpu": reference_gpu_leg()})
         print(json.dumps(out))
     if pool is not None:
         pool.close()
