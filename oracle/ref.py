@@ -46,6 +46,10 @@ _SIGNATURES = {
 _lib = None
 
 
+class LibraryMissing(FileNotFoundError):
+    """The oracle library has not been built (it needs the reference's sources)."""
+
+
 def available() -> bool:
     return LIBRARY_PATH.exists()
 
@@ -54,7 +58,7 @@ def lib() -> ctypes.CDLL:
     global _lib
     if _lib is None:
         if not LIBRARY_PATH.exists():
-            raise FileNotFoundError(
+            raise LibraryMissing(
                 f"{LIBRARY_PATH} is missing; build it with `make -C oracle`")
         handle = ctypes.CDLL(str(LIBRARY_PATH))
         handle.gjxl_ref_last_error.restype = ctypes.c_char_p
@@ -517,6 +521,8 @@ def _split(values: np.ndarray, contexts: np.ndarray, offsets: np.ndarray):
 class RefEntropyCode:
     """An EntropyCode built by the reference over split token sections
     (values uint32, contexts uint16, offsets uint32 [count + 1])."""
+
+    handle = None
 
     def __init__(self, kind: str, values, contexts, offsets, context_count: int,
                  max_clusters: int = 32):
