@@ -165,33 +165,6 @@ struct CostLayout {
   }
 };
 
-// Sequential float sum t[0] + t[1] + ... + t[n-1] (the reference's loop
-// order), 16 terms at a time with the next 16 loaded during the adds.
-template <int kCount>
-__device__ __forceinline__ float OrderedSum(const float* t) {
-  static_assert(kCount % 16 == 0, "whole groups");
-  float4 now[4], next[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) now[q] = reinterpret_cast<const float4*>(t)[q];
-  float sum = 0.0f;
-#pragma unroll 2
-  for (int j = 0; j < kCount; j += 16) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (j + 16 < kCount) next[q] = reinterpret_cast<const float4*>(t + j + 16)[q];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      sum += now[q].x;
-      sum += now[q].y;
-      sum += now[q].z;
-      sum += now[q].w;
-      now[q] = next[q];
-    }
-  }
-  return sum;
-}
-
 // Four consecutive floats, in one load where their alignment allows.
 __device__ __forceinline__ float4 LoadFour(const float* p, bool aligned) {
   if (aligned) return __ldg(reinterpret_cast<const float4*>(p));
@@ -526,9 +499,9 @@ CandidateCostKernel(const __grid_constant__ CostParams p, uint32_t candidate_cou
   const auto present = [&](int plane) { return anchor_x[plane / 3] >= 0; };
   const double* staged = Lay::kStagedBasis ? basis : nullptr;
   if constexpr (kExact) {
-    BatchRowPass<W, H, KC, true, true>(A, T, tid, kCostThreads, present, staged);
+    BatchRowPass<W, H, KC, true>(A, T, tid, kCostThreads, present, staged);
     __syncthreads();
-    BatchColumnPass<W, H, KC, true, true>(T, B, tid, kCostThreads, present, staged);
+    BatchColumnPass<W, H, KC, true>(T, B, tid, kCostThreads, present, staged);
   } else {
     BatchRowPassF<W, H, KC, true>(A, T, tid, kCostThreads, present);
     __syncthreads();

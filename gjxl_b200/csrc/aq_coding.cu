@@ -114,9 +114,9 @@ ForwardCoefficientsKernel(const float* opsin, size_t stride, size_t pitch, const
   __syncthreads();
   const auto present = [&](int plane) { return plane < 3 * active; };
   const double* staged = kBasis > 0 ? basis : nullptr;
-  BatchRowPass<W, H, KC, true>(px, tmp, threadIdx.x, kTransformThreads, present, staged);
+  BatchRowPass<W, H, KC>(px, tmp, threadIdx.x, kTransformThreads, present, staged);
   __syncthreads();
-  BatchColumnPass<W, H, KC, true>(tmp, px, threadIdx.x, kTransformThreads, present, staged);
+  BatchColumnPass<W, H, KC>(tmp, px, threadIdx.x, kTransformThreads, present, staged);
   __syncthreads();
   // Coefficient j = coefficient_index(v, u) goes to footprint (j % W, j / W).
   for (int i = threadIdx.x; i < active * 3 * N; i += kTransformThreads) {
@@ -587,7 +587,7 @@ FinalCflKernel(const __grid_constant__ CflFinalParams p) {
     if (b == 63) total_terms = offset + n;
   }
   __syncthreads();
-  // Every thread takes terms e = tid, tid + 128, ... of the tile; every
+  // Every thread takes terms e = tid, tid + kFinalCflThreads, ... of the tile; every
   // anchor's term count is a multiple of 64, so term e belongs to the anchor
   // of group e / 64. Batches of kBatch terms: all their global loads are
   // issued before the first term is computed.
@@ -930,34 +930,6 @@ struct CodingParams {
   uint32_t* error;
 };
 
-// t[0] + t[1] + ... + t[N-1] in order, 16 terms at a time with the next 16
-// loaded during the adds; `t` 16-byte aligned.
-template <int N>
-__device__ __forceinline__ float CodingOrderedSum(const float* t) {
-  static_assert(N % 16 == 0, "whole groups");
-  const float4* v = reinterpret_cast<const float4*>(t);
-  float4 now[4], next[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) now[k] = next[k] = v[k];
-  float sum = 0.0f;
-#pragma unroll 2
-  for (int j = 0; j < N / 4; j += 4) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (j + 4 < N / 4) next[k] = v[j + 4 + k];
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      sum += now[k].x;
-      sum += now[k].y;
-      sum += now[k].z;
-      sum += now[k].w;
-      now[k] = next[k];
-    }
-  }
-  return sum;
-}
-
 // ComputeQuantizedCoefficientsImpl's per-transform body
 // (reconstruction.cpp:480-700), one CTA per anchor.
 //
@@ -1139,7 +1111,7 @@ CodingKernel(const __grid_constant__ CodingParams p) {
     } else {
       // The ordered sums: error terms in storage order (+0.0 on the LLF
       // leaves the never -0.0 sum unchanged), and the border terms.
-      const float error_sum = CodingOrderedSum<N>(adjust_err[c]);
+      const float error_sum = OrderedSum<N>(adjust_err[c]);
       float border_sum = 0.0f;
 #pragma unroll 4
       for (int i = 0; i < kBorder; ++i) border_sum += border[c][i];

@@ -192,10 +192,10 @@ __device__ __forceinline__ void BlurRowBorders(const float* in, float* out, int 
                                                size_t in_pitch, size_t out_pitch,
                                                const Kernel17& k);
 
-template <int R>
 // The CTAs per SM bound the registers to what the row pass needs: the ends'
 // unrolled sums would take a third more and cost every CTA its occupancy (26 us
 // for a 2048x1536 plane triple and its half scale at R = 7 against 16).
+template <int R>
 __global__ void __launch_bounds__(kThreads, R > 8 ? 4 : 6)
 BlurRowsKernel(const float* in, float* out, int w, int h, size_t in_pitch, size_t out_pitch,
                const __grid_constant__ Kernel17 k) {

@@ -50,6 +50,34 @@ __device__ __forceinline__ float WarpMax(float v) {
   return v;
 }
 
+// Sequential float sum t[0] + t[1] + ... + t[n-1] (the reference's loop
+// order), 16 terms at a time with the next 16 loaded during the adds; `t`
+// 16-byte aligned.
+template <int kCount>
+__device__ __forceinline__ float OrderedSum(const float* t) {
+  static_assert(kCount % 16 == 0, "whole groups");
+  float4 now[4], next[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) now[q] = reinterpret_cast<const float4*>(t)[q];
+  float sum = 0.0f;
+#pragma unroll 2
+  for (int j = 0; j < kCount; j += 16) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (j + 16 < kCount) next[q] = reinterpret_cast<const float4*>(t + j + 16)[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      sum += now[q].x;
+      sum += now[q].y;
+      sum += now[q].z;
+      sum += now[q].w;
+      now[q] = next[q];
+    }
+  }
+  return sum;
+}
+
 // libjxl's CubeRootAndAdd (three reciprocal-cube-root Newton steps and one
 // refinement), as pinned in the reference's codec/color_transform.cpp:54.
 __device__ __forceinline__ float CubeRootAndAdd(float value, float add) {

@@ -16,9 +16,10 @@
 // fully unrolled, every basis value is a compile-time offset into constant
 // memory that enters the multiply as a constant-bank operand. Length 32 keeps
 // the sample loop rolled, because its fully unrolled code thrashes the
-// instruction cache, and reads the basis with a runtime (warp-uniform) index:
+// instruction cache, and reads the basis with a runtime (warp-uniform) index
 // from a copy that the caller staged in shared memory, four 128-bit broadcast
-// loads per sample, or else from constant memory.
+// loads per sample. The inverse passes are folded (below); their sequential
+// sums serve the few columns that the folded ones don't settle.
 #pragma once
 
 #include <cstdint>
@@ -44,11 +45,10 @@ __device__ __forceinline__ double DctBasis(int index) {
   return 0.0;
 }
 
-// Outputs k = C*8 .. C*8+7 of one line of length L:
-//   forward: out[k] = sum_s in[s] * basis[k * L + s]   (k = frequency)
-//   inverse: out[k] = sum_s in[s] * basis[s * L + k]   (k = sample, s = frequency)
+// Outputs k = C*8 .. C*8+7 of one line of length L, forward:
+// out[k] = sum_s in[s] * basis[k * L + s] (k = frequency).
 // `in` advances by InStep elements per sample, `out` by OutStep per output.
-template <int L, bool kForward, int C, int InStep, int OutStep, typename In, typename Out>
+template <int L, int C, int InStep, int OutStep, typename In, typename Out>
 __device__ __forceinline__ void LineChunk(const In* __restrict__ in, Out* __restrict__ out) {
   double acc[8];
 #pragma unroll
@@ -59,15 +59,14 @@ __device__ __forceinline__ void LineChunk(const In* __restrict__ in, Out* __rest
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int k = C * 8 + j;
-      acc[j] += v * DctBasis<L, kForward>(kForward ? k * L + s : s * L + k);
+      acc[j] += v * DctBasis<L, true>(k * L + s);
     }
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) out[j * OutStep] = static_cast<Out>(acc[j]);
 }
 
-// As LineChunk of a forward transform, where the sign of a zero output does
-// not matter: the first product starts the sum (instead of being added to
+// As LineChunk, where the sign of a zero output does not matter: the first product starts the sum (instead of being added to
 // +0.0), and the terms of frequency 0, whose basis 1/L is a power of two, are
 // exact, so their multiply-adds fuse. The other bits are LineChunk's.
 template <int L, int C, int InStep, int OutStep, typename In, typename Out>
@@ -91,45 +90,9 @@ __device__ __forceinline__ void LineChunkForward(const In* __restrict__ in,
   for (int j = 0; j < 8; ++j) out[j * OutStep] = static_cast<Out>(acc[j]);
 }
 
-// basis table laid out [s][k]: the transposed forward basis, or the inverse
-// basis as stored.
-template <int L, bool kForward>
-__device__ __forceinline__ double DctTable(int index) {
-  if constexpr (kForward) {
-    if constexpr (L == 8) return kDctForwardT8[index];
-    if constexpr (L == 16) return kDctForwardT16[index];
-    if constexpr (L == 32) return kDctForwardT32[index];
-  } else {
-    if constexpr (L == 8) return kDctInverse8[index];
-    if constexpr (L == 16) return kDctInverse16[index];
-    if constexpr (L == 32) return kDctInverse32[index];
-  }
-  return 0.0;
-}
-
-// Outputs k = chunk*8 .. chunk*8+7 of one line of length L, reading the basis
-// from constant memory with a runtime (warp-uniform) index:
-// out[k] = sum_s in[s] * table[s * L + k]. The sample loop is only partly
-// unrolled, so the code stays small.
-template <int L, bool kForward, int InStep, int OutStep, typename In, typename Out>
-__device__ __forceinline__ void LineChunkTable(int chunk, const In* __restrict__ in,
-                                               Out* __restrict__ out) {
-  double acc[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j] = 0.0;
-#pragma unroll 4
-  for (int s = 0; s < L; ++s) {
-    const double v = static_cast<double>(in[s * InStep]);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] += v * DctTable<L, kForward>(s * L + chunk * 8 + j);
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) out[j * OutStep] = static_cast<Out>(acc[j]);
-}
-
-// As LineChunkTable, with the basis table staged in shared memory by the
-// caller (laid out [s][k], 16-byte aligned): every lane of the warp reads the
-// same eight entries per sample, four 128-bit broadcast loads.
+// The same for chunk `chunk`, with the basis table staged in shared memory by
+// the caller (transposed, [s][k], 16-byte aligned): every lane of the warp reads
+// the same eight entries per sample, four 128-bit broadcast loads.
 template <int L, int InStep, int OutStep, typename In, typename Out>
 __device__ __forceinline__ void LineChunkShared(int chunk, const double* __restrict__ table,
                                                 const In* __restrict__ in,
@@ -185,37 +148,27 @@ __device__ __forceinline__ void LinePairShared(int part, const double* __restric
 }
 
 // Runtime chunk index (warp-uniform). Lengths 8 and 16 use the unrolled form
-// with compile-time basis offsets; length 32 reads its basis from a shared
-// table when the caller staged one (`table`), else from constant memory,
-// because the fully unrolled length-32 passes outgrow the instruction cache.
-// kSignless: LineChunkForward (forward transforms of lengths 8 and 16).
-template <int L, bool kForward, int InStep, int OutStep, bool kSignless = false, typename In,
-          typename Out>
+// with compile-time basis offsets; length 32 reads its basis from `table`, the
+// caller's shared copy, because the fully unrolled length-32 passes outgrow the
+// instruction cache. kSignless: LineChunkForward (lengths 8 and 16).
+template <int L, int InStep, int OutStep, bool kSignless = false, typename In, typename Out>
 __device__ __forceinline__ void LineChunkAt(int chunk, const In* __restrict__ in,
-                                            Out* __restrict__ out,
-                                            const double* table = nullptr) {
-  if constexpr (kSignless && L <= 16) {
-    static_assert(kForward, "forward transforms");
-    (void)table;
+                                            Out* __restrict__ out, const double* table) {
+  if constexpr (L == 32) {
+    LineChunkShared<L, InStep, OutStep>(chunk, table, in, out);
+  } else if constexpr (kSignless) {
     if (chunk == 0) {
       LineChunkForward<L, 0, InStep, OutStep>(in, out);
     } else if constexpr (L > 8) {
       LineChunkForward<L, 1, InStep, OutStep>(in, out);
     }
-  } else if constexpr (L == 32) {
-    if (table != nullptr) {
-      LineChunkShared<L, InStep, OutStep>(chunk, table, in, out);
-    } else {
-      LineChunkTable<L, kForward, InStep, OutStep>(chunk, in, out);
-    }
   } else {
-    (void)table;
     switch (chunk) {
       case 0:
-        LineChunk<L, kForward, 0, InStep, OutStep>(in, out);
+        LineChunk<L, 0, InStep, OutStep>(in, out);
         break;
       case 1:
-        if constexpr (L > 8) LineChunk<L, kForward, 1, InStep, OutStep>(in, out);
+        if constexpr (L > 8) LineChunk<L, 1, InStep, OutStep>(in, out);
         break;
       default:
         break;
@@ -245,67 +198,61 @@ struct PlaneBatch {
   }
 };
 
-// Row pass over all KC * H rows of `in` into `out` (same layout): item
+// Forward row pass over all KC * H rows of `in` into `out` (same layout): item
 // `item` is chunk item / (KC * H) of row item % (KC * H). `valid(plane)`
 // skips planes of absent transforms.
-// `table`: a shared copy of the width-length basis laid out [s][k], or null.
-template <int W, int H, int KC, bool kForward, bool kSignless = false, typename In,
-          typename Valid>
+// `table`: for a width of 32, a shared copy of the basis laid out [s][k].
+template <int W, int H, int KC, bool kSignless = false, typename In, typename Valid>
 __device__ __forceinline__ void BatchRowPass(const In* in, double* out, int tid, int threads,
-                                             Valid valid, const double* table = nullptr) {
+                                             Valid valid, const double* table) {
   using B = PlaneBatch<W, H, KC>;
   constexpr int kLines = KC * H;
   if constexpr (W == 32 && H == 32 && kLines % 2 == 0) {
     // Two lines half the batch apart; an absent transform's plane is computed
     // along with a present one's, and not used. (The 16x32 and 32x16 families,
     // with one length-32 pass, measure the same either way.)
-    if (table != nullptr) {
-      constexpr int kPairs = kLines / 2;
-      for (int item = tid; item < B::Items; item += threads) {
-        const int part = item / kPairs, line = item % kPairs;
-        if (!valid(line / H) && !valid((line + kPairs) / H)) continue;
-        LinePairShared<W, 1, 1>(part, table, in + line * B::RowPitch,
-                                out + line * B::RowPitch + part * 4, kPairs * B::RowPitch);
-      }
-      return;
+    constexpr int kPairs = kLines / 2;
+    for (int item = tid; item < B::Items; item += threads) {
+      const int part = item / kPairs, line = item % kPairs;
+      if (!valid(line / H) && !valid((line + kPairs) / H)) continue;
+      LinePairShared<W, 1, 1>(part, table, in + line * B::RowPitch,
+                              out + line * B::RowPitch + part * 4, kPairs * B::RowPitch);
     }
+    return;
   }
   for (int item = tid; item < B::Items; item += threads) {
     const int chunk = item / kLines, line = item % kLines;
     if (!valid(line / H)) continue;
-    LineChunkAt<W, kForward, 1, 1, kSignless>(chunk, in + line * B::RowPitch,
-                                   out + line * B::RowPitch + chunk * 8, table);
+    LineChunkAt<W, 1, 1, kSignless>(chunk, in + line * B::RowPitch,
+                                    out + line * B::RowPitch + chunk * 8, table);
   }
 }
 
 // Column pass over all KC * W columns: item `item` is chunk item / (KC * W)
-// of column item % (KC * W). `table`: as for the row pass, height-length.
-template <int W, int H, int KC, bool kForward, bool kSignless = false, typename Out,
-          typename Valid>
+// of column item % (KC * W). `table`: as for the row pass, for a height of 32.
+template <int W, int H, int KC, bool kSignless = false, typename Out, typename Valid>
 __device__ __forceinline__ void BatchColumnPass(const double* in, Out* out, int tid, int threads,
-                                                Valid valid, const double* table = nullptr) {
+                                                Valid valid, const double* table) {
   using B = PlaneBatch<W, H, KC>;
   constexpr int kLines = KC * W;
   if constexpr (W == 32 && H == 32 && kLines % 2 == 0) {
-    if (table != nullptr) {
-      constexpr int kPairs = kLines / 2;
-      for (int item = tid; item < B::Items; item += threads) {
-        const int part = item / kPairs, line = item % kPairs, other = line + kPairs;
-        if (!valid(line / W) && !valid(other / W)) continue;
-        const int base = line / W * B::PlanePitch + line % W;
-        LinePairShared<H, B::RowPitch, B::RowPitch>(
-          part, table, in + base, out + base + part * 4 * B::RowPitch,
-          other / W * B::PlanePitch + other % W - base);
-      }
-      return;
+    constexpr int kPairs = kLines / 2;
+    for (int item = tid; item < B::Items; item += threads) {
+      const int part = item / kPairs, line = item % kPairs, other = line + kPairs;
+      if (!valid(line / W) && !valid(other / W)) continue;
+      const int base = line / W * B::PlanePitch + line % W;
+      LinePairShared<H, B::RowPitch, B::RowPitch>(
+        part, table, in + base, out + base + part * 4 * B::RowPitch,
+        other / W * B::PlanePitch + other % W - base);
     }
+    return;
   }
   for (int item = tid; item < B::Items; item += threads) {
     const int chunk = item / kLines, line = item % kLines;
     const int plane = line / W, u = line % W;
     if (!valid(plane)) continue;
     const int base = plane * B::PlanePitch + u;
-    LineChunkAt<H, kForward, B::RowPitch, B::RowPitch, kSignless>(
+    LineChunkAt<H, B::RowPitch, B::RowPitch, kSignless>(
       chunk, in + base, out + base + chunk * 8 * B::RowPitch, table);
   }
 }
