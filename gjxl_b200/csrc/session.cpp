@@ -620,12 +620,12 @@ int Run(Session* s, const uint8_t* pixels, size_t row_stride, int channels,
 }
 
 // Runs the analysis as a replay of its captured graph: one launch instead of
-// ~350, with the same kernels and arguments. The graph reads the session's
-// input buffer; input elsewhere on the device is first copied there (one
-// stream-ordered 2D copy, 37 MB at 12 MP), so a new input pointer per image
-// costs that copy and never a recapture. Stage profiling, a caller stream
-// that is itself being captured, or a failed capture run the stages directly
-// on the caller's pointer.
+// 227 (effort 7; 339 at effort 9), with the same kernels and arguments. The
+// graph reads the session's input buffer; input elsewhere on the device is
+// first copied there (one stream-ordered 2D copy, 37 MB at 12 MP), so a new
+// input pointer per image costs that copy and never a recapture. Stage
+// profiling, a caller stream that is itself being captured, or a failed capture
+// run the stages directly on the caller's pointer.
 int RunReplay(Session* s, const uint8_t* pixels, size_t row_stride, int channels,
               cudaStream_t stream) {
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;

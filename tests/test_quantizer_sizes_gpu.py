@@ -29,3 +29,25 @@ def test_quantizer_from_the_final_field(cuda, w, h):
     scale = int(np.clip(F(65536) * (median - mad) / F(5), F(1), F(32768)))
     assert int(got["quantizer_params"][0]) == scale
     s.close()
+
+
+# 640 x 640 = 409600 blocks are the most that the cluster's shared memory holds;
+# above, the selections run as grid-wide kernels.
+@pytest.mark.parametrize("w,h", [(5120, 5120), (5128, 5120)])
+def test_quantizer_around_the_largest_cluster_field(cuda, w, h):
+    tile = generate_srgb8(640, 512, 77, sensor_noise=True)
+    img = np.tile(tile, (h // 512, -(-w // 640), 1))[:, :w].copy()
+    # Each tile darker than the last, so that the field does not repeat.
+    img[::2] //= np.linspace(1, 4, w).astype(np.uint8)[None, :, None]
+    s = AnalysisSession(w, h, butteraugli_target=1.0, effort=5)
+    s.analyze_host(img, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert s.host_error() == 0
+    got = s.host_results()
+    field = got["final_quant"].astype(F).ravel()
+    assert field.size == (w // 8) * (h // 8)
+    median = np.sort(field)[field.size // 2]
+    mad = np.sort(np.abs(field - median))[field.size // 2]
+    scale = int(np.clip(F(65536) * (median - mad) / F(5), F(1), F(32768)))
+    assert int(got["quantizer_params"][0]) == scale
+    s.close()
