@@ -200,11 +200,11 @@ def candidate_anchors(blocks_x: int, blocks_y: int) -> list[tuple[tuple[int, int
 
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of the seven
-# candidate-cost launches of one analysis: 354.57 MB measured by ncu on the
+# candidate-cost launches of one analysis: 354.94 MB measured by ncu on the
 # 2048x1536 image of the same generator, scaled by the pixel ratio to
 # 4032x3024 (each launch reads the three XYB planes and the pixel mask once,
 # 16 B per pixel, so traffic grows with the image area).
-COST_KERNEL_DRAM_BYTES = round(354_570_240 * (4032 * 3024) / (2048 * 1536))
+COST_KERNEL_DRAM_BYTES = round(354_938_880 * (4032 * 3024) / (2048 * 1536))
 
 
 def fp64_peak_tflops(stream: int) -> float:

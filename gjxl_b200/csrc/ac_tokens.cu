@@ -233,11 +233,12 @@ struct PopulationParams {
 // One CTA per strip of kStripRows block rows of a group (blockIdx.z) and
 // channel (blockIdx.y): a whole group per CTA left all but 3 SMs idle on a
 // 256x256 image and waited for one load after another (119 us there, 152 us
-// at 2048x1536). The strip's anchors are first listed per family, with the log2 of their footprint width; then, family by
-// family, each thread owns one physical index (and a share of the anchors
-// when the family has fewer than 256 indices) and counts zeros in a
-// register, four anchors' coefficients loaded at a time, so shared-memory
-// atomics happen once per thread and index, not once per coefficient.
+// at 2048x1536). The strip's anchors are first listed per family, with the log2
+// of their footprint width; then, family by family, each thread owns one
+// physical index (and a share of the anchors when the family has fewer than 256
+// indices) and counts zeros in a register, four anchors' coefficients loaded at
+// a time, so shared-memory atomics happen once per thread and index, not once
+// per coefficient.
 constexpr int kStripRows = 4;
 constexpr int kStripBlocks = kStripRows * kGroupBlocks;
 

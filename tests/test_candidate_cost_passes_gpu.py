@@ -2,8 +2,9 @@
 sequential double sums (EstimateAcStrategyCost, src/codec/ac_strategy.cpp:
 880-994), for residuals that the folded inverse transforms settle, that they
 have to transform again (magnitudes outside the settled range) and that are
-zero. Every float is the same up to the final eighth root: within one ulp of
-it, which the cost's last additions keep within two ulp."""
+zero: within one ulp of the eighth root, which the cost's last additions keep
+within two ulp. A pixel's last bit rarely shows in a cost; the passes' pixels are
+compared in test_folded_passes_gpu.py."""
 
 import numpy as np
 import pytest
