@@ -16,20 +16,22 @@ BINDING = ROOT / "integration" / "_build" / "libgjxl_b200_encoder.so"
 
 
 def _skip_without_reference(outcome):
-    """A test that ends at the oracle's library, or at the encoder binding, being
-    absent is skipped: both are built from the reference's sources. Built, but
-    not loading, either fails the test as ever."""
+    """A test that ends at the oracle's library, the reference's CUDA path or the
+    encoder binding being absent is skipped: all are built from the reference's
+    sources. Built, but not loading, they fail the test as ever."""
     if outcome.excinfo is None:
         return
     from oracle import ref
+    if ref.available():
+        return
     error = outcome.excinfo[1]
     if isinstance(error, ref.LibraryMissing):
         missing = ref.LIBRARY_PATH
-    elif BINDING.name in str(error) and not BINDING.exists() and not ref.available():
-        missing = BINDING
     else:
-        return
-    outcome.force_exception(pytest.skip.Exception(f"{missing.name} is not built"))
+        missing = next((p for p in (BINDING, ref.CUDA_LIBRARY_PATH)
+                        if p.name in str(error) and not p.exists()), None)
+    if missing is not None:
+        outcome.force_exception(pytest.skip.Exception(f"{missing.name} is not built"))
 
 
 @pytest.hookimpl(hookwrapper=True)

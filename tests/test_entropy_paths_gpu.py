@@ -11,7 +11,8 @@ import pytest
 import torch
 
 from gjxl_b200 import _lib
-from gjxl_b200.entropy import ANS, PREFIX, EntropyCode, _sections, write_sections
+from gjxl_b200.entropy import (ANS, PREFIX, EntropyCode, _sections, count_sections,
+                               write_sections)
 from tests.gpu_util import host
 
 pytestmark = pytest.mark.gpu
@@ -104,6 +105,11 @@ def check(t: dict, values, ctx, offsets):
         assert packed[at:at + size] == stream.to_bytes(size, "little"), f"section {s}"
         at += size
     assert host(got["byte_offsets"])[-1] == at
+    counted = count_sections([code], torch.from_numpy(offsets.astype(np.int32)).cuda(),
+                             values=torch.from_numpy(values.view(np.int32)).cuda(),
+                             contexts=torch.from_numpy(ctx.view(np.int16)).cuda())
+    assert int(host(counted["error"])[0]) == 0
+    assert np.array_equal(host(counted["bit_counts"])[:, 0], bits)
 
 
 SIZES = [0, 1, 2, 127, 128, 129, 255, 257, 1000, 3]
